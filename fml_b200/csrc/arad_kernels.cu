@@ -42,6 +42,7 @@ struct SetWs {
     float4 *pk;           // (nm, amax, amax) {r, xi, xi*c, xi*s} (FP32 paths)
     float2 *pz;           // (nm, amax, amax) {row, col}         (generic FP32 path)
     float *self32;        // (nm, amax)       self terms (generic FP32 path)
+    signed char *asc;     // (nm, amax)       1: the neighbour list ascends in r (fast FP64 path)
     signed char *cls;     // (nm, amax, amax) element class of each neighbour (fast path)
     signed char *acls;    // (nm, amax)       element class of each atom (fast path)
     float *selff;         // (nm, amax)       self terms (fast path)
@@ -50,8 +51,8 @@ struct SetWs {
     int *nrec;            // (nm)             records per molecule
 };
 
-// Element classes (distinct periodic-table positions) of the fast FP32 path:
-// the stoichiometric factor between two classes comes from a small table.
+// Element classes (distinct periodic-table positions) of the fast paths: the
+// stoichiometric factor between two classes comes from a small table.
 constexpr int FC_MAXC = 16;
 constexpr int FC_NPOS = 8 * 34;  // (row 0..7) * 34 + (col 0..33)
 struct ClassInfo {
@@ -60,6 +61,7 @@ struct ClassInfo {
     int present[FC_NPOS];
     signed char map[FC_NPOS]; // position -> class, -1 if absent
     float stoch[FC_MAXC * FC_MAXC];
+    double stoch64[FC_MAXC * FC_MAXC];  // the factor as the pair loop forms it, in FP64
 };
 
 __host__ __device__ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -70,7 +72,8 @@ size_t set_ws_bytes(int nm, int amax) {
            align256(a1 * sizeof(double)) + align256(a2 * sizeof(float4)) +
            align256(a2 * sizeof(float2)) + align256(a1 * sizeof(float)) + align256(a2) +
            align256(a1) + align256(a1 * sizeof(float)) + align256(a2 * sizeof(float4)) +
-           align256(a2 * sizeof(int)) + align256((size_t)nm * sizeof(int));
+           align256(a2 * sizeof(int)) + align256((size_t)nm * sizeof(int)) +
+           align256(a1);
 }
 
 SetWs carve(char *&p, int nm, int amax) {
@@ -88,6 +91,7 @@ SetWs carve(char *&p, int nm, int amax) {
     w.spk = reinterpret_cast<float4 *>(p); p += align256(a2 * sizeof(float4));
     w.smeta = reinterpret_cast<int *>(p); p += align256(a2 * sizeof(int));
     w.nrec = reinterpret_cast<int *>(p); p += align256((size_t)nm * sizeof(int));
+    w.asc = reinterpret_cast<signed char *>(p); p += align256(a1);
     return w;
 }
 
@@ -152,40 +156,89 @@ __host__ __device__ inline double fp32_scale(const AradParams &P) {
     return sqrt(-P.inv_width * 1.4426950408889634);
 }
 
-// Stage 1: one thread per (molecule, atom).
-__global__ void arad_prep_kernel(const double *__restrict__ X, const int *__restrict__ N, int nm,
-                                 int amax, AradParams P, int conditional_sine, SetWs w) {
-    const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ int ptp_pos(double row, double col) {
+    const double r = rint(row), c = rint(col);
+    if (r != row || c != col || r < 0.0 || r > 7.0 || c < 0.0 || c > 33.0) return -1;
+    return (int)r * 34 + (int)c;
+}
+
+// Marks a periodic-table position as present. The plain read first: nearly
+// every mark repeats one already made, and thousands of atomics on the same
+// few words serialise.
+__device__ __forceinline__ void mark_class(ClassInfo *ci, int pos) {
+    int *word = pos < 0 ? &ci->flag : &ci->present[pos];
+    if (*(volatile int *)word == 0) atomicOr(word, 1);
+}
+
+// Stage 1: one warp per (molecule, atom), lanes over its neighbours
+// (coalesced rows of the descriptor). With `ci` set, the periodic-table
+// positions of the atom (Z) and of its neighbours are marked for the class
+// tables in the same pass.
+constexpr int PREP_WARPS = 4;
+__global__ void __launch_bounds__(PREP_WARPS * 32)
+arad_prep_kernel(const double *__restrict__ X, const double *__restrict__ Z,
+                 const int *__restrict__ N, int nm, int amax, AradParams P, int conditional_sine,
+                 SetWs w, ClassInfo *ci) {
+    const long long gid = (long long)blockIdx.x * PREP_WARPS + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
     if (gid >= (long long)nm * amax) return;
     const int m = (int)(gid / amax), a = (int)(gid % amax);
     const int n = min(max(N[m], 0), amax);  // counts beyond amax are clamped
     const size_t base = (size_t)m * amax + a;
     if (a >= n) {
-        w.nnb[base] = 0;
-        w.self[base] = 0.0;
-        w.self32[base] = 0.0f;
+        if (lane == 0) w.nnb[base] = 0;
         return;
     }
     const double *x = X + base * 5 * amax;
     // neighbour prefix: the loop of atomic_distl2 exits at the first r > cut
-    int cnt = 0;
-    while (cnt < n && !(x[cnt] > P.cut)) ++cnt;
-    w.nnb[base] = cnt;
+    int cnt = n;
+    for (int k0 = 0; k0 < n; k0 += 32) {
+        const unsigned stop = __ballot_sync(0xffffffffu, k0 + lane < n && x[k0 + lane] > P.cut);
+        if (stop) {
+            cnt = k0 + __ffs(stop) - 1;
+            break;
+        }
+    }
     double *xi = w.xi + base * amax;
     float4 *pk = w.pk + base * amax;
     float2 *pz = w.pz + base * amax;
-    for (int k = 0; k < n; ++k) {
+    bool ascends = true;
+    for (int k = lane; k < n; k += 32) {
         const double r = x[k];
         double s = 0.0;  // farad_kernels.f90:516 zero-initialised table
         if (!conditional_sine || r < P.cut) s = __dsub_rn(1.0, sin(__dmul_rn(r, P.inv_cut)));
         xi[k] = s;
         if (k < cnt) {
             const double c = x[3 * amax + k], sn = x[4 * amax + k];
+            const double row = x[amax + k], col = x[2 * amax + k];
             pk[k] = make_float4((float)(r * fp32_scale(P)), (float)s, (float)(s * c),
                                 (float)(s * sn));
-            pz[k] = make_float2((float)x[amax + k], (float)x[2 * amax + k]);
+            pz[k] = make_float2((float)row, (float)col);
+            ascends = ascends && (k == 0 || r >= x[k - 1]);
+            if (ci) mark_class(ci, ptp_pos(row, col));
         }
     }
+    ascends = __all_sync(0xffffffffu, ascends);
+    if (lane == 0) {
+        w.nnb[base] = cnt;
+        w.asc[base] = ascends ? 1 : 0;
+        if (ci) mark_class(ci, ptp_pos(Z[base * 2 + 0], Z[base * 2 + 1]));
+    }
+}
+
+// Self terms of the generic pair kernel, one thread per (molecule, atom).
+// With `fast_ci` set they are needed only if the fast path is not usable.
+__global__ void arad_generic_self_kernel(const double *__restrict__ X, const int *__restrict__ N,
+                                         int nm, int amax, AradParams P, SetWs w,
+                                         const ClassInfo *fast_ci) {
+    if (fast_ci && fast_ci->flag == 0) return;
+    const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (gid >= (long long)nm * amax) return;
+    const size_t base = (size_t)gid;
+    const int cnt = w.nnb[base];
+    const double *x = X + base * 5 * amax, *xi = w.xi + base * amax;
+    const float4 *pk = w.pk + base * amax;
+    const float2 *pz = w.pz + base * amax;
     w.self[base] = distl2_f64(x, xi, cnt, x, xi, cnt, amax, P);
     const float maxg2s = (float)(P.maxg2 * fp32_scale(P) * fp32_scale(P));
     w.self32[base] = distl2_f32(pk, pz, cnt, pk, pz, cnt, maxg2s, (float)P.rw2, (float)P.cw2);
@@ -293,75 +346,66 @@ arad_pair_kernel(const double *__restrict__ X1, const double *__restrict__ Z1,
 constexpr int FC_BM = 8, FC_WARPS = 8, FC_MAXREC = 1024, FC_MAXA = 32, FC_MAXSIG = 8;
 constexpr int FC_SST = FC_MAXC + 1;
 
-__device__ __forceinline__ int ptp_pos(double row, double col) {
-    const double r = rint(row), c = rint(col);
-    if (r != row || c != col || r < 0.0 || r > 7.0 || c < 0.0 || c > 33.0) return -1;
-    return (int)r * 34 + (int)c;
-}
-
-// marks the periodic-table positions of the atoms and their neighbours
-__global__ void arad_class_scan_kernel(const double *__restrict__ X, const double *__restrict__ Z,
-                                       const int *__restrict__ N, int nm, int amax, double cut,
-                                       ClassInfo *ci) {
-    const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= (long long)nm * amax) return;
-    const int m = (int)(gid / amax), a = (int)(gid % amax);
-    const int n = min(max(N[m], 0), amax);
-    if (a >= n) return;
-    const size_t base = (size_t)m * amax + a;
-    int pos = ptp_pos(Z[base * 2 + 0], Z[base * 2 + 1]);
-    if (pos < 0) { atomicOr(&ci->flag, 1); return; }
-    atomicOr(&ci->present[pos], 1);
-    const double *x = X + base * 5 * amax;
-    for (int k = 0; k < n && !(x[k] > cut); ++k) {
-        pos = ptp_pos(x[amax + k], x[2 * amax + k]);
-        if (pos < 0) { atomicOr(&ci->flag, 1); return; }
-        atomicOr(&ci->present[pos], 1);
+// One CTA: class ids in position order and the stoichiometric tables
+// (farad_kernels.f90:80-81).
+constexpr int CB_TPB = 288;  // >= FC_NPOS and FC_MAXC^2
+static_assert(CB_TPB >= FC_NPOS && CB_TPB >= FC_MAXC * FC_MAXC, "one thread per entry");
+__global__ void __launch_bounds__(CB_TPB)
+arad_class_build_kernel(ClassInfo *ci, double rw2, double cw2) {
+    __shared__ int rows[FC_MAXC], cols[FC_MAXC], before[CB_TPB / 32 + 1];
+    const int pos = threadIdx.x, warp = pos >> 5, lane = pos & 31;
+    const bool here = pos < FC_NPOS && ci->present[pos];
+    const unsigned mask = __ballot_sync(0xffffffffu, here);
+    if (lane == 0) before[warp + 1] = __popc(mask);
+    if (pos == 0) before[0] = 0;
+    __syncthreads();
+    if (pos == 0)
+        for (int q = 0; q < CB_TPB / 32; ++q) before[q + 1] += before[q];
+    __syncthreads();
+    const int nc = min(before[CB_TPB / 32], FC_MAXC);
+    const int c = before[warp] + __popc(mask & ((1u << lane) - 1));
+    if (pos < FC_NPOS) ci->map[pos] = here && c < FC_MAXC ? (signed char)c : -1;
+    if (here && c < FC_MAXC) {
+        rows[c] = pos / 34;
+        cols[c] = pos % 34;
+    }
+    __syncthreads();
+    if (pos == 0) {
+        ci->ncls = nc;
+        if (before[CB_TPB / 32] > FC_MAXC) ci->flag |= 2;
+    }
+    if (pos < FC_MAXC * FC_MAXC) {
+        const int a = pos / FC_MAXC, b = pos % FC_MAXC;
+        double v = 0.0;
+        if (a < nc && b < nc) {
+            const double dr = (double)(rows[a] - rows[b]), dc = (double)(cols[a] - cols[b]);
+            // the operations of the pair loop (distl2_f64), so the same value
+            v = __ddiv_rn(__dmul_rn(__ddiv_rn(rw2, __dadd_rn(rw2, __dmul_rn(dr, dr))), cw2),
+                          __dadd_rn(cw2, __dmul_rn(dc, dc)));
+        }
+        ci->stoch64[pos] = v;
+        ci->stoch[pos] = (float)v;
     }
 }
 
-// one thread: class ids and the stoichiometric table (farad_kernels.f90:80-81)
-__global__ void arad_class_build_kernel(ClassInfo *ci, double rw2, double cw2) {
-    int rows[FC_MAXC], cols[FC_MAXC];
-    int nc = 0;
-    for (int pos = 0; pos < FC_NPOS; ++pos) {
-        ci->map[pos] = -1;
-        if (ci->present[pos]) {
-            if (nc == FC_MAXC) { ci->flag |= 2; break; }
-            rows[nc] = pos / 34;
-            cols[nc] = pos % 34;
-            ci->map[pos] = (signed char)nc;
-            ++nc;
-        }
-    }
-    ci->ncls = nc;
-    for (int a = 0; a < FC_MAXC; ++a)
-        for (int b = 0; b < FC_MAXC; ++b) {
-            double v = 0.0;
-            if (a < nc && b < nc) {
-                const double dr = (double)(rows[a] - rows[b]), dc = (double)(cols[a] - cols[b]);
-                v = rw2 / (rw2 + dr * dr) * cw2 / (cw2 + dc * dc);
-            }
-            ci->stoch[a * FC_MAXC + b] = (float)v;
-        }
-}
-
-// element classes of every neighbour record and atom (after the class build)
+// Element classes of every neighbour record and atom (after the class build);
+// one thread per (molecule, atom, neighbour).
 __global__ void arad_class_assign_kernel(const double *__restrict__ X, const double *__restrict__ Z,
                                          const int *__restrict__ N, int nm, int amax,
                                          const ClassInfo *ci, SetWs w) {
     const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= (long long)nm * amax) return;
-    const int m = (int)(gid / amax), a = (int)(gid % amax);
+    if (gid >= (long long)nm * amax * amax) return;
+    const size_t base = (size_t)(gid / amax);
+    const int k = (int)(gid % amax);
+    const int m = (int)(base / amax), a = (int)(base % amax);
     const int n = min(max(N[m], 0), amax);
-    const size_t base = (size_t)m * amax + a;
-    if (a >= n) { w.acls[base] = 0; return; }
-    int pos = ptp_pos(Z[base * 2 + 0], Z[base * 2 + 1]);
-    w.acls[base] = pos >= 0 ? max((int)ci->map[pos], 0) : 0;
-    const double *x = X + base * 5 * amax;
-    const int cnt = w.nnb[base];
-    for (int k = 0; k < cnt; ++k) {
-        pos = ptp_pos(x[amax + k], x[2 * amax + k]);
+    if (k == 0) {
+        const int pos = a < n ? ptp_pos(Z[base * 2 + 0], Z[base * 2 + 1]) : -1;
+        w.acls[base] = pos >= 0 ? max((int)ci->map[pos], 0) : 0;
+    }
+    if (a < n && k < w.nnb[base]) {
+        const double *x = X + base * 5 * amax;
+        const int pos = ptp_pos(x[amax + k], x[2 * amax + k]);
         w.cls[base * amax + k] = pos >= 0 ? (signed char)max((int)ci->map[pos], 0) : 0;
     }
 }
@@ -905,6 +949,336 @@ arad_fast_pair_kernel(SetWs w1, const int *__restrict__ N1, int nm1, SetWs w2,
     }
 }
 
+// ---- fast FP64 path ---------------------------------------------------------
+// atomic_distl2 in FP64 for descriptors of at most FC_MAXA atoms and FC_MAXC
+// element classes, bit for bit what the generic kernel gives: one thread sums
+// an atom pair's terms in the reference's order with the reference's
+// operations. At sigma 0.1 the exponent carries l2 / sigma^2 = 100 l2, and sums
+// in any other order leave the 1e-12 agreement with the reference.
+//
+// Per molecule pair, both molecules staged in shared memory:
+//   1. the run of neighbours m2 of j1 inside the (8 w)^2 window of every
+//      record (i1, m1), walking both ascending lists together (a list that
+//      does not ascend keeps its whole length, and its terms are tested);
+//   2. the atom pairs bucketed by their number of terms, so that the 32 pairs
+//      of a warp have nearly the same number (86 % of the lanes work, against
+//      59 % with loops over m1 and m2 in lockstep);
+//   3. one thread per atom pair walks its runs as one flat loop;
+//   4. the kernel exponentials of every l2 and sigma, summed in a fixed order.
+// Bound by the FP64 pipe: 28 FP64 instructions per term, 16 of them the
+// exponential. The stoichiometric factor comes from the class table, formed by
+// the same operations (two FP64 divisions per term before), and the operands
+// from shared memory (per-lane gathers from global memory before).
+constexpr int F6_TPB = 256, F6_BUCKETS = 64;
+constexpr int F6_WIN = 4096;  // runs held at a time (8 KB): the atoms j1 go in chunks above that
+constexpr int F6_SST = FC_MAXC + 1;
+
+struct F64Side {
+    double2 *A, *B;    // records by atom: (r, sine factor), (cos, sin)
+    double *self;
+    int *off;          // record offsets of the atoms
+    int *acls, *asc;
+    unsigned char *C;  // class of each record
+};
+struct F64View {
+    F64Side i, j;
+    double *l2;           // l2 of every atom pair
+    double *st;           // stoichiometric table, row stride F6_SST
+    double *red;          // (F6_TPB / 32) * MAXSIG
+    int *tot;             // terms of every atom pair
+    int *bucket;          // F6_BUCKETS + 1
+    unsigned short *win;  // F6_WIN: [m1][atom pair] first neighbour | length << 8
+    unsigned short *perm; // atom pairs by number of terms
+};
+
+__host__ __device__ inline int f64_pad(int n) { return (n + 7) & ~7; }
+inline size_t f64_smem_bytes(int amax) {
+    const size_t R = (size_t)f64_pad(amax * amax);
+    return R * 4 * sizeof(double2) +
+           (R + FC_MAXC * F6_SST + (F6_TPB / 32) * MAXSIG + 2 * FC_MAXA) * sizeof(double) +
+           (R + F6_BUCKETS + 8 + 2 * (3 * FC_MAXA + 8)) * sizeof(int) +
+           (F6_WIN + R) * sizeof(unsigned short) + 2 * R;
+}
+// the self kernel: one side and the table
+inline size_t f64_self_smem_bytes(int amax) {
+    const size_t R = (size_t)f64_pad(amax * amax);
+    return R * 2 * sizeof(double2) + (FC_MAXC * F6_SST + FC_MAXA) * sizeof(double) +
+           (3 * FC_MAXA + 8) * sizeof(int) + R;
+}
+
+__device__ __forceinline__ F64View f64_view(unsigned char *p, int amax) {
+    const int R = f64_pad(amax * amax);
+    F64View v;
+    v.i.A = reinterpret_cast<double2 *>(p);
+    v.i.B = v.i.A + R;
+    v.j.A = v.i.B + R;
+    v.j.B = v.j.A + R;
+    v.l2 = reinterpret_cast<double *>(v.j.B + R);
+    v.st = v.l2 + R;
+    v.red = v.st + FC_MAXC * F6_SST;
+    v.i.self = v.red + (F6_TPB / 32) * MAXSIG;
+    v.j.self = v.i.self + FC_MAXA;
+    v.tot = reinterpret_cast<int *>(v.j.self + FC_MAXA);
+    v.bucket = v.tot + R;
+    int *q = v.bucket + F6_BUCKETS + 8;
+    for (F64Side *s : {&v.i, &v.j}) {
+        s->off = q;
+        s->acls = q + FC_MAXA + 8;
+        s->asc = s->acls + FC_MAXA;
+        q += 3 * FC_MAXA + 8;
+    }
+    v.win = reinterpret_cast<unsigned short *>(q);
+    v.perm = v.win + F6_WIN;
+    v.i.C = reinterpret_cast<unsigned char *>(v.perm + R);
+    v.j.C = v.i.C + R;
+    return v;
+}
+
+// Whole CTA (of any size >= 32): molecule m's records and atoms. Synchronises
+// between the offsets and the records; the caller synchronises after.
+__device__ void f64_load(const F64Side &s, const double *__restrict__ X, const SetWs &w, int m,
+                         int amax, int n, bool use_self) {
+    const size_t mol = (size_t)m * amax;
+    if (threadIdx.x < 32) {
+        const int a = threadIdx.x;
+        const int cnt = a < n ? w.nnb[mol + a] : 0;
+        int incl = cnt;
+        for (int d = 1; d < 32; d <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, incl, d);
+            if (a >= d) incl += o;
+        }
+        s.off[a] = incl - cnt;
+        if (a == 31) s.off[32] = incl;
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < n * amax; t += blockDim.x) {
+        const int a = t / amax, k = t - a * amax;
+        const int beg = s.off[a];
+        if (k < s.off[a + 1] - beg) {
+            const double *x = X + (mol + a) * 5 * amax + k;
+            s.A[beg + k] = make_double2(x[0], w.xi[(mol + a) * amax + k]);
+            s.B[beg + k] = make_double2(x[3 * amax], x[4 * amax]);
+            s.C[beg + k] = (unsigned char)w.cls[(mol + a) * amax + k];
+        }
+    }
+    for (int a = threadIdx.x; a < n; a += blockDim.x) {
+        s.self[a] = use_self ? w.self[mol + a] : 0.0;
+        s.acls[a] = w.acls[mol + a];
+        s.asc[a] = w.asc[mol + a];
+    }
+}
+
+__device__ __forceinline__ void f64_load_table(double *st, const ClassInfo *ci) {
+    for (int t = threadIdx.x; t < FC_MAXC * FC_MAXC; t += blockDim.x)
+        st[(t / FC_MAXC) * F6_SST + t % FC_MAXC] = ci->stoch64[t];
+}
+
+// One term of atomic_distl2 (the operations and order of distl2_f64).
+__device__ __forceinline__ double f64_term(double t, double inv_width, const double2 &A1,
+                                           const double2 &B1, const double2 &A2, const double2 &B2,
+                                           double st) {
+    double d = __dmul_rn(__dmul_rn(exp(__dmul_rn(t, inv_width)), A1.y), A2.y);
+    d = __dmul_rn(d, st);
+    const double ang = __dadd_rn(__dadd_rn(1.0, __dmul_rn(B1.x, B2.x)), __dmul_rn(B1.y, B2.y));
+    return __dmul_rn(d, ang);
+}
+
+// Self terms, one warp per molecule, one lane per atom.
+__global__ void __launch_bounds__(32)
+arad_f64_self_kernel(const double *__restrict__ X, SetWs w, const int *__restrict__ N, int nm,
+                     int amax, AradParams P, const ClassInfo *ci) {
+    extern __shared__ __align__(16) unsigned char fc_smem_raw[];
+    if (ci->flag) return;
+    const int m = blockIdx.x;
+    if (m >= nm) return;
+    const int R = f64_pad(amax * amax);
+    F64Side s;
+    s.A = reinterpret_cast<double2 *>(fc_smem_raw);
+    s.B = s.A + R;
+    double *st = reinterpret_cast<double *>(s.B + R);
+    s.self = st + FC_MAXC * F6_SST;
+    s.off = reinterpret_cast<int *>(s.self + FC_MAXA);
+    s.acls = s.off + FC_MAXA + 8;
+    s.asc = s.acls + FC_MAXA;
+    s.C = reinterpret_cast<unsigned char *>(s.asc + FC_MAXA);
+    const int n = min(max(N[m], 0), amax), a = threadIdx.x;
+    f64_load_table(st, ci);
+    f64_load(s, X, w, m, amax, n, false);
+    __syncthreads();
+    if (a >= n) return;
+    double sum = 0.0;
+    for (int k1 = s.off[a]; k1 < s.off[a + 1]; ++k1) {
+        const double2 A1 = s.A[k1], B1 = s.B[k1];
+        const double *strow = st + s.C[k1] * F6_SST;
+        for (int k2 = s.off[a]; k2 < s.off[a + 1]; ++k2) {
+            const double2 A2 = s.A[k2];
+            const double dr = __dsub_rn(A2.x, A1.x);
+            const double t = __dmul_rn(dr, dr);
+            if (t < P.maxg2)
+                sum = __dadd_rn(sum, f64_term(t, P.inv_width, A1, B1, A2, s.B[k2], strow[s.C[k2]]));
+        }
+    }
+    w.self[(size_t)m * amax + a] = sum;
+}
+
+// Sum of atom pair ap = (i1, j1) of a chunk of nap over its runs, in (m1, m2)
+// order. kTest: some list
+// of J does not ascend, so terms outside the window occur in the runs.
+template <bool kTest>
+__device__ __forceinline__ double f64_pair_sum(const F64View &v, int i1, int j1, int ap, int nap,
+                                               const AradParams &P) {
+    const unsigned short *win = v.win + ap;
+    double sum = 0.0;
+    int k1 = v.i.off[i1] - 1, k2 = 0, rem = 0;
+    const int jbeg = v.j.off[j1];
+    double2 A1 = make_double2(0.0, 0.0), B1 = A1;
+    const double *strow = v.st;
+    for (int left = v.tot[ap]; left > 0; --left) {
+        while (rem == 0) {  // the next run that holds a term
+            const int w = *win;
+            win += nap;
+            ++k1;
+            rem = w >> 8;
+            k2 = jbeg + (w & 0xff);
+            A1 = v.i.A[k1];
+            B1 = v.i.B[k1];
+            strow = v.st + v.i.C[k1] * F6_SST;
+        }
+        const double2 A2 = v.j.A[k2];
+        const double dr = __dsub_rn(A2.x, A1.x);
+        const double t = __dmul_rn(dr, dr);
+        if (!kTest || t < P.maxg2)
+            sum = __dadd_rn(sum, f64_term(t, P.inv_width, A1, B1, A2, v.j.B[k2],
+                                          strow[v.j.C[k2]]));
+        ++k2;
+        --rem;
+    }
+    return sum;
+}
+
+// bm x bm molecule block per CTA.
+__global__ void __launch_bounds__(F6_TPB, 4)
+arad_f64_pair_kernel(const double *__restrict__ X1, SetWs w1, const int *__restrict__ N1, int nm1,
+                     const double *__restrict__ X2, SetWs w2, const int *__restrict__ N2, int nm2,
+                     int amax, AradParams P, const ClassInfo *ci,
+                     const __grid_constant__ SigmaTable sig, int nsig, int symmetric, int bm,
+                     double *__restrict__ K) {
+    extern __shared__ __align__(16) unsigned char fc_smem_raw[];
+    if (ci->flag) return;
+    const F64View v = f64_view(fc_smem_raw, amax);
+    int bi, bj;
+    pair_block(blockIdx.x, symmetric, (nm2 + bm - 1) / bm, bi, bj);
+    f64_load_table(v.st, ci);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    for (int il = 0; il < bm; ++il) {
+        const int I = bi * bm + il;
+        if (I >= nm1) break;
+        const int nI = min(max(N1[I], 0), amax);
+        __syncthreads();  // the previous pair is done with shared memory
+        f64_load(v.i, X1, w1, I, amax, nI, true);
+        for (int jl = 0; jl < bm; ++jl) {
+            const int J = bj * bm + jl;
+            if (J >= nm2) break;
+            if (symmetric && J < I) continue;
+            const int nJ = min(max(N2[J], 0), amax);
+            __syncthreads();
+            f64_load(v.j, X2, w2, J, amax, nJ, true);
+            const int jstep = nI > 0 ? F6_WIN / (nI * nI) : FC_MAXA;
+            for (int j0 = 0; j0 < nJ; j0 += jstep) {
+                const int jn = min(jstep, nJ - j0), nap = nI * jn;
+                if (tid < F6_BUCKETS) v.bucket[tid] = 0;
+                __syncthreads();
+                // 1. the runs; atom pair ap = (j1 - j0) nI + i1, a thread each. Both
+                // ends of the window only move up while r1 ascends.
+                for (int ap = tid; ap < nap; ap += F6_TPB) {
+                    const int jq = ap / nI, i1 = ap - jq * nI, j1 = j0 + jq;
+                    const double2 *J2 = v.j.A + v.j.off[j1];
+                    const int cnt = v.j.off[j1 + 1] - v.j.off[j1], k1 = v.i.off[i1];
+                    const bool ascends = v.j.asc[j1] != 0;
+                    int lo = 0, hi = ascends ? 0 : cnt, total = 0;
+                    double before = 0.0;
+                    for (int m1 = 0; m1 < v.i.off[i1 + 1] - k1; ++m1) {
+                        const double r1 = v.i.A[k1 + m1].x;
+                        if (ascends) {
+                            if (!(r1 >= before)) lo = hi = 0;
+                            before = r1;
+                            while (lo < cnt) {  // to the first neighbour not below the window
+                                const double dr = __dsub_rn(J2[lo].x, r1);
+                                if (!(dr < 0.0) || __dmul_rn(dr, dr) < P.maxg2) break;
+                                ++lo;
+                            }
+                            hi = max(hi, lo);
+                            while (hi < cnt) {  // to the first neighbour above it
+                                const double dr = __dsub_rn(J2[hi].x, r1);
+                                if (!(dr < 0.0) && !(__dmul_rn(dr, dr) < P.maxg2)) break;
+                                ++hi;
+                            }
+                        }
+                        v.win[m1 * nap + ap] = (unsigned short)(lo | ((hi - lo) << 8));
+                        total += hi - lo;
+                    }
+                    v.tot[ap] = total;
+                }
+                const bool test = __syncthreads_or(tid < jn && !v.j.asc[j0 + tid]);
+                // 2. atom pairs by number of terms, largest first (which lane
+                // takes a pair does not change its sum)
+                auto bucket_of = [&](int ap) {
+                    return F6_BUCKETS - 1 -
+                           min(F6_BUCKETS - 1, v.tot[ap] * F6_BUCKETS / (nI * nJ));
+                };
+                for (int t = tid; t < nap; t += F6_TPB) atomicAdd(&v.bucket[bucket_of(t)], 1);
+                __syncthreads();
+                if (warp == 0) {  // exclusive prefix over the 64 buckets
+                    const int b0 = v.bucket[2 * lane], b1 = v.bucket[2 * lane + 1];
+                    int incl = b0 + b1;
+                    for (int d = 1; d < 32; d <<= 1) {
+                        const int o = __shfl_up_sync(0xffffffffu, incl, d);
+                        if (lane >= d) incl += o;
+                    }
+                    v.bucket[2 * lane] = incl - b0 - b1;
+                    v.bucket[2 * lane + 1] = incl - b1;
+                }
+                __syncthreads();
+                for (int t = tid; t < nap; t += F6_TPB)
+                    v.perm[atomicAdd(&v.bucket[bucket_of(t)], 1)] = (unsigned short)t;
+                __syncthreads();
+                // 3. the sums and l2
+                for (int t = tid; t < nap; t += F6_TPB) {
+                    const int ap = v.perm[t], jq = ap / nI, i1 = ap - jq * nI, j1 = j0 + jq;
+                    const double S = test ? f64_pair_sum<true>(v, i1, j1, ap, nap, P)
+                                          : f64_pair_sum<false>(v, i1, j1, ap, nap, P);
+                    const double stz = v.st[v.i.acls[i1] * F6_SST + v.j.acls[j1]];
+                    double l2 = __dsub_rn(__dadd_rn(v.i.self[i1], v.j.self[j1]),
+                                          __dmul_rn(__dmul_rn(2.0, S), stz));
+                    if (fabs(l2) < P.eps) l2 = 0.0;  // farad_kernels.f90:594
+                    v.l2[j0 * nI + ap] = l2;
+                }
+                __syncthreads();
+            }
+            const int nall = nI * nJ;
+            // 4. the kernel exponentials
+            for (int s = 0; s < nsig; ++s) {
+                double e = 0.0;
+                for (int t = tid; t < nall; t += F6_TPB) e += exp(v.l2[t] * sig.inv_sigma2[s]);
+                for (int o = 16; o; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+                if (lane == 0) v.red[warp * MAXSIG + s] = e;
+            }
+            __syncthreads();
+            if (tid < nsig) {
+                double e = 0.0;
+                for (int q = 0; q < F6_TPB / 32; ++q) e += v.red[q * MAXSIG + tid];
+                K[((size_t)tid * nm1 + I) * nm2 + J] = e;
+                if (symmetric) K[((size_t)tid * nm1 + J) * nm2 + I] = e;
+            }
+        }
+    }
+}
+
+// Molecule block of the FP64 pair kernel: 2 x 2 once the blocks fill the GPU
+// several times over (each molecule is then staged for two pairs), else one
+// pair per CTA.
+inline int f64_block(long long npairs) { return npairs >= (1LL << 13) ? 2 : 1; }
+
 // The fast kernels' shared memory is dynamic (above the 48 KB static limit);
 // the attribute is set once per device.
 int fast_smem_attrs() {
@@ -920,6 +1294,14 @@ int fast_smem_attrs() {
                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)sizeof(FastSmem)),
                          "fmlb_arad_kernels: pair kernel smem attribute"));
+    FMLB_TRY(cuda_status(cudaFuncSetAttribute(arad_f64_self_kernel,
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)f64_self_smem_bytes(FC_MAXA)),
+                         "fmlb_arad_kernels: FP64 self kernel smem attribute"));
+    FMLB_TRY(cuda_status(cudaFuncSetAttribute(arad_f64_pair_kernel,
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)f64_smem_bytes(FC_MAXA)),
+                         "fmlb_arad_kernels: FP64 pair kernel smem attribute"));
     attr_dev = dev;
     return FMLB_OK;
 }
@@ -1114,46 +1496,51 @@ static int arad_kernels_impl(const double *X1, const double *Z1, const int *N1, 
     SetWs w2 = symmetric ? w1 : carve(p, nm2, amax);
     ClassInfo *ci = reinterpret_cast<ClassInfo *>(p);
     const int tpb = 128;
-    {
-        const long long n = (long long)nm1 * amax;
-        arad_prep_kernel<<<ceil_div(n, tpb), tpb, 0, st>>>(X1, N1, nm1, amax, P, symmetric ? 0 : 1,
-                                                           w1);
-        FMLB_TRY(launch_status("arad_prep_kernel"));
-    }
-    if (!symmetric) {
-        const long long n = (long long)nm2 * amax;
-        arad_prep_kernel<<<ceil_div(n, tpb), tpb, 0, st>>>(X2, N2, nm2, amax, P, 1, w2);
-        FMLB_TRY(launch_status("arad_prep_kernel"));
-    }
-    // fast FP32 path: amax <= 32 and at most 16 element classes (decided on the device)
-    const bool try_fast = precision == 1 && amax <= FC_MAXA;
-    if (try_fast) {
+    // fast paths: amax <= 32 and at most 16 element classes (decided on the device)
+    const bool try_fast = amax <= FC_MAXA;
+    ClassInfo *fast_ci = try_fast ? ci : nullptr;
+    if (try_fast)
         FMLB_TRY(cuda_status(cudaMemsetAsync(ci, 0, sizeof(ClassInfo), st), "clear class info"));
-        arad_class_scan_kernel<<<ceil_div((long long)nm1 * amax, tpb), tpb, 0, st>>>(
-            X1, Z1, N1, nm1, amax, P.cut, ci);
-        if (!symmetric)
-            arad_class_scan_kernel<<<ceil_div((long long)nm2 * amax, tpb), tpb, 0, st>>>(
-                X2, Z2, N2, nm2, amax, P.cut, ci);
-        arad_class_build_kernel<<<1, 1, 0, st>>>(ci, P.rw2, P.cw2);
-        arad_class_assign_kernel<<<ceil_div((long long)nm1 * amax, tpb), tpb, 0, st>>>(
-            X1, Z1, N1, nm1, amax, ci, w1);
-        if (!symmetric)
-            arad_class_assign_kernel<<<ceil_div((long long)nm2 * amax, tpb), tpb, 0, st>>>(
-                X2, Z2, N2, nm2, amax, ci, w2);
+    struct Set {
+        const double *X, *Z;
+        const int *N;
+        int nm;
+        SetWs w;
+    } sets[2] = {{X1, Z1, N1, nm1, w1}, {X2, Z2, N2, nm2, w2}};
+    const int nsets = symmetric ? 1 : 2;
+    for (int q = 0; q < nsets; ++q) {
+        const Set &s = sets[q];
+        arad_prep_kernel<<<ceil_div((long long)s.nm * amax, PREP_WARPS), PREP_WARPS * 32, 0, st>>>(
+            s.X, s.Z, s.N, s.nm, amax, P, symmetric ? 0 : 1, s.w, fast_ci);
+        FMLB_TRY(launch_status("arad_prep_kernel"));
+    }
+    if (try_fast) {
         FMLB_TRY(fast_smem_attrs());
-        arad_sort_records_kernel<<<nm1, FC_WARPS * 32, 0, st>>>(w1, N1, nm1, amax, ci);
-        if (!symmetric)
-            arad_sort_records_kernel<<<nm2, FC_WARPS * 32, 0, st>>>(w2, N2, nm2, amax, ci);
-        arad_fast_self_kernel<<<nm1, FC_WARPS * 32, sizeof(FastSmem), st>>>(w1, N1, nm1, amax, P,
-                                                                            ci);
-        if (!symmetric)
-            arad_fast_self_kernel<<<nm2, FC_WARPS * 32, sizeof(FastSmem), st>>>(w2, N2, nm2, amax,
-                                                                                P, ci);
+        arad_class_build_kernel<<<1, CB_TPB, 0, st>>>(ci, P.rw2, P.cw2);
+        for (int q = 0; q < nsets; ++q) {
+            const Set &s = sets[q];
+            arad_class_assign_kernel<<<ceil_div((long long)s.nm * amax * amax, 256), 256, 0, st>>>(
+                s.X, s.Z, s.N, s.nm, amax, ci, s.w);
+            if (precision == 1) {
+                arad_sort_records_kernel<<<s.nm, FC_WARPS * 32, 0, st>>>(s.w, s.N, s.nm, amax, ci);
+                arad_fast_self_kernel<<<s.nm, FC_WARPS * 32, sizeof(FastSmem), st>>>(
+                    s.w, s.N, s.nm, amax, P, ci);
+            } else {
+                arad_f64_self_kernel<<<s.nm, 32, f64_self_smem_bytes(amax), st>>>(
+                    s.X, s.w, s.N, s.nm, amax, P, ci);
+            }
+        }
         FMLB_TRY(launch_status("arad fast-path preparation"));
+    }
+    for (int q = 0; q < nsets; ++q) {
+        const Set &s = sets[q];
+        arad_generic_self_kernel<<<ceil_div((long long)s.nm * amax, tpb), tpb, 0, st>>>(
+            s.X, s.N, s.nm, amax, P, s.w, fast_ci);
+        FMLB_TRY(launch_status("arad_generic_self_kernel"));
     }
     const long long npairs = symmetric ? (long long)nm1 * (nm1 + 1) / 2 : (long long)nm1 * nm2;
     const int blocks = (int)std::min<long long>(ceil_div(npairs, tpb / 32), (long long)sm_count() * 64);
-    const int chunk = try_fast ? FC_MAXSIG : MAXSIG;
+    const int chunk = try_fast && precision == 1 ? FC_MAXSIG : MAXSIG;
     for (int s0 = 0; s0 < nsigma; s0 += chunk) {
         const int ns = nsigma - s0 < chunk ? nsigma - s0 : chunk;
         SigmaTable sig;
@@ -1161,8 +1548,18 @@ static int arad_kernels_impl(const double *X1, const double *Z1, const int *N1, 
             sig.inv_sigma2[s] = -1.0 / (sigmas_host[s0 + s] * sigmas_host[s0 + s]);
         double *Ks = K + (size_t)s0 * nm1 * nm2;
         if (precision == 0) {
+            if (try_fast) {
+                const int bm = f64_block(npairs);
+                const long long nbi = ceil_div(nm1, bm), nbj = ceil_div(nm2, bm);
+                const long long nblk = symmetric ? nbi * (nbi + 1) / 2 : nbi * nbj;
+                FMLB_REQUIRE(nblk < (1LL << 31), "fmlb_arad_kernels: too many molecule blocks");
+                arad_f64_pair_kernel<<<(unsigned)nblk, F6_TPB, f64_smem_bytes(amax), st>>>(
+                    X1, w1, N1, nm1, X2, w2, N2, nm2, amax, P, ci, sig, ns, symmetric, bm, Ks);
+                FMLB_TRY(launch_status("arad_f64_pair_kernel"));
+            }
             arad_pair_kernel<true><<<blocks, tpb, 0, st>>>(X1, Z1, N1, w1, nm1, X2, Z2, N2, w2, nm2,
-                                                           amax, P, sig, ns, symmetric, Ks, nullptr);
+                                                           amax, P, sig, ns, symmetric, Ks,
+                                                           fast_ci);
         } else {
             if (try_fast) {
                 const long long nbi = ceil_div(nm1, FC_BM), nbj = ceil_div(nm2, FC_BM);
@@ -1174,7 +1571,7 @@ static int arad_kernels_impl(const double *X1, const double *Z1, const int *N1, 
             }
             arad_pair_kernel<false><<<blocks, tpb, 0, st>>>(X1, Z1, N1, w1, nm1, X2, Z2, N2, w2,
                                                             nm2, amax, P, sig, ns, symmetric, Ks,
-                                                            try_fast ? ci : nullptr);
+                                                            fast_ci);
         }
         FMLB_TRY(launch_status("arad_pair_kernel"));
     }
@@ -1242,12 +1639,17 @@ extern "C" int fmlb_arad_distances(const double *X1, const double *Z1, const int
     SetWs w1 = carve(p, nm1, amax);
     SetWs w2 = carve(p, nm2, amax);
     const int tpb = 128;
-    arad_prep_kernel<<<ceil_div((long long)nm1 * amax, tpb), tpb, 0, st>>>(X1, N1, nm1, amax, P,
-                                                                           0, w1);
-    FMLB_TRY(launch_status("arad_prep_kernel"));
-    arad_prep_kernel<<<ceil_div((long long)nm2 * amax, tpb), tpb, 0, st>>>(X2, N2, nm2, amax, P,
-                                                                           0, w2);
-    FMLB_TRY(launch_status("arad_prep_kernel"));
+    for (int q = 0; q < 2; ++q) {
+        const double *X = q ? X2 : X1, *Z = q ? Z2 : Z1;
+        const int *N = q ? N2 : N1, nm = q ? nm2 : nm1;
+        const SetWs &w = q ? w2 : w1;
+        arad_prep_kernel<<<ceil_div((long long)nm * amax, PREP_WARPS), PREP_WARPS * 32, 0, st>>>(
+            X, Z, N, nm, amax, P, 0, w, nullptr);
+        FMLB_TRY(launch_status("arad_prep_kernel"));
+        arad_generic_self_kernel<<<ceil_div((long long)nm * amax, tpb), tpb, 0, st>>>(
+            X, N, nm, amax, P, w, nullptr);
+        FMLB_TRY(launch_status("arad_generic_self_kernel"));
+    }
     FMLB_TRY(cuda_status(cudaMemsetAsync(D, 0, sizeof(double) * nm1 * nm2 * amax * amax, st),
                          "fmlb_arad_distances: clear D"));
     const long long npairs = (long long)nm1 * nm2;

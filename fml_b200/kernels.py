@@ -217,11 +217,12 @@ def _arad(X1, X2, Z1, Z2, sigmas, width, cut_distance, r_width, c_width, symmetr
 
 def arad_launches(symmetric, precision, amax, nsigma):
     """Kernel launches of one ``fmlb_arad_kernels`` call (mirrors its host code)."""
-    fast = precision == "fp32" and amax <= 32
     sets = 1 if symmetric else 2
-    if fast:  # prep, class scan, assign, record sort, self per set; class build; fast + gated
-        return 5 * sets + 1 + 2 * -(-nsigma // 8)  # generic pair per sigma chunk
-    return sets + -(-nsigma // 16)
+    chunks = -(-nsigma // (8 if precision == "fp32" and amax <= 32 else 16))
+    if amax <= 32:  # prep, class assign, self, gated generic self (FP32: record sort) per set;
+        # class build; fast + gated generic pair per sigma chunk
+        return (5 if precision == "fp32" else 4) * sets + 1 + 2 * chunks
+    return 2 * sets + chunks
 
 
 def _atomic_inputs(q1a, q2a, z1, z2, n1, n2):
