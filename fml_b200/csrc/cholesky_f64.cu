@@ -7,16 +7,18 @@
 // argument this is its dpotrf('U') factor U = L^T.
 //
 // Two levels of blocking. Inner panels of NB = 128 columns:
-//   1. potf2 + inversion of the diagonal block in shared memory (one CTA); a
+//   1. potf2 of the diagonal block in shared memory (one CTA), with the inverses
+//      of its 32 x 32 diagonal sub-blocks; a
 //      non-positive pivot records the LAPACK info (1-based column) and every
 //      later kernel of the factorisation returns at once;
-//   2. panel solve L21 = A21 L11^-T as a product with the stored inverse;
+//   2. panel solve L21 = A21 L11^-T by 32-column blocks with those inverses;
 // outer panels of 256, 512 or 1024 columns (wider at larger n):
 //   3. trailing update A22 -= L21 L21^T with k = the outer width, on the FP64
 //      tensor cores (mma.sync m8n8k4 f64), 128x64 tiles on or below the
 //      diagonal, operands streamed through a 3-stage cp.async pipeline;
 // with the next outer panel factored on a second stream under step 3.
-// The inverted diagonal blocks stay in the workspace for the solve (section 4).
+// The inverses of the 128 x 128 diagonal blocks, formed at the end for all
+// blocks side by side, stay in the workspace for the solve (section 4).
 #include <math.h>
 #include <stdint.h>
 
@@ -51,85 +53,80 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 
 // ---- 1. diagonal block ----------------------------------------------------
 // The 128 x 128 block is factored in four 32-column steps. In step J one warp
-// factors (and inverts) the 32 x 32 diagonal sub-block in registers with warp
+// factors and inverts the 32 x 32 diagonal sub-block in registers with warp
 // shuffles only; the whole CTA then solves the 32-column sub-panel below it
-// and updates the rest of the block. The block inverse is assembled from the
-// sub-block inverses: inv(L)_IJ = -inv(L_II) sum_{K=J}^{I-1} L_IK inv(L)_KJ,
-// with the off-diagonal blocks kept (transposed) in the unused upper triangle.
-constexpr int LDL = NB + 1;
-constexpr int SB = 32, NSB = NB / SB, LDW = SB + 1;
-constexpr size_t kPotf2Smem =
-    ((size_t)NB * LDL + (size_t)NSB * SB * LDW + (size_t)(NSB - 1) * SB * LDW) * sizeof(double);
+// (a product with the sub-block's inverse) and updates the rest of the block,
+// both on the FP64 tensor cores. Only the four 32 x 32 inverses are formed
+// here: the panel solve needs no more, and the block inverses of the triangular
+// solves come from block_inverse_kernel, once, for all blocks side by side.
+//
+// Bound by the latency of the 128 serial pivots. With factor and inverse in
+// separate passes, each a shuffle per entry and a division per column, the
+// block products as shared-memory FMA loops and the whole inverse assembled on
+// this path, a block took 190 us.
+constexpr int LDL = NB + 4;  // row pitch: the fragments' rows fall in distinct banks
+constexpr int SB = 32, NSB = NB / SB, LDW = SB + 4;
+constexpr size_t kPotf2Smem = ((size_t)NB * LDL + (size_t)SB * LDW) * sizeof(double);
 
-// One warp factors the 32 x 32 diagonal sub-block at L[b0.., b0..] in place
-// and writes its inverse into W (row-major). Lane r holds row r of the block
-// in registers; the entries other lanes need come by shuffles. The column
-// steps are unrolled by template recursion, so every register index is a
-// constant. The arithmetic (order of the FMAs, reciprocal-multiply scaling,
-// the division in the substitution) is that of right-looking elimination
-// and forward substitution in shared memory, bit for bit.
+__device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                 : "+d"(d[0]), "+d"(d[1])
+                 : "d"(a), "d"(b));
+}
+
+// One warp factors the 32 x 32 diagonal sub-block and inverts the factor. Lane
+// r holds row r of the block (a) and column r of the inverse (v) in registers;
+// the column steps are unrolled by template recursion, so every register index
+// is a constant. A step scales column J by 1 / sqrt(pivot) and then, from one
+// shuffle per entry L[c][J], updates both the rest of the block and the
+// inverse's forward substitution (right-looking): two independent FMA streams
+// that cover each other's and the next pivot's latency. Entries above the
+// diagonal hold values that nothing reads.
 template <int J>
-struct WarpFactor32 {
-    __device__ __forceinline__ static void run(double (&a)[SB], int lane, int &fail) {
+struct WarpFactorInvert32 {
+    __device__ __forceinline__ static void run(double (&a)[SB], double (&v)[SB], int lane,
+                                               int &fail) {
         const double piv = __shfl_sync(0xffffffffu, a[J], J);
         if (!(piv > 0.0) && !fail) fail = J + 1;  // later columns are NaN and not stored
-        const double r = sqrt(piv), inv = 1.0 / r;
-        if (lane == J) a[J] = r;
-        else if (lane > J) a[J] *= inv;
-        const double lij = a[J];
+        const double inv = rsqrt(piv);
+        double root = piv * inv;  // sqrt(piv), corrected once
+        root = fma(0.5 * inv, fma(-root, root, piv), root);
+        a[J] = lane == J ? root : a[J] * inv;
+        v[J] *= inv;
+        const double lij = a[J], vj = v[J];
 #pragma unroll
         for (int c = J + 1; c < SB; ++c) {
-            const double lcj = __shfl_sync(0xffffffffu, a[J], c);  // L[c][J]
-            if (c <= lane) a[c] = fma(-lij, lcj, a[c]);
+            const double lcj = __shfl_sync(0xffffffffu, lij, c);  // L[c][J]
+            a[c] = fma(-lij, lcj, a[c]);
+            v[c] = fma(-lcj, vj, v[c]);
         }
-        WarpFactor32<J + 1>::run(a, lane, fail);
+        WarpFactorInvert32<J + 1>::run(a, v, lane, fail);
     }
 };
 template <>
-struct WarpFactor32<SB> {
-    __device__ __forceinline__ static void run(double (&)[SB], int, int &) {}
-};
-// Column `lane` of the inverse by forward substitution, right-looking: once
-// w[K] = W[K][lane] is final it is subtracted from every later row's sum, so
-// the serial chain per step is one division and one FMA. Each row's sum takes
-// its terms in ascending column order, as the left-looking loop does; v[K]
-// holds that sum until step K turns it into w[K].
-template <int K>
-struct WarpInverse32 {
-    __device__ __forceinline__ static void run(const double (&a)[SB], double (&v)[SB], int lane) {
-        const double lkk = __shfl_sync(0xffffffffu, a[K], K);
-        v[K] = (K < lane) ? 0.0 : v[K] / lkk;
-#pragma unroll
-        for (int r = K + 1; r < SB; ++r) {
-            const double lrk = __shfl_sync(0xffffffffu, a[K], r);  // L[r][K]
-            if (K >= lane) v[r] = fma(-lrk, v[K], v[r]);
-        }
-        WarpInverse32<K + 1>::run(a, v, lane);
-    }
-};
-template <>
-struct WarpInverse32<SB> {
-    __device__ __forceinline__ static void run(const double (&)[SB], double (&)[SB], int) {}
+struct WarpFactorInvert32<SB> {
+    __device__ __forceinline__ static void run(double (&)[SB], double (&)[SB], int, int &) {}
 };
 
-// Returns the 1-based failing column or 0 (the same value in every lane).
-__device__ __forceinline__ int warp_potrf_inv32(double (*L)[NB + 1], int b0, double (*W)[SB + 1]) {
+// Factors the sub-block at L[b0.., b0..] in place and writes its inverse into W
+// (row-major, zeros above the diagonal). Returns the 1-based failing column or
+// 0 (the same value in every lane).
+__device__ __forceinline__ int warp_potrf_inv32(double (*L)[LDL], int b0, double (*W)[LDW]) {
     const int lane = threadIdx.x & 31;
-    double a[SB];
+    double a[SB], v[SB];
 #pragma unroll
-    for (int c = 0; c < SB; ++c) a[c] = c <= lane ? L[b0 + lane][b0 + c] : 0.0;
+    for (int c = 0; c < SB; ++c) {
+        a[c] = c <= lane ? L[b0 + lane][b0 + c] : 0.0;
+        v[c] = c == lane ? 1.0 : 0.0;
+    }
     int fail = 0;
-    WarpFactor32<0>::run(a, lane, fail);
+    WarpFactorInvert32<0>::run(a, v, lane, fail);
     if (fail) return fail;
 #pragma unroll
-    for (int c = 0; c < SB; ++c)
+    for (int c = 0; c < SB; ++c) {
         if (c <= lane) L[b0 + lane][b0 + c] = a[c];
-    double w[SB];
-#pragma unroll
-    for (int k = 0; k < SB; ++k) w[k] = (k == lane) ? 1.0 : 0.0;
-    WarpInverse32<0>::run(a, w, lane);
-#pragma unroll
-    for (int k = 0; k < SB; ++k) W[k][lane] = w[k];
+        W[c][lane] = v[c];
+    }
     __syncwarp();
     return 0;
 }
@@ -139,14 +136,12 @@ potf2_block_kernel(double *__restrict__ A, long long lda, int k0, int kn,
                    double *__restrict__ Linv, int *__restrict__ info) {
     extern __shared__ double potf2_smem[];
     double(*L)[LDL] = reinterpret_cast<double(*)[LDL]>(potf2_smem);
-    double(*W)[SB][LDW] = reinterpret_cast<double(*)[SB][LDW]>(potf2_smem + NB * LDL);
-    // T[J]: sum_{K=J}^{I-1} L_IK inv(L)_KJ for every J < I of one block row I
-    double(*T)[SB][LDW] =
-        reinterpret_cast<double(*)[SB][LDW]>(potf2_smem + NB * LDL + NSB * SB * LDW);
+    double(*W)[LDW] = reinterpret_cast<double(*)[LDW]>(potf2_smem + NB * LDL);
     __shared__ int bad;
     pdl_wait();
     if (failed(info)) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int g = lane >> 2, tq = lane & 3;  // fragment row / k (A, B), row / column pair (C)
     for (int t = tid; t < NB * NB; t += TPB) {
         const int r = t >> 7, c = t & (NB - 1);
         double v = 0.0;
@@ -157,9 +152,9 @@ potf2_block_kernel(double *__restrict__ A, long long lda, int k0, int kn,
     if (tid == 0) bad = 0;
     __syncthreads();
     for (int J = 0; J < NSB; ++J) {
-        const int b0 = J * SB;
+        const int b0 = J * SB, r0 = b0 + SB;
         if (warp == 0) {
-            const int f = warp_potrf_inv32(L, b0, W[J]);
+            const int f = warp_potrf_inv32(L, b0, W);
             if (f && lane == 0) bad = b0 + f;
         }
         __syncthreads();
@@ -167,37 +162,44 @@ potf2_block_kernel(double *__restrict__ A, long long lda, int k0, int kn,
             if (tid == 0) atomicCAS(info, 0, k0 + bad);
             return;
         }
-        const int r0 = b0 + SB;
-        // sub-panel solve: L[r][b0..b0+31] <- L[r][b0..] inv(D)^T, one row per thread
-        for (int r = r0 + tid; r < NB; r += TPB) {
-            double a[SB];
+        // the sub-block's inverse to its place in the block inverse
+        for (int t = tid; t < SB * SB; t += TPB)
+            Linv[(size_t)(b0 + t / SB) * NB + b0 + t % SB] = W[t / SB][t % SB];
+        // sub-panel solve, 8 rows per warp and turn: X <- X inv(D)^T
+        for (int m = r0 + warp * 8; m < NB; m += 8 * (TPB / 32)) {
+            double x[SB / 4], o[SB / 8][2];
 #pragma unroll
-            for (int k = 0; k < SB; ++k) a[k] = L[r][b0 + k];
+            for (int k = 0; k < SB / 4; ++k) x[k] = L[m + g][b0 + 4 * k + tq];
 #pragma unroll
-            for (int c = 0; c < SB; ++c) {
-                double sacc = 0.0;
+            for (int c = 0; c < SB / 8; ++c) {
+                o[c][0] = o[c][1] = 0.0;
 #pragma unroll
-                for (int k = 0; k <= c; ++k) sacc = fma(a[k], W[J][c][k], sacc);
-                L[r][b0 + c] = sacc;
+                for (int k = 0; k < 2 * c + 2; ++k)  // inv(D) is lower triangular
+                    dmma_8x8x4(o[c], x[k], W[8 * c + g][4 * k + tq]);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < SB / 8; ++c) {
+                L[m + g][b0 + 8 * c + 2 * tq] = o[c][0];
+                L[m + g][b0 + 8 * c + 2 * tq + 1] = o[c][1];
             }
         }
         __syncthreads();
-        // update of the rest of the block: L[r][c] -= sum_k X[r][k] X[c][k], r0 <= c <= r;
-        // two columns per step, so two independent FMA chains share the row loads
-        for (int r = r0 + (tid >> 4); r < NB; r += TPB / 16) {
-            for (int c = r0 + (tid & 15); c <= r; c += 32) {
-                const bool two = c + 16 <= r;
-                const int c2 = two ? c + 16 : c;
-                double s0 = 0.0, s1 = 0.0;
-#pragma unroll 8
-                for (int k = 0; k < SB; ++k) {
-                    const double x = L[r][b0 + k];
-                    s0 = fma(x, L[c][b0 + k], s0);
-                    s1 = fma(x, L[c2][b0 + k], s1);
-                }
-                L[r][c] -= s0;
-                if (two) L[r][c2] -= s1;
+        // update of the rest of the block, 8 x 8 tiles on or below the diagonal
+        const int nt = (NB - r0) / 8;
+        for (int t = warp; t < nt * (nt + 1) / 2; t += TPB / 32) {
+            int ti = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
+            while (ti * (ti + 1) / 2 > t) --ti;
+            while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
+            const int m = r0 + 8 * ti, c = r0 + 8 * (t - ti * (ti + 1) / 2);
+            double o0[2] = {0.0, 0.0}, o1[2] = {0.0, 0.0};
+#pragma unroll
+            for (int k = 0; k < SB; k += 8) {
+                dmma_8x8x4(o0, L[m + g][b0 + k + tq], L[c + g][b0 + k + tq]);
+                dmma_8x8x4(o1, L[m + g][b0 + k + 4 + tq], L[c + g][b0 + k + 4 + tq]);
             }
+            L[m + g][c + 2 * tq] -= o0[0] + o1[0];
+            L[m + g][c + 2 * tq + 1] -= o0[1] + o1[1];
         }
         __syncthreads();
     }
@@ -206,67 +208,168 @@ potf2_block_kernel(double *__restrict__ A, long long lda, int k0, int kn,
         const int r = t >> 7, c = t & (NB - 1);
         if (r < kn && c <= r) A[(size_t)(k0 + r) * lda + (k0 + c)] = L[r][c];
     }
-    // block inverse; inv(L)_IJ for I > J is stored transposed at L[b0J + c][b0I + r].
-    // Block row I needs the rows before it only, so its J < I blocks are formed
-    // together: T[J] for every J, then inv(L)_IJ = -inv(L_II) T[J].
-    // Thread tid forms, for every J, the four rows r = tid / 32 + 8 i of column
-    // c = tid % 32: the column operand is loaded once for four independent FMA
-    // chains (each entry's sum in the same order as one chain per entry).
-    static_assert(TPB == 8 * SB, "four rows per thread and column block");
-    const int rq = tid >> 5, cq = tid & 31;
-    for (int I = 1; I < NSB; ++I) {
-        for (int J = 0; J < I; ++J) {
-            double sacc[4] = {0.0, 0.0, 0.0, 0.0};
-            for (int K = J; K < I; ++K) {
-                for (int q = 0; q < SB; ++q) {
-                    const double inv = (K == J) ? W[J][q][cq] : L[J * SB + cq][K * SB + q];
+    pdl_launch_dependents();
+}
+
+// ---- 2. panel solve: rows [r0, n) of columns [k0, k0+kn): X <- X L11^-T ----
+// Forward substitution by 32-column blocks on the FP64 tensor cores: X_J <-
+// (X_J - sum_{K < J} X_K L_JK^T) W_J^T with the factored diagonal block and its
+// 32 x 32 inverses W_J. Chunks of 32 rows, one CTA per SM taking them in turn
+// with the diagonal block kept in shared memory; warp w owns 8 rows and 16 of
+// each block's 32 columns.
+constexpr int TRSM_ROWS = 32;
+constexpr int TRSM_BLK = SB * LDW;  // doubles of a 32 x 32 block of the lower triangle
+constexpr size_t kTrsmSmem =
+    ((size_t)TRSM_ROWS * LDL + (size_t)NSB * (NSB + 1) / 2 * TRSM_BLK) * sizeof(double);
+
+__global__ void __launch_bounds__(TPB)
+panel_trsm_kernel(double *__restrict__ A, long long lda, int n, int k0,
+                  const double *__restrict__ Linv, const int *__restrict__ info) {
+    extern __shared__ double trsm_smem[];
+    double(*X)[LDL] = reinterpret_cast<double(*)[LDL]>(trsm_smem);
+    double *blocks = trsm_smem + TRSM_ROWS * LDL;  // (R, C) at R (R + 1) / 2 + C
+    pdl_wait();
+    if (failed(info)) return;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int g = lane >> 2, tq = lane & 3;
+    for (int t = tid; t < NB * NB; t += TPB) {
+        const int r = t / NB, c = t % NB, R = r / SB, C = c / SB;
+        if (C <= R)
+            blocks[(R * (R + 1) / 2 + C) * TRSM_BLK + (r % SB) * LDW + c % SB] =
+                C == R ? Linv[t] : A[(size_t)(k0 + r) * lda + k0 + c];
+    }
+    const int m = (warp & 3) * 8, h = (warp >> 2) * 16;  // rows m.., columns h.. of each block
+    for (int r0 = k0 + NB + blockIdx.x * TRSM_ROWS; r0 < n; r0 += gridDim.x * TRSM_ROWS) {
+        for (int t = tid; t < TRSM_ROWS * NB; t += TPB) {
+            const int r = t / NB, c = t % NB;
+            X[r][c] = r0 + r < n ? A[(size_t)(r0 + r) * lda + k0 + c] : 0.0;
+        }
+        for (int J = 0; J < NSB; ++J) {
+            const double *row = blocks + J * (J + 1) / 2 * TRSM_BLK + (h + g) * LDW + tq;
+            __syncthreads();
+            double o[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+            for (int K = 0; K < J; ++K) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        sacc[i] = fma(L[I * SB + rq + 8 * i][K * SB + q], inv, sacc[i]);
+                for (int k = 0; k < SB; k += 4) {
+                    const double x = X[m + g][K * SB + k + tq];
+#pragma unroll
+                    for (int c = 0; c < 2; ++c)
+                        dmma_8x8x4(o[c], x, row[K * TRSM_BLK + 8 * c * LDW + k]);
                 }
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) T[J][rq + 8 * i][cq] = sacc[i];
-        }
-        __syncthreads();
-        for (int J = 0; J < I; ++J) {
-            double sacc[4] = {0.0, 0.0, 0.0, 0.0};
-            for (int q = 0; q <= rq + 24; ++q) {
-                const double tq = T[J][q][cq];
+            for (int c = 0; c < 2; ++c)
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (q <= rq + 8 * i) sacc[i] = fma(W[I][rq + 8 * i][q], tq, sacc[i]);
+                for (int q = 0; q < 2; ++q) X[m + g][J * SB + h + 8 * c + 2 * tq + q] -= o[c][q];
+            __syncthreads();
+            o[0][0] = o[0][1] = o[1][0] = o[1][1] = 0.0;
+            for (int k = 0; k < h + 16; k += 4) {  // W_J is lower triangular
+                const double x = X[m + g][J * SB + k + tq];
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+                    dmma_8x8x4(o[c], x, row[J * TRSM_BLK + 8 * c * LDW + k]);
             }
+            __syncthreads();
 #pragma unroll
-            for (int i = 0; i < 4; ++i) L[J * SB + cq][I * SB + rq + 8 * i] = -sacc[i];
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) X[m + g][J * SB + h + 8 * c + 2 * tq + q] = o[c][q];
         }
         __syncthreads();
-    }
-    for (int t = tid; t < NB * NB; t += TPB) {
-        const int r = t >> 7, c = t & (NB - 1);
-        const int I = r / SB, J = c / SB;
-        double v = 0.0;
-        if (I == J) v = (c <= r) ? W[I][r - I * SB][c - J * SB] : 0.0;
-        else if (I > J) v = L[c][r];
-        Linv[t] = v;
+        for (int t = tid; t < TRSM_ROWS * NB; t += TPB) {
+            const int r = t / NB, c = t % NB;
+            if (r0 + r < n) A[(size_t)(r0 + r) * lda + k0 + c] = X[r][c];
+        }
+        __syncthreads();
     }
     pdl_launch_dependents();
 }
 
-// ---- 2. panel solve: rows [r0, n) of columns [k0, k0+kn): X <- X Linv^T ----
-constexpr int TRSM_ROWS = 64;
-constexpr size_t kTrsmSmem = (size_t)(NB + TRSM_ROWS) * LDL * sizeof(double);
+// Inverses of the 128 x 128 diagonal blocks of the factor for the triangular
+// solves, one CTA per block: from the 32 x 32 inverses that the factorisation
+// left on their diagonal,
+//   inv(L)_IJ = -inv(L_II) sum_{K=J}^{I-1} L_IK inv(L)_KJ,  I > J,
+// block row by block row, and zeros above the diagonal.
+constexpr int LDT = NB - SB + 4;  // a block row of L left of the diagonal: 32 x 96
+constexpr size_t kBlockInvSmem = ((size_t)NB * LDL + (size_t)SB * LDT) * sizeof(double);
 
-// Rows [r0, r0 + TRSM_ROWS) (clipped to rend) of columns [k0, k0 + kn):
-// out[r][c] = sum_{k <= c} X[r][k] * Linv[c][k], in place.
-__device__ __forceinline__ void trsm_rows(double *__restrict__ A, long long lda, int r0, int rend,
-                                          int k0, int kn, const double *__restrict__ Linv,
-                                          double *smem) {
-    double(*Li)[LDL] = reinterpret_cast<double(*)[LDL]>(smem);
-    double(*P)[LDL] = reinterpret_cast<double(*)[LDL]>(smem + NB * LDL);
+__global__ void __launch_bounds__(TPB)
+block_inverse_kernel(const double *__restrict__ A, long long lda, int n, double *__restrict__ Linv,
+                     const int *__restrict__ info) {
+    extern __shared__ double potf2_smem[];
+    double(*V)[LDL] = reinterpret_cast<double(*)[LDL]>(potf2_smem);  // the inverse
+    double(*T)[LDT] = reinterpret_cast<double(*)[LDT]>(potf2_smem + NB * LDL);
+    pdl_wait();
+    if (failed(info)) return;
+    const int k0 = blockIdx.x * NB, kn = min(NB, n - k0);
+    double *Li = Linv + (size_t)blockIdx.x * NB * NB;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int g = lane >> 2, tq = lane & 3;
+    for (int t = tid; t < NB * NB; t += TPB) {
+        const int r = t >> 7, c = t & (NB - 1);
+        V[r][c] = c / SB == r / SB ? Li[t] : 0.0;
+    }
+    for (int I = 1; I < NSB; ++I) {
+        // T: block row I of L, then sum_K L_IK inv(L)_KJ in its place
+        __syncthreads();
+        for (int t = tid; t < SB * I * SB; t += TPB) {
+            const int r = t / (I * SB), c = t % (I * SB);
+            T[r][c] = I * SB + r < kn ? A[(size_t)(k0 + I * SB + r) * lda + k0 + c] : 0.0;
+        }
+        __syncthreads();
+        double o[6][2];  // 8 x 8 tiles of the (32 x 32 I) block row, 16 I of them over 8 warps
+        for (int pass = 0; pass < 2; ++pass) {
+            // pass 0: T <- T V_0..I-1,J;  pass 1: V_I <- -V_II T
+#pragma unroll
+            for (int q = 0; q < 6; ++q) {
+                const int t = warp + q * (TPB / 32);
+                if (t < 16 * I) {
+                    const int m = (t & 3) * 8, c = (t >> 2) * 8;
+                    o[q][0] = o[q][1] = 0.0;
+                    if (pass == 0)
+                        for (int k = c / SB * SB; k < I * SB; k += 4)
+                            dmma_8x8x4(o[q], T[m + g][k + tq], V[k + tq][c + g]);
+                    else
+                        for (int k = 0; k < m + 8; k += 4)  // V_II is lower triangular
+                            dmma_8x8x4(o[q], V[I * SB + m + g][I * SB + k + tq], T[k + tq][c + g]);
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < 6; ++q) {
+                const int t = warp + q * (TPB / 32);
+                if (t < 16 * I) {
+                    const int m = (t & 3) * 8, c = (t >> 2) * 8 + 2 * tq;
+                    if (pass == 0) {
+                        T[m + g][c] = o[q][0];
+                        T[m + g][c + 1] = o[q][1];
+                    } else {
+                        V[I * SB + m + g][c] = -o[q][0];
+                        V[I * SB + m + g][c + 1] = -o[q][1];
+                    }
+                }
+            }
+            __syncthreads();
+        }
+    }
+    for (int t = tid; t < NB * NB; t += TPB) Li[t] = V[t >> 7][t & (NB - 1)];
+}
+
+// Rows [0, rend) of columns [k0, k0 + kn): X <- X Linv^T (the inverse's
+// column-block step, section 5): out[r][c] = sum_{k <= c} X[r][k] Linv[c][k].
+constexpr int RTRSM_ROWS = 64, LDR = NB + 1;
+constexpr size_t kRowsTrsmSmem = (size_t)(NB + RTRSM_ROWS) * LDR * sizeof(double);
+__global__ void __launch_bounds__(TPB)
+rows_trsm_kernel(double *__restrict__ A, long long lda, int rend, int k0, int kn,
+                 const double *__restrict__ Linv, const int *__restrict__ info) {
+    extern __shared__ double trsm_smem[];
+    if (failed(info)) return;
+    const int r0 = blockIdx.x * RTRSM_ROWS;
+    double(*Li)[LDR] = reinterpret_cast<double(*)[LDR]>(trsm_smem);
+    double(*P)[LDR] = reinterpret_cast<double(*)[LDR]>(trsm_smem + NB * LDR);
     const int tid = threadIdx.x;
     for (int t = tid; t < NB * NB; t += TPB) Li[t / NB][t % NB] = Linv[t];
-    for (int t = tid; t < TRSM_ROWS * NB; t += TPB) {
+    for (int t = tid; t < RTRSM_ROWS * NB; t += TPB) {
         const int r = t / NB, c = t % NB;
         P[r][c] = (r0 + r < rend && c < kn) ? A[(size_t)(r0 + r) * lda + k0 + c] : 0.0;
     }
@@ -285,26 +388,6 @@ __device__ __forceinline__ void trsm_rows(double *__restrict__ A, long long lda,
         const int r = r0 + rq * 32 + i;
         if (r < rend && c < kn) A[(size_t)r * lda + k0 + c] = out[i];
     }
-}
-
-__global__ void __launch_bounds__(TPB)
-panel_trsm_kernel(double *__restrict__ A, long long lda, int n, int k0, int kn,
-                  const double *__restrict__ Linv, const int *__restrict__ info) {
-    extern __shared__ double trsm_smem[];
-    pdl_wait();
-    if (failed(info)) return;
-    trsm_rows(A, lda, k0 + kn + blockIdx.x * TRSM_ROWS, n, k0, kn, Linv, trsm_smem);
-    pdl_launch_dependents();
-}
-
-// Rows [0, rend) of columns [k0, k0 + kn): X <- X Linv^T (the inverse's
-// column-block step, section 5).
-__global__ void __launch_bounds__(TPB)
-rows_trsm_kernel(double *__restrict__ A, long long lda, int rend, int k0, int kn,
-                 const double *__restrict__ Linv, const int *__restrict__ info) {
-    extern __shared__ double trsm_smem[];
-    if (failed(info)) return;
-    trsm_rows(A, lda, blockIdx.x * TRSM_ROWS, rend, k0, kn, Linv, trsm_smem);
 }
 
 // ---- 3. trailing update on the FP64 tensor cores ---------------------------
@@ -332,12 +415,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
-}
-
-__device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                 : "+d"(d[0]), "+d"(d[1])
-                 : "d"(a), "d"(b));
 }
 
 // Loads rows [row0, row0+ROWS) x k-columns [kc0, kc0+16) of P into a ROWS x
@@ -911,7 +988,10 @@ int set_smem_attrs() {
                                               (int)kTrsmSmem), "trsm smem attribute"));
     FMLB_TRY(cuda_status(cudaFuncSetAttribute(rows_trsm_kernel,
                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)kTrsmSmem), "trsm smem attribute"));
+                                              (int)kRowsTrsmSmem), "rows trsm smem attribute"));
+    FMLB_TRY(cuda_status(cudaFuncSetAttribute(block_inverse_kernel,
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)kBlockInvSmem), "block inverse smem attribute"));
     attr_dev = dev;
     return FMLB_OK;
 }
@@ -992,9 +1072,10 @@ static int panel_factor(double *A, long long lda, int n, int k0, double *Li, int
                               "potf2_block_kernel", A, lda, k0, kn, Li, info));
     const int rest = n - k0 - kn;
     if (rest > 0)
-        FMLB_TRY(launch_maybe_pdl(true, panel_trsm_kernel, dim3(ceil_div(rest, TRSM_ROWS)),
-                                  dim3(TPB), kTrsmSmem, st, "panel_trsm_kernel", A, lda, n, k0, kn,
-                                  (const double *)Li, (const int *)info));
+        FMLB_TRY(launch_maybe_pdl(
+            true, panel_trsm_kernel, dim3(std::min(ceil_div(rest, TRSM_ROWS), sm_count())),
+            dim3(TPB), kTrsmSmem, st, "panel_trsm_kernel", A, lda, n, k0, (const double *)Li,
+            (const int *)info));
     return FMLB_OK;
 }
 
@@ -1075,7 +1156,8 @@ static int potrf_blocked(double *A, long long lda, int n, void *work, int *info,
     }
     if (panel_used)
         FMLB_TRY(cuda_status(cudaStreamWaitEvent(st, la->panel_done, 0), "join panel stream"));
-    return FMLB_OK;
+    block_inverse_kernel<<<ceil_div(n, NB), TPB, kBlockInvSmem, st>>>(A, lda, n, Linv, info);
+    return launch_status("block_inverse_kernel");
 }
 
 extern "C" int fmlb_potrf_f64(double *A, long long lda, int n, void *work, int *info,
@@ -1182,7 +1264,7 @@ extern "C" int fmlb_potri_f64(double *A, long long lda, int n, const void *work,
     FMLB_TRY(launch_status("identity_kernel"));
     for (int k0 = 0, kb = 0; k0 < n; k0 += NB, ++kb) {
         const int kn = std::min(NB, n - k0), R = k0 + kn;
-        rows_trsm_kernel<<<ceil_div(R, TRSM_ROWS), TPB, kTrsmSmem, st>>>(
+        rows_trsm_kernel<<<ceil_div(R, RTRSM_ROWS), TPB, kRowsTrsmSmem, st>>>(
             V, ldv, R, k0, kn, Linv + (size_t)kb * NB * NB, info);
         FMLB_TRY(launch_status("rows_trsm_kernel"));
         if (R < n)

@@ -35,7 +35,7 @@ def potrf_launches(n, ozaki=False):
     """Kernel launches of fmlb_potrf_f64 / fmlb_potrf_ozaki_f64 for an n x n
     matrix (mirrors their loops)."""
     W = outer_panel(n)
-    count = 0
+    count = 1  # the block inverses
     for K0 in range(0, n, W):
         end = min(K0 + W, n)
         for k0 in range(K0, end, PANEL):
