@@ -5,35 +5,34 @@
 // scale = -0.5/sigma^2) or abs (Laplacian, scale = -1/sigma). Every sigma is
 // emitted from one pass over the descriptors.
 //
-// Tiling: a 64x64 output tile per 256-thread CTA, descriptors staged through
-// shared memory in k-chunks of 16, 4x4 outputs per thread with a stride-16
-// mapping so global stores are coalesced. Symmetric mode launches only the
-// tiles on or below the diagonal and writes the mirror through a shared-memory
-// transpose.
+// Tiles of 64 x 64 outputs (16 x 64 for small problems) per 128-thread CTA,
+// dist_tile.cuh. Symmetric mode launches only the tiles on or below the
+// diagonal and writes the mirror through a shared-memory transpose.
 #include <math.h>
 
 #include "common.cuh"
+#include "dist_tile.cuh"
 
 namespace fmlb {
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, TPB = 256, MAXSIG = 32;
+constexpr int BM = 64, BN = dist::DT_N, TPB = dist::DT_TPB, MAXSIG = 32;
+
+constexpr int kSmallTilesPerSm = 4;  // 16-row tiles per SM up to which they are used
 
 struct SigmaScales {
     double s[MAXSIG];
 };
 
-template <bool kL1>
-__global__ void __launch_bounds__(TPB)
+template <bool kL1, int RI>
+__global__ void __launch_bounds__(TPB, RI == 4 ? 4 : 8)
 distance_kernel_f64(const double *__restrict__ A, int na, int lda, const double *__restrict__ B,
-                    int nb, int ldb, int d, SigmaScales sc, int nsig, double *__restrict__ K,
-                    long long ldk, long long sstride, int symmetric) {
-    // the staging tiles and the transpose tile share one buffer: the
-    // transpose is only used after the last k-chunk
-    __shared__ double smem_raw[BM * (BN + 1)];
-    double(*As)[BM + 1] = reinterpret_cast<double(*)[BM + 1]>(smem_raw);
-    double(*Bs)[BN + 1] = reinterpret_cast<double(*)[BN + 1]>(smem_raw + BK * (BM + 1));
-    double(*T)[BN + 1] = reinterpret_cast<double(*)[BN + 1]>(smem_raw);
+                    int nb, int ldb, int d, const __grid_constant__ SigmaScales sc, int nsig,
+                    double *__restrict__ K, long long ldk, long long sstride, int symmetric) {
+    // the stage and (square tiles) the transpose share one buffer
+    constexpr int kT = BN * (BM + 1);
+    __shared__ double smem[RI == 4 && kT > dist::DT_STAGE ? kT : dist::DT_STAGE];
+    double(*T)[BM + 1] = reinterpret_cast<double(*)[BM + 1]>(smem);
 
     int by, bx;
     if (symmetric) {
@@ -46,75 +45,38 @@ distance_kernel_f64(const double *__restrict__ A, int na, int lda, const double 
         bx = blockIdx.x;
         by = blockIdx.y;
     }
-    const int row0 = by * BM, col0 = bx * BN;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const int row0 = by * 16 * RI, col0 = bx * BN;
+    const int nr = min(16 * RI, na - row0), nc = min(BN, nb - col0);
+    double acc[RI][8];
+    dist::dist_tile<kL1 ? dist::kAbs : dist::kSquare, RI>(
+        acc, smem, [&](int r) { return A + (size_t)(row0 + r) * lda; },
+        [&](int c) { return B + (size_t)(col0 + c) * ldb; }, nr, nc, d);
 
-    double acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-
-    // loader mapping: 16 consecutive k of one row per half-warp
-    const int lk = threadIdx.x & 15, lr = threadIdx.x >> 4;  // lr in 0..15
-    for (int k0 = 0; k0 < d; k0 += BK) {
-        const int k = k0 + lk;
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int ra = row0 + lr + 16 * r;
-            As[lk][lr + 16 * r] = (ra < na && k < d) ? A[(size_t)ra * lda + k] : 0.0;
-            const int rb = col0 + lr + 16 * r;
-            Bs[lk][lr + 16 * r] = (rb < nb && k < d) ? B[(size_t)rb * ldb + k] : 0.0;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            double a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][ty + 16 * i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const double t = a[i] - b[j];
-                    if (kL1)
-                        acc[i][j] += fabs(t);
-                    else
-                        acc[i][j] = fma(t, t, acc[i][j]);
-                }
-        }
-        __syncthreads();
-    }
-
-    const bool mirror = symmetric && by > bx;
+    const int r0 = dist::first_row<RI>(), c0 = dist::first_col();
+    const bool mirror = RI == 4 && symmetric && by > bx;
+    if (mirror) __syncthreads();  // the stage becomes the transpose
     for (int s = 0; s < nsig; ++s) {
         double *Ks = K + s * sstride;
         const double scale = sc.s[s];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int r = row0 + ty + 16 * i;
+        for (int i = 0; i < RI; ++i) {
+            const int r = r0 + 4 * i;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int c = col0 + tx + 16 * j;
-                const double v = exp(scale * acc[i][j]);
-                if (r < na && c < nb) Ks[(size_t)r * ldk + c] = v;
-                if (mirror) T[tx + 16 * j][ty + 16 * i] = v;
+            for (int j = 0; j < 8; ++j) {
+                const int c = c0 + 8 * j;
+                if (r < nr && c < nc) {
+                    const double v = exp(scale * acc[i][j]);
+                    Ks[(size_t)(row0 + r) * ldk + col0 + c] = v;
+                    if (mirror) T[c][r] = v;
+                }
             }
         }
         if (mirror) {
             __syncthreads();
-            // T[c_local][r_local] -> K[col0 + c_local][row0 + r_local], coalesced in r
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int cl = ty + 16 * i;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int rl = tx + 16 * j;
-                    const int gr = col0 + cl, gc = row0 + rl;
-                    if (gr < nb && gc < na) Ks[(size_t)gr * ldk + gc] = T[cl][rl];
-                }
+            // T[c][r] -> K[col0 + c][row0 + r], coalesced in r
+            for (int t = threadIdx.x; t < BN * BM; t += TPB) {
+                const int c = t / BM, r = t % BM;
+                if (c < nc && r < nr) Ks[(size_t)(col0 + c) * ldk + row0 + r] = T[c][r];
             }
             __syncthreads();
         }
@@ -141,17 +103,24 @@ int launch_distance(const double *A, int na, int lda, const double *B, int nb, i
             sc.s[s] = kL1 ? -1.0 / sg : -0.5 / (sg * sg);  // fkernels.f90:334 / :367
         }
         double *Ks = K + s0 * sstride;
-        if (symmetric) {
-            const long long nt = ceil_div(na, BM);
-            const long long nblk = nt * (nt + 1) / 2;
+        // 64-row tiles, only those on or below the diagonal where symmetric; the
+        // whole matrix in 16-row tiles while that is at most a few tiles per SM
+        // (the k-loop's latency counts there, not the rate)
+        const long long nt = ceil_div(na, BM), ntc = ceil_div(nb, BN);
+        const long long nblk = symmetric ? nt * (nt + 1) / 2 : nt * ntc;
+        if (4 * nt * ntc <= kSmallTilesPerSm * sm_count()) {
+            const dim3 grid((unsigned)ntc, ceil_div(na, 16));
+            distance_kernel_f64<kL1, 1><<<grid, TPB, 0, st>>>(A, na, lda, B, nb, ldb, d, sc, ns,
+                                                              Ks, ldk, sstride, 0);
+        } else if (symmetric) {
             FMLB_REQUIRE(nblk < (1LL << 31), "%s: too many tiles", name);
-            distance_kernel_f64<kL1><<<(unsigned)nblk, TPB, 0, st>>>(A, na, lda, B, nb, ldb, d, sc,
-                                                                       ns, Ks, ldk, sstride, 1);
+            distance_kernel_f64<kL1, 4><<<(unsigned)nblk, TPB, 0, st>>>(
+                A, na, lda, B, nb, ldb, d, sc, ns, Ks, ldk, sstride, 1);
         } else {
-            dim3 grid(ceil_div(nb, BN), ceil_div(na, BM));
+            const dim3 grid((unsigned)ntc, (unsigned)nt);
             FMLB_REQUIRE(grid.y <= 65535, "%s: na too large for one launch", name);
-            distance_kernel_f64<kL1><<<grid, TPB, 0, st>>>(A, na, lda, B, nb, ldb, d, sc, ns, Ks,
-                                                             ldk, sstride, 0);
+            distance_kernel_f64<kL1, 4><<<grid, TPB, 0, st>>>(A, na, lda, B, nb, ldb, d, sc, ns,
+                                                              Ks, ldk, sstride, 0);
         }
         FMLB_TRY(launch_status(name));
     }

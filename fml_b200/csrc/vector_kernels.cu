@@ -9,23 +9,34 @@
 // Layout: X (nm, amax, d) row-major FP64 (molecule, atom, feature); K
 // (nsig, nm1, nm2) row-major, the reference's kernels(k, i, j) order.
 //
-// One CTA per molecule pair. Feature chunks of both molecules' atoms are staged
-// in shared memory; each thread owns up to PP atom pairs (p = ja * n1 + ia, the
-// reference's column-major atomic_distance order) and accumulates d in feature
-// order, as the reference's sum does. exp(c_k d) is summed per thread into a
-// per-sigma slot and the slots are combined by a fixed tree, so the result does
-// not depend on scheduling.
+// A CTA takes a group of molecules of each side. Their atoms, packed into one
+// row and one column list, form a dense block that is worked through in 64 x 64
+// distance tiles (dist_tile.cuh). A tile's distances go to shared memory, each
+// row is summed over the columns of one molecule and these sums over the rows
+// of one molecule, in a fixed order, so the result does not depend on
+// scheduling.
+//
+// Bound by FP64 issue: subtract, multiply, add per feature and atom pair, as
+// the reference rounds them (a contracted FMA moves kernels of 1e-100 by more
+// than the 1e-13 they agree with it to). A CTA per molecule pair with one atom
+// pair per thread and load pair was bound by shared memory (300 x 401 molecules
+// of up to 23 atoms, d = 276, 3 sigmas: 6.27 ms, now 2.22 ms).
 #include <math.h>
 
+#include <algorithm>
+
 #include "common.cuh"
+#include "dist_tile.cuh"
 #include "fmlb.h"
 
 namespace fmlb {
 namespace {
 
-constexpr int VK_TPB = 64;     // threads per CTA
-constexpr int VK_FCH = 32;     // features per shared-memory chunk
-constexpr int VK_FS = 33;      // padded row stride of a chunk
+constexpr int VK_TPB = dist::DT_TPB;
+constexpr int VK_T = dist::DT_N;      // tile rows and columns
+constexpr int VK_P = VK_T + 1;        // row pitch of the distance tile
+constexpr int VK_MAX_GROUP = 8;
+constexpr int VK_ROWS = 160;   // atoms of a group: group size x amax stays below, or one molecule
 constexpr int VK_MAX_ATOMS = 128;
 constexpr int VK_MAX_SIGMAS = 32;
 
@@ -33,128 +44,132 @@ struct Coefs {
     double c[VK_MAX_SIGMAS];
 };
 
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+struct VkSide {
+    const double *X;
+    const int *N, *O;  // atoms per molecule, or (packed) the molecules' first rows
+    int nm, amax, group;
+};
+
+// Atom list of molecules [m0, m0 + group): seg[q] = first list entry of
+// molecule m0 + q, row[] = its rows in X. One whole warp.
+__device__ __forceinline__ void vk_list(const VkSide &s, int m0, int *seg, int *row, int *status) {
+    const int lane = threadIdx.x & 31;
+    int n = 0, first = 0;
+    if (lane < s.group && m0 + lane < s.nm) {
+        const int m = m0 + lane;
+        n = s.O ? s.O[m + 1] - s.O[m] : s.N[m];
+        first = s.O ? s.O[m] : m * s.amax;
+        if (n < 0 || n > s.amax) {  // rejected on the host as well
+            if (status) atomicCAS(status, 0, 1);
+            n = min(max(n, 0), s.amax);
+        }
+    }
+    int incl = n;
+    for (int d = 1; d <= VK_MAX_GROUP; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += o;
+    }
+    if (lane <= s.group) seg[lane] = incl - n;
+    for (int q = 0; q < s.group; ++q) {
+        const int nq = __shfl_sync(0xffffffffu, n, q), f = __shfl_sync(0xffffffffu, first, q);
+        const int at = __shfl_sync(0xffffffffu, incl - n, q);
+        for (int a = lane; a < nq; a += 32) row[at + a] = f + a;
+    }
 }
 
-// PP atom pairs per thread per pass: the distance sums of the PP pairs are
-// independent chains, interleaved feature by feature.
-// Packed mode (O1 / O2 not null): molecule m's atoms are rows O[m] .. O[m+1]
-// of a (total_atoms, d) matrix; N and amax then bound the counts only.
-template <int KIND, int PP>
-__global__ void __launch_bounds__(VK_TPB)
-vector_kernels_kernel(const double *__restrict__ X1, const int *__restrict__ N1, int nm1,
-                      int amax1, const double *__restrict__ X2, const int *__restrict__ N2,
-                      int nm2, int amax2, int d, const Coefs coef, int nsig,
-                      double *__restrict__ K, int *__restrict__ status,
-                      const int *__restrict__ O1, const int *__restrict__ O2) {
-    extern __shared__ double sm[];
-    double *A = sm;                                   // [amax1][VK_FS]
-    double *B = A + (size_t)amax1 * VK_FS;            // [amax2][VK_FS]
-    double *acc = B + (size_t)amax2 * VK_FS;          // [nsig][VK_TPB]
-    double *red = acc + (size_t)nsig * VK_TPB;        // [nsig][VK_TPB / 32]
-    const long long pair = blockIdx.x;
-    const int i = (int)(pair / nm2), j = (int)(pair % nm2);
-    const int t = threadIdx.x;
-    int ni = O1 ? O1[i + 1] - O1[i] : N1[i], nj = O2 ? O2[j + 1] - O2[j] : N2[j];
-    if (ni < 0 || ni > amax1 || nj < 0 || nj > amax2) {  // rejected on the host as well
-        if (t == 0 && status) atomicCAS(status, 0, 1);
-        ni = min(max(ni, 0), amax1);
-        nj = min(max(nj, 0), amax2);
-    }
-    for (int k = 0; k < nsig; ++k) acc[k * VK_TPB + t] = 0.0;
-    const double *x1 = X1 + (O1 ? (size_t)O1[i] : (size_t)i * amax1) * d;
-    const double *x2 = X2 + (O2 ? (size_t)O2[j] : (size_t)j * amax2) * d;
-    const int np = ni * nj;
-    for (int p0 = 0; p0 < np; p0 += VK_TPB * PP) {
-        double dist[PP];
-        int oa[PP], ob[PP];
-#pragma unroll
-        for (int q = 0; q < PP; ++q) {
-            const int p = min(p0 + t + q * VK_TPB, np - 1);
-            const int ja = p / ni;
-            oa[q] = (p - ja * ni) * VK_FS;
-            ob[q] = ja * VK_FS;
-            dist[q] = 0.0;
-        }
-        for (int f0 = 0; f0 < d; f0 += VK_FCH) {
-            const int fc = min(VK_FCH, d - f0);
-            __syncthreads();
-            for (int e = t; e < ni * VK_FCH; e += VK_TPB) {
-                const int a = e / VK_FCH, f = e - a * VK_FCH;
-                if (f < fc) A[a * VK_FS + f] = x1[(size_t)a * d + f0 + f];
-            }
-            for (int e = t; e < nj * VK_FCH; e += VK_TPB) {
-                const int b = e / VK_FCH, f = e - b * VK_FCH;
-                if (f < fc) B[b * VK_FS + f] = x2[(size_t)b * d + f0 + f];
-            }
-            __syncthreads();
-#pragma unroll 4
-            for (int f = 0; f < fc; ++f) {
-#pragma unroll
-                for (int q = 0; q < PP; ++q) {
-                    const double e = __dsub_rn(A[oa[q] + f], B[ob[q] + f]);
-                    dist[q] = __dadd_rn(dist[q], KIND == 0 ? __dmul_rn(e, e) : fabs(e));
-                }
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < PP; ++q) {
-            if (p0 + t + q * VK_TPB < np)
-                for (int k = 0; k < nsig; ++k)
-                    acc[k * VK_TPB + t] += exp(dist[q] * coef.c[k]);
-        }
-    }
-    // fixed-order combination: shuffle tree per warp, then the warps in order
-    const int lane = t & 31, warp = t >> 5;
-    for (int k = 0; k < nsig; ++k) {
-        const double s = warp_sum_d(acc[k * VK_TPB + t]);
-        if (lane == 0) red[k * (VK_TPB / 32) + warp] = s;
-    }
+// Packed mode (O set): molecule m's atoms are rows O[m] .. O[m+1] of a
+// (total_atoms, d) matrix; amax then bounds the counts only.
+template <int KIND>
+__global__ void __launch_bounds__(VK_TPB, 4)
+vector_kernels_kernel(const VkSide s1, const VkSide s2, int d, const __grid_constant__ Coefs coef,
+                      int nsig, double *__restrict__ K, int *__restrict__ status) {
+    extern __shared__ double ksum[];  // [nsig][group1][group2]
+    __shared__ double stage[dist::DT_STAGE];  // of the features, then the distance tile
+    __shared__ double part[VK_T][VK_MAX_GROUP + 1];
+    __shared__ int seg1[VK_MAX_GROUP + 1], seg2[VK_MAX_GROUP + 1], row1[VK_ROWS], row2[VK_ROWS];
+    static_assert(VK_T * VK_P <= dist::DT_STAGE, "the tile fits");
+    double(*D)[VK_P] = reinterpret_cast<double(*)[VK_P]>(stage);
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int nb2 = (s2.nm + s2.group - 1) / s2.group;
+    const int m1 = (int)(blockIdx.x / nb2) * s1.group, m2 = (int)(blockIdx.x % nb2) * s2.group;
+    const int g12 = s1.group * s2.group;
+    if (warp == 0) vk_list(s1, m1, seg1, row1, status);
+    if (warp == 1) vk_list(s2, m2, seg2, row2, status);
+    for (int t = tid; t < nsig * g12; t += VK_TPB) ksum[t] = 0.0;
     __syncthreads();
-    for (int k = t; k < nsig; k += VK_TPB) {
-        double s = 0.0;
-        for (int w = 0; w < VK_TPB / 32; ++w) s += red[k * (VK_TPB / 32) + w];
-        K[((size_t)k * nm1 + i) * nm2 + j] = s;
+    const int R1 = seg1[s1.group], R2 = seg2[s2.group];
+    const int tr = dist::first_row<4>(), tc = dist::first_col();
+
+    for (int r0 = 0; r0 < R1; r0 += VK_T) {
+        for (int c0 = 0; c0 < R2; c0 += VK_T) {
+            const int nr = min(VK_T, R1 - r0), nc = min(VK_T, R2 - c0);
+            double acc[4][8];
+            dist::dist_tile<KIND == 0 ? dist::kSquareUnfused : dist::kAbs, 4>(
+                acc, stage, [&](int r) { return s1.X + (size_t)row1[r0 + r] * d; },
+                [&](int c) { return s2.X + (size_t)row2[c0 + c] * d; }, nr, nc, d);
+            __syncthreads();  // the stage becomes the distance tile
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) D[tr + 4 * i][tc + 8 * j] = acc[i][j];
+            __syncthreads();
+            for (int k = 0; k < nsig; ++k) {
+                const double c = coef.c[k];
+                // rows of the tile x molecules of the second side
+                for (int t = tid; t < VK_T * s2.group; t += VK_TPB) {
+                    const int r = t & (VK_T - 1), q = t / VK_T;
+                    if (r < nr) {
+                        double s = 0.0;
+                        const int e = min(seg2[q + 1] - c0, nc);
+                        for (int x = max(seg2[q] - c0, 0); x < e; ++x) s += exp(D[r][x] * c);
+                        part[r][q] = s;
+                    }
+                }
+                __syncthreads();
+                for (int t = tid; t < g12; t += VK_TPB) {
+                    const int p = t / s2.group, q = t - p * s2.group;
+                    double s = ksum[k * g12 + t];
+                    const int e = min(seg1[p + 1] - r0, nr);
+                    for (int x = max(seg1[p] - r0, 0); x < e; ++x) s += part[x][q];
+                    ksum[k * g12 + t] = s;
+                }
+                __syncthreads();
+            }
+        }
+    }
+    for (int t = tid; t < nsig * g12; t += VK_TPB) {
+        const int k = t / g12, p = (t - k * g12) / s2.group, q = t % s2.group;
+        if (m1 + p < s1.nm && m2 + q < s2.nm)
+            K[((size_t)k * s1.nm + m1 + p) * s2.nm + m2 + q] = ksum[t];
     }
 }
 
-size_t vk_smem_bytes(int amax1, int amax2, int nsig) {
-    return sizeof(double) * ((size_t)(amax1 + amax2) * VK_FS + (size_t)nsig * VK_TPB +
-                             (size_t)nsig * (VK_TPB / 32));
+// Molecules per group: about 80 atoms at the usual fill of a padded row (the
+// tile's unused rows and columns then cost a sixth), fewer while the blocks
+// would not fill the GPU a few times over.
+void vk_groups(VkSide &s1, VkSide &s2) {
+    auto most = [](const VkSide &s) { return std::max(1, std::min(VK_MAX_GROUP, VK_ROWS / s.amax)); };
+    s1.group = most(s1);
+    s2.group = most(s2);
+    auto blocks = [&] {
+        return (long long)ceil_div(s1.nm, s1.group) * ceil_div(s2.nm, s2.group);
+    };
+    while (blocks() < 8LL * sm_count() && (s1.group > 1 || s2.group > 1)) {
+        int &g = s1.group >= s2.group ? s1.group : s2.group;
+        g = (g + 1) / 2;
+    }
 }
 
-template <int KIND, int PP>
-int launch_vk(const double *X1, const int *N1, int nm1, int amax1, const double *X2,
-              const int *N2, int nm2, int amax2, int d, const Coefs &coef, int nsig, double *K,
-              int *status, const int *O1, const int *O2, cudaStream_t st) {
-    const size_t smem = vk_smem_bytes(amax1, amax2, nsig);
-    FMLB_TRY(cuda_status(cudaFuncSetAttribute(vector_kernels_kernel<KIND, PP>,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)smem),
-                         "cudaFuncSetAttribute"));
-    vector_kernels_kernel<KIND, PP><<<(unsigned)((long long)nm1 * nm2), VK_TPB, smem, st>>>(
-        X1, N1, nm1, amax1, X2, N2, nm2, amax2, d, coef, nsig, K, status, O1, O2);
+template <int KIND>
+int launch_vk(VkSide s1, VkSide s2, int d, const Coefs &coef, int nsig, double *K, int *status,
+              cudaStream_t st) {
+    vk_groups(s1, s2);
+    const size_t smem = sizeof(double) * (size_t)nsig * s1.group * s2.group;  // <= 16 KB
+    const long long blocks = (long long)ceil_div(s1.nm, s1.group) * ceil_div(s2.nm, s2.group);
+    vector_kernels_kernel<KIND><<<(unsigned)blocks, VK_TPB, smem, st>>>(s1, s2, d, coef, nsig, K,
+                                                                      status);
     return launch_status(KIND == 0 ? "vector_kernels_kernel<gaussian>"
                                    : "vector_kernels_kernel<laplacian>");
-}
-
-// pairs per thread: the smallest of 2, 4, 6, 9, 12, 16 that covers the
-// largest molecule pair in one pass (16 and several passes above that)
-template <int KIND>
-int launch_vk_pp(int pairs, const double *X1, const int *N1, int nm1, int amax1,
-                 const double *X2, const int *N2, int nm2, int amax2, int d, const Coefs &coef,
-                 int nsig, double *K, int *status, const int *O1, const int *O2,
-                 cudaStream_t st) {
-#define FMLB_VK(PP)                                                                            \
-    if (pairs <= PP * VK_TPB || PP == 16)                                                     \
-        return launch_vk<KIND, PP>(X1, N1, nm1, amax1, X2, N2, nm2, amax2, d, coef, nsig, K,  \
-                                   status, O1, O2, st);
-    FMLB_VK(2) FMLB_VK(4) FMLB_VK(6) FMLB_VK(9) FMLB_VK(12) FMLB_VK(16)
-#undef FMLB_VK
-    return FMLB_OK;
 }
 
 }  // namespace
@@ -183,12 +198,9 @@ static int vector_kernels_impl(int kind, const double *X1, const int *N1, int nm
     cudaStream_t st = FMLB_STREAM(stream);
     FMLB_REQUIRE((long long)nm1 * nm2 < 0x7fffffffLL,
                  "fmlb_vector_kernels_f64: too many molecule pairs");
-    const int pairs = amax1 * amax2;
-    if (kind == 0)
-        return launch_vk_pp<0>(pairs, X1, N1, nm1, amax1, X2, N2, nm2, amax2, d, coef, nsig, K,
-                               status, O1, O2, st);
-    return launch_vk_pp<1>(pairs, X1, N1, nm1, amax1, X2, N2, nm2, amax2, d, coef, nsig, K,
-                           status, O1, O2, st);
+    const VkSide s1 = {X1, N1, O1, nm1, amax1, 1}, s2 = {X2, N2, O2, nm2, amax2, 1};
+    return kind == 0 ? launch_vk<0>(s1, s2, d, coef, nsig, K, status, st)
+                     : launch_vk<1>(s1, s2, d, coef, nsig, K, status, st);
 }
 
 extern "C" int fmlb_vector_kernels_f64(int kind, const double *X1, const int *N1, int nm1,
