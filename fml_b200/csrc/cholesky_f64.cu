@@ -446,10 +446,21 @@ __device__ __forceinline__ void syrk_load_tile(double *dst, const double *__rest
     }
 }
 
-template <bool kAligned16>
-__global__ void __launch_bounds__(SY_TPB, 2)
+// Tile of TM x TN = TM/2 of the trailing update; a warp holds TM/2 x TN/2.
+template <int TM>
+struct SyTile {
+    static constexpr int kM = TM, kN = TM / 2, kFr = TM / 16, kFc = TM / 32;
+    static constexpr int kStage = (kM + kN) * SY_LD, kCld = kN + 8;
+    static constexpr size_t kSmem = (size_t)SY_STAGES * kStage * sizeof(double);
+    static_assert(kM * kCld <= SY_STAGES * kStage, "C tile must fit in the stages");
+};
+
+template <bool kAligned16, int TM>
+__global__ void __launch_bounds__(SY_TPB, TM == 128 ? 2 : 4)
 syrk_dmma_kernel(double *__restrict__ C, long long ldc, int m, const double *__restrict__ P,
                  long long ldp, int k, int strip_tiles, const int *__restrict__ info) {
+    using T = SyTile<TM>;
+    constexpr int kFr = T::kFr, kFc = T::kFc;  // fragments of a warp: rows, columns
     extern __shared__ __align__(16) double sy_smem[];
     pdl_wait();
     if (failed(info)) return;
@@ -459,31 +470,31 @@ syrk_dmma_kernel(double *__restrict__ C, long long ldc, int m, const double *__r
         by = (int)(t / strip_tiles);
         bx = (int)(t % strip_tiles);
         if (bx > 2 * by + 1) return;
-    } else {  // tile t -> (row block by of 128, column block bx of 64), bx <= 2 by + 1
+    } else {  // tile t -> (row block by, column block bx of half its width), bx <= 2 by + 1
         by = (int)((sqrt(4.0 * (double)t + 1.0) - 1.0) * 0.5);
         while ((long long)by * by + by > t) --by;
         while ((long long)(by + 1) * (by + 1) + (by + 1) <= t) ++by;
         bx = (int)(t - (long long)by * by - by);
     }
-    const int row0 = by * SY_TM, col0 = bx * SY_TN;
+    const int row0 = by * T::kM, col0 = bx * T::kN;
     if (col0 >= m || row0 >= m) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wr = warp >> 1, wc = warp & 1;
     const int g = lane >> 2, tq = lane & 3;
 
-    double acc[8][4][2];
+    double acc[kFr][kFc][2];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < kFr; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+        for (int j = 0; j < kFc; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
     const int nk = (k + SY_TK - 1) / SY_TK;
 #pragma unroll
     for (int s = 0; s < SY_STAGES - 1; ++s) {
         if (s < nk) {
-            double *st = sy_smem + s * SY_STAGE_DOUBLES;
-            syrk_load_tile<SY_TM, kAligned16>(st, P, ldp, m, k, row0, s * SY_TK);
-            syrk_load_tile<SY_TN, kAligned16>(st + SY_TM * SY_LD, P, ldp, m, k, col0, s * SY_TK);
+            double *st = sy_smem + s * T::kStage;
+            syrk_load_tile<T::kM, kAligned16>(st, P, ldp, m, k, row0, s * SY_TK);
+            syrk_load_tile<T::kN, kAligned16>(st + T::kM * SY_LD, P, ldp, m, k, col0, s * SY_TK);
         }
         cp_async_commit();
     }
@@ -492,24 +503,24 @@ syrk_dmma_kernel(double *__restrict__ C, long long ldc, int m, const double *__r
         __syncthreads();
         const int nxt = kt + SY_STAGES - 1;
         if (nxt < nk) {
-            double *st = sy_smem + (nxt % SY_STAGES) * SY_STAGE_DOUBLES;
-            syrk_load_tile<SY_TM, kAligned16>(st, P, ldp, m, k, row0, nxt * SY_TK);
-            syrk_load_tile<SY_TN, kAligned16>(st + SY_TM * SY_LD, P, ldp, m, k, col0, nxt * SY_TK);
+            double *st = sy_smem + (nxt % SY_STAGES) * T::kStage;
+            syrk_load_tile<T::kM, kAligned16>(st, P, ldp, m, k, row0, nxt * SY_TK);
+            syrk_load_tile<T::kN, kAligned16>(st + T::kM * SY_LD, P, ldp, m, k, col0, nxt * SY_TK);
         }
         cp_async_commit();
-        const double *As = sy_smem + (kt % SY_STAGES) * SY_STAGE_DOUBLES;
-        const double *Bs = As + SY_TM * SY_LD;
+        const double *As = sy_smem + (kt % SY_STAGES) * T::kStage;
+        const double *Bs = As + T::kM * SY_LD;
 #pragma unroll
         for (int kk = 0; kk < SY_TK / 4; ++kk) {
-            double a[8], b[4];
+            double a[kFr], b[kFc];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) a[i] = As[(wr * 64 + i * 8 + g) * SY_LD + kk * 4 + tq];
+            for (int i = 0; i < kFr; ++i) a[i] = As[(wr * (T::kM / 2) + i * 8 + g) * SY_LD + kk * 4 + tq];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Bs[(wc * 32 + j * 8 + g) * SY_LD + kk * 4 + tq];
+            for (int j = 0; j < kFc; ++j) b[j] = Bs[(wc * (T::kN / 2) + j * 8 + g) * SY_LD + kk * 4 + tq];
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < kFr; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) dmma_8x8x4(acc[i][j], a[i], b[j]);
+                for (int j = 0; j < kFc; ++j) dmma_8x8x4(acc[i][j], a[i], b[j]);
         }
     }
     cp_async_wait<0>();
@@ -517,10 +528,10 @@ syrk_dmma_kernel(double *__restrict__ C, long long ldc, int m, const double *__r
     // Epilogue through shared memory: one coalesced pass loads the C tile,
     // the fragments are subtracted there, one coalesced masked pass stores it
     // (keeps the 64 read-modify-writes per thread from serialising).
-    double *Cs = sy_smem;  // SY_TM x SY_CLD doubles, fits in the stage area
+    double *Cs = sy_smem;  // T::kM x T::kCld doubles, fits in the stage area
     const int tid = threadIdx.x;
-    for (int e = tid; e < SY_TM * (SY_TN / 2); e += SY_TPB) {
-        const int r = e / (SY_TN / 2), c = (e % (SY_TN / 2)) * 2;
+    for (int e = tid; e < T::kM * (T::kN / 2); e += SY_TPB) {
+        const int r = e / (T::kN / 2), c = (e % (T::kN / 2)) * 2;
         const int gr = row0 + r, gc = col0 + c;
         double v0 = 0.0, v1 = 0.0;
         if (gr < m) {
@@ -528,29 +539,29 @@ syrk_dmma_kernel(double *__restrict__ C, long long ldc, int m, const double *__r
             if (gc < m) v0 = src[0];
             if (gc + 1 < m) v1 = src[1];
         }
-        Cs[r * SY_CLD + c] = v0;
-        Cs[r * SY_CLD + c + 1] = v1;
+        Cs[r * T::kCld + c] = v0;
+        Cs[r * T::kCld + c + 1] = v1;
     }
     __syncthreads();
-    // fragment (i, j): rows wr*64 + i*8 + g, columns wc*32 + j*8 + 2*tq + {0, 1}
+    // fragment (i, j): rows 8 i + g and columns 8 j + 2 tq + {0, 1} of the warp's tile
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int rl = wr * 64 + i * 8 + g;
+    for (int i = 0; i < kFr; ++i) {
+        const int rl = wr * (T::kM / 2) + i * 8 + g;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int cl = wc * 32 + j * 8 + 2 * tq;
-            Cs[rl * SY_CLD + cl] -= acc[i][j][0];
-            Cs[rl * SY_CLD + cl + 1] -= acc[i][j][1];
+        for (int j = 0; j < kFc; ++j) {
+            const int cl = wc * (T::kN / 2) + j * 8 + 2 * tq;
+            Cs[rl * T::kCld + cl] -= acc[i][j][0];
+            Cs[rl * T::kCld + cl + 1] -= acc[i][j][1];
         }
     }
     __syncthreads();
-    for (int e = tid; e < SY_TM * (SY_TN / 2); e += SY_TPB) {
-        const int r = e / (SY_TN / 2), c = (e % (SY_TN / 2)) * 2;
+    for (int e = tid; e < T::kM * (T::kN / 2); e += SY_TPB) {
+        const int r = e / (T::kN / 2), c = (e % (T::kN / 2)) * 2;
         const int gr = row0 + r, gc = col0 + c;
         if (gr >= m) continue;
         double *dst = C + (size_t)gr * ldc + gc;
-        if (gc < m && gc <= gr) dst[0] = Cs[r * SY_CLD + c];
-        if (gc + 1 < m && gc + 1 <= gr) dst[1] = Cs[r * SY_CLD + c + 1];
+        if (gc < m && gc <= gr) dst[0] = Cs[r * T::kCld + c];
+        if (gc + 1 < m && gc + 1 <= gr) dst[1] = Cs[r * T::kCld + c + 1];
     }
     pdl_launch_dependents();
 }
@@ -574,25 +585,39 @@ int launch_maybe_pdl(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, 
     return launch_status(name);
 }
 
-template <bool kAligned16>
-int launch_syrk_impl(double *C, long long ldc, int m, const double *P, long long ldp, int k,
+template <bool kAligned16, int TM>
+int launch_syrk_tile(double *C, long long ldc, int m, const double *P, long long ldp, int k,
                      int strip_cols, const int *info, cudaStream_t st, bool pdl) {
+    using T = SyTile<TM>;
     static int attr_dev = -1;
     int dev = 0;
     FMLB_TRY(cuda_status(cudaGetDevice(&dev), "syrk: cudaGetDevice"));
     if (attr_dev != dev) {
-        FMLB_TRY(cuda_status(cudaFuncSetAttribute(syrk_dmma_kernel<kAligned16>,
+        FMLB_TRY(cuda_status(cudaFuncSetAttribute(syrk_dmma_kernel<kAligned16, TM>,
                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)kSyrkSmem), "syrk smem attribute"));
+                                                  (int)T::kSmem), "syrk smem attribute"));
         attr_dev = dev;
     }
-    const long long Tr = ceil_div(m, SY_TM);
-    const int strip_tiles = strip_cols > 0 ? ceil_div(std::min(strip_cols, m), SY_TN) : 0;
+    const long long Tr = ceil_div(m, T::kM);
+    const int strip_tiles = strip_cols > 0 ? ceil_div(std::min(strip_cols, m), T::kN) : 0;
     // full: row block by holds 2 by + 2 column tiles; strip: strip_tiles per row block
     const long long ntiles = strip_tiles ? Tr * strip_tiles : Tr * Tr + Tr;
-    return launch_maybe_pdl(pdl, syrk_dmma_kernel<kAligned16>, dim3((unsigned)ntiles),
-                            dim3(SY_TPB), kSyrkSmem, st, "syrk_dmma_kernel", C, ldc, m, P, ldp, k,
+    return launch_maybe_pdl(pdl, syrk_dmma_kernel<kAligned16, TM>, dim3((unsigned)ntiles),
+                            dim3(SY_TPB), T::kSmem, st, "syrk_dmma_kernel", C, ldc, m, P, ldp, k,
                             strip_tiles, info);
+}
+
+// 128 x 64 tiles, or 64 x 32 ones while the former would fill their two slots
+// per SM less than twice: then the last wave and a tile's own latency count
+// (every entry's sum runs in the same order in both).
+template <bool kAligned16>
+int launch_syrk_impl(double *C, long long ldc, int m, const double *P, long long ldp, int k,
+                     int strip_cols, const int *info, cudaStream_t st, bool pdl) {
+    const long long Tr = ceil_div(m, 128);
+    const long long big = strip_cols > 0 ? Tr * ceil_div(std::min(strip_cols, m), 64) : Tr * Tr + Tr;
+    if (big < 4LL * sm_count())
+        return launch_syrk_tile<kAligned16, 64>(C, ldc, m, P, ldp, k, strip_cols, info, st, pdl);
+    return launch_syrk_tile<kAligned16, 128>(C, ldc, m, P, ldp, k, strip_cols, info, st, pdl);
 }
 
 // strip_cols = 0: lower triangle of the m x m block; > 0: only its first
