@@ -30,19 +30,21 @@
 // (21 products instead of 28); the error of one entry stays below
 // k (s + 3) 2^(e_r + e_c + 2 - 8 s).
 //
-// Kernel (one CTA per SM at a time, four tiles per CTA, 320 threads), output
-// tile 128 x 64:
-//   warp 0      TMA producer: per 32-byte k step, the s digit planes of the
-//               128 A rows and 64 B rows (one 3-D box each, 32-byte swizzle)
-//               into a ring as deep as shared memory allows (5 stages at
-//               s = 6, at most 8);
-//   warp 1      allocates 512 TMEM columns (s <= 8 accumulators of 64 int32
-//               columns) and issues tcgen05.mma kind::i8 (M 128, N 64, K 32);
-//   warps 2..9  epilogue, two warps per TMEM lane quarter (32 columns each):
-//               drain the s accumulators into FP64 (Horner), release TMEM to
-//               the next tile's MMAs, scale by the row and column exponents,
-//               and subtract from C through a shared-memory transpose
-//               (coalesced read-modify-write of the lower triangle).
+// Kernel (one CTA per SM at a time, four tiles per CTA, 384 threads), output
+// tile 128 x 128, diagonals in passes of at most four (512 TMEM columns):
+//   warp 0       TMA producer: per stage of 64 k values, the pass's digit planes
+//                of the 128 A rows and 128 B rows (one 3-D box each, 64-byte
+//                swizzle) into a ring as deep as shared memory allows (2 stages
+//                at s = 6; 64-byte box rows move 1.6 times what 32-byte ones do);
+//   warp 1       allocates the 512 TMEM columns and issues tcgen05.mma kind::i8
+//                (M 128, N 128, K 32), the stage's MMAs fully unrolled;
+//   warps 4..11  epilogue (registers moved there from the first warpgroup).
+// C goes through registers and a small stage per warp: a whole tile of it in
+// shared memory left room for 32-byte k steps only.
+// m = 16384, k = 1024, s = 6: 3.13 ms = 88 FP64-equivalent TFLOP/s (4.71 ms before
+// the wider stages, the unrolled issue and the separate drain). Shared memory is
+// what bounds it now: the MMAs read 8 KB per 64 cycles of work, and their operands'
+// copies and the epilogue pass through it as well.
 // Every mbarrier wait is bounded; a wait that runs out stores FMLB_ETIMEDOUT
 // in *info, and every kernel that reads info returns at once.
 #include <math.h>
@@ -68,36 +70,40 @@ constexpr int OZ_BM = 128, OZ_BN = 128;
 constexpr int OZ_PASS_Q = OZ_PASS_DIAGONALS;
 constexpr int OZ_TMEM_BUFS = 4 / OZ_PASS_Q;  // 512 columns: 2 buffers of 2, 1 of 3 or 4
 constexpr int OZ_MAX_PASSES = (8 + OZ_PASS_Q - 1) / OZ_PASS_Q;
-static_assert(OZ_PASS_Q >= 2 && OZ_PASS_Q <= 4, "passes of 2 to 4 diagonals");
-constexpr int OZ_KB = 32;          // int8 k values (bytes) per stage: one MMA K step
+static_assert(OZ_PASS_Q == 4, "one TMEM buffer of four diagonals, at most two passes");
+constexpr int OZ_KB = 64;          // int8 k values (bytes) per stage: two MMA K steps
+constexpr int OZ_MMA_K = 32;       // k values of one MMA
 constexpr int OZ_MAX_STAGES = 8;  // the ring depth is set per launch from shared memory
-constexpr int OZ_THREADS = 320;    // 10 warps
+constexpr int OZ_THREADS = 384;    // 3 warpgroups: producer and MMA issuer, two of epilogue
+// Registers a thread. The block starts with 168 each (65536 / 384, as the
+// compiler grants them); the first warpgroup gives back what the epilogue takes,
+// which keeps 64 drained columns in registers. The host checks the start.
+constexpr int OZ_REGS = 168, OZ_REGS_LOAD = 40, OZ_REGS_EPI = 232;
+static_assert(OZ_REGS_LOAD + 2 * OZ_REGS_EPI <= 3 * OZ_REGS, "the registers of the block");
 constexpr int OZ_EPI_WARPS = 8;
 constexpr int OZ_TMEM_COLS = 512;
-constexpr int OZ_CPITCH = OZ_BN + 1;  // doubles per row of the staged C tile (odd: rows of
-                                      // one column fall in 16 distinct banks per half-warp)
-constexpr int OZ_A_PLANE = OZ_BM * OZ_KB;   // 4096 bytes per A digit plane per stage
-constexpr int OZ_B_PLANE = OZ_BN * OZ_KB;   // 4096
-constexpr int OZ_CTILE_BYTES = OZ_BM * OZ_CPITCH * (int)sizeof(double);  // 132096
-constexpr int OZ_COLF_BYTES = OZ_BN * (int)sizeof(double);
-constexpr int OZ_ALIGN = 256;  // shared-memory base: the 32-byte swizzle atom
+constexpr int OZ_A_PLANE = OZ_BM * OZ_KB;   // 8192 bytes per A digit plane per stage
+constexpr int OZ_B_PLANE = OZ_BN * OZ_KB;   // 8192
+constexpr int OZ_CHUNK = 8;        // columns of C that pass through shared memory at a time
+// doubles of an epilogue warp: a 32 x 8 chunk of the update, the data of its 64
+// columns and 32 rows
+constexpr int OZ_WARP_STAGE = 32 * OZ_CHUNK + 2 * 64 + 2 * 32;
+constexpr int OZ_CSTAGE_BYTES = OZ_EPI_WARPS * OZ_WARP_STAGE * (int)sizeof(double);  // 28 KB
+constexpr int OZ_ALIGN = 1024;
 constexpr int OZ_NONFINITE = 0x7fffffff;    // exponent marking a row with Inf / NaN
 
 constexpr long long kOzDefaultBudget = 4000000000LL;  // clock cycles (~2 s)
 constexpr int OZ_SMEM_LIMIT = 232448 - 64;  // opt-in shared memory per CTA, less static
-constexpr int OZ_BAR_BYTES = (2 * OZ_MAX_STAGES + 2 * OZ_TMEM_BUFS + 2) * 8 + 8;
+constexpr int OZ_BAR_BYTES = (2 * OZ_MAX_STAGES + 2 * OZ_TMEM_BUFS + 1) * 8 + 8;
 
 struct OzParams {
     int m;             // rows (= columns) of C
     int p_row0;        // slice row of C's row 0 (and column 0)
-    int ns;            // digit planes
-    int nkb;           // 32-byte k steps
+    int nkb;           // stages of OZ_KB k values
     int strip_cols;    // > 0: only the first strip_cols columns
     int strip_tiles;   // column tiles per row block in strip mode
     long long ntiles;
     long long ldc;
-    int exp_bias;      // -8 (ns + 1)
-    int npass;         // passes: diagonals [0, Q), [Q, 2Q), ... [.., ns)
     double zp_c;       // c' (zero point of the digit planes)
     double zp_kc2;     // kp c'^2
     int skip_loads;    // test hook: the producer issues no copies
@@ -113,14 +119,13 @@ struct OzMaps {
 // K-major, M = 128, N = 128.
 constexpr uint32_t kIdescI8 = (2u << 4) | (1u << 7) | (1u << 10) |
                               ((uint32_t)(OZ_BN >> 3) << 17) | ((uint32_t)(OZ_BM >> 4) << 24);
-__device__ __forceinline__ uint32_t idesc_i8(int, int) { return kIdescI8; }
 
 __device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                       uint32_t idesc, uint32_t accumulate) {
+                                       uint32_t accumulate) {
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
         " tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+        "l"(adesc), "l"(bdesc), "r"(kIdescI8), "r"(accumulate));
 }
 
 // Tile t -> (row0, col0) of the lower triangle of 128 x 128 tiles (row block
@@ -163,6 +168,12 @@ __device__ __forceinline__ double oz_pow2_factor(int e) {
     return (e >= -500 && e <= 500) ? __longlong_as_double((long long)(e + 1 + 1023) << 52) : 0.0;
 }
 
+// The scaling for a non-finite row or column, or an exponent outside +-500.
+__device__ __forceinline__ double oz_scale_far(double core, int er, int ec) {
+    return (er == OZ_NONFINITE || ec == OZ_NONFINITE) ? __longlong_as_double(0x7ff8000000000000LL)
+                                                      : ldexp(core, er + ec + 2);
+}
+
 // First tile t' >= t of this CTA's sequence (stride gridDim.x) inside C, or ntiles.
 __device__ __forceinline__ long long oz_next_tile(long long t, const OzParams &p, int &row0,
                                                   int &col0) {
@@ -171,24 +182,48 @@ __device__ __forceinline__ long long oz_next_tile(long long t, const OzParams &p
     return p.ntiles;
 }
 
-// 8-byte asynchronous global -> shared copies (completion per thread).
-__device__ __forceinline__ void cp_async8(double *dst, const double *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(tc::smem_u32(dst)), "l"(src)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() {
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+// Exact int32 -> double: the value's bits beside the exponent of 2^52, then one
+// addition (the conversion instruction runs at a quarter of the FP64 rate).
+__device__ __forceinline__ double oz_double(uint32_t v) {
+    return __dadd_rn(__hiloint2double(0x43300000, (int)(v ^ 0x80000000u)),
+                     -4503601774854144.0);  // -(2^52 + 2^31)
 }
 
-// Pass q0..q1 of the diagonals needs the digit planes 0..q1-1.
-__device__ __forceinline__ void oz_pass(const OzParams &p, int ps, int &q0, int &q1) {
-    q0 = ps * OZ_PASS_Q;
-    q1 = min(p.ns, q0 + OZ_PASS_Q);
+// Double (row, c) of an epilogue warp's 32 x 8 stage: pairs of columns are
+// permuted by the row, so that rows written by one lane each (16 bytes at a
+// time) and rows read by 8 lanes each both spread over the banks.
+__device__ __forceinline__ int oz_stage_at(int row, int c) {
+    return row * OZ_CHUNK + (((c >> 1) ^ ((row >> 1) & 3)) << 1) + (c & 1);
 }
 
+// Passes over the diagonals: [0, Q), [Q, 2Q), .. [.., NS). A pass that ends
+// before diagonal q1 reads the digit planes 0 .. q1-1.
+constexpr int oz_passes(int ns) { return (ns + OZ_PASS_Q - 1) / OZ_PASS_Q; }
+__host__ __device__ constexpr int oz_pass_end(int ns, int ps) {
+    return (ps + 1) * OZ_PASS_Q < ns ? (ps + 1) * OZ_PASS_Q : ns;
+}
+
+// The MMAs of one stage of pass PS, all of them unrolled: one thread issues
+// them, and with the loops and their index arithmetic an MMA took 148 cycles,
+// 84 unrolled.
+template <int NS, int PS>
+__device__ __forceinline__ void oz_issue(uint32_t tmem, uint64_t da, uint64_t db, uint32_t first) {
+    constexpr int q0 = PS * OZ_PASS_Q, q1 = oz_pass_end(NS, PS);
+#pragma unroll
+    for (int h = 0; h < OZ_KB / OZ_MMA_K; ++h) {
+#pragma unroll
+        for (int q = q0; q < q1; ++q) {
+#pragma unroll
+            for (int a = 0; a <= q; ++a)  // offsets in 16-byte units of the descriptor address
+                mma_i8(tmem + (uint32_t)((q - q0) * OZ_BN),
+                       da + (uint64_t)((a * OZ_A_PLANE + h * OZ_MMA_K) >> 4),
+                       db + (uint64_t)(((q - a) * OZ_B_PLANE + h * OZ_MMA_K) >> 4),
+                       h == 0 && a == 0 ? first : 1u);
+        }
+    }
+}
+
+template <int NS>
 __global__ void __launch_bounds__(OZ_THREADS, 1)
 ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
                   const int *__restrict__ exps, const double *__restrict__ rsum, OzParams p,
@@ -196,18 +231,15 @@ ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
     extern __shared__ uint8_t oz_smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>(
         (reinterpret_cast<uintptr_t>(oz_smem_raw) + OZ_ALIGN - 1) & ~(uintptr_t)(OZ_ALIGN - 1));
-    const int stage_bytes = p.ns * (OZ_A_PLANE + OZ_B_PLANE);  // B planes after ns A planes
+    constexpr int stage_bytes = NS * (OZ_A_PLANE + OZ_B_PLANE);  // B planes after NS A planes
+    constexpr int npass = oz_passes(NS);
     const int nst = p.stages;
-    // C tile, 128 x 129: column 128 holds the tile's column digit sums S_c
-    double *cs = reinterpret_cast<double *>(smem + nst * stage_bytes);
-    // 2^(e_c + 1) per column of the tile, 0 where the exact scaling needs ldexp
-    double *colf = reinterpret_cast<double *>(smem + nst * stage_bytes + OZ_CTILE_BYTES);
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + nst * stage_bytes + OZ_CTILE_BYTES +
-                                                  OZ_COLF_BYTES);
+    double *cstage = reinterpret_cast<double *>(smem + nst * stage_bytes);
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + nst * stage_bytes + OZ_CSTAGE_BYTES);
     uint64_t *full = bars, *empty = bars + OZ_MAX_STAGES;
     uint64_t *tmem_full = bars + 2 * OZ_MAX_STAGES, *tmem_empty = tmem_full + OZ_TMEM_BUFS,
-             *mma_done = tmem_empty + OZ_TMEM_BUFS, *epi_bar = mma_done + 1;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(epi_bar + 1);
+             *mma_done = tmem_empty + OZ_TMEM_BUFS;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mma_done + 1);
     __shared__ int abort_cta;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -222,7 +254,6 @@ ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
             tc::mbar_init(&tmem_empty[b], OZ_EPI_WARPS);
         }
         tc::mbar_init(mma_done, 1);
-        tc::mbar_init(epi_bar, OZ_EPI_WARPS * 32);
         tc::mbar_fence_init();
     }
     __syncthreads();
@@ -233,6 +264,9 @@ ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
     tc::fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
+    // each warpgroup sets its registers inside its own branch: where the two meet
+    // the compiler can count on the smaller number only
+    if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(OZ_REGS_LOAD));
     if (warp == 0) {
         // ------------------------------------------------------------ producer
         if (lane == 0) {
@@ -241,9 +275,8 @@ ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
             for (long long t = blockIdx.x; t < p.ntiles && ok; t += gridDim.x) {
                 int row0, col0;
                 if (!oz_tile(t, p, row0, col0)) continue;
-                for (int ps = 0; ps < p.npass && ok; ++ps) {
-                    int q0, q1;
-                    oz_pass(p, ps, q0, q1);
+                for (int ps = 0; ps < npass && ok; ++ps) {
+                    const int q1 = oz_pass_end(NS, ps);
                     const CUtensorMap *map = &maps.m[ps];  // boxes of q1 planes
                     for (int kb = 0; kb < p.nkb && !p.skip_loads; ++kb, ++issued) {
                         const int st = (int)(issued % nst);
@@ -254,7 +287,7 @@ ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
                             break;
                         }
                         uint8_t *sa = smem + st * stage_bytes;
-                        uint8_t *sb = sa + p.ns * OZ_A_PLANE;
+                        uint8_t *sb = sa + NS * OZ_A_PLANE;
                         tc::mbar_arrive_expect_tx(&full[st], (uint32_t)(q1 * (OZ_A_PLANE + OZ_B_PLANE)));
                         tc::tma_load_3d(sa, map, &full[st], kb * OZ_KB, p.p_row0 + row0, 0);
                         tc::tma_load_3d(sb, map, &full[st], kb * OZ_KB, p.p_row0 + col0, 0);
@@ -275,9 +308,7 @@ ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
             for (long long t = blockIdx.x; t < p.ntiles && ok; t += gridDim.x) {
                 int row0, col0;
                 if (!oz_tile(t, p, row0, col0)) continue;
-                for (int ps = 0; ps < p.npass; ++ps, ++lp) {
-                    int q0, q1;
-                    oz_pass(p, ps, q0, q1);
+                for (int ps = 0; ps < npass; ++ps, ++lp) {
                     const int buf = lp % OZ_TMEM_BUFS;
                     if (!tc::mbar_wait(&tmem_empty[buf], (uint32_t)(((lp / OZ_TMEM_BUFS) & 1) ^ 1),
                                        budget)) {
@@ -296,20 +327,12 @@ ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
                         }
                         tc::fence_after_sync();
                         const uint8_t *sa = smem + st * stage_bytes;
-                        const uint8_t *sb = sa + p.ns * OZ_A_PLANE;
+                        const uint8_t *sb = sa + NS * OZ_A_PLANE;
                         const uint64_t da = tc::smem_desc_kmajor(sa, OZ_KB);
                         const uint64_t db = tc::smem_desc_kmajor(sb, OZ_KB);
-                        for (int q = q0; q < q1; ++q) {
-                            const uint32_t dacc =
-                                tmem_base + (uint32_t)((buf * OZ_PASS_Q + q - q0) * OZ_BN);
-                            for (int a = 0; a <= q; ++a) {
-                                const int b = q - a;
-                                // plane offsets in 16-byte units of the descriptor address
-                                mma_i8(dacc, da + (uint64_t)((a * OZ_A_PLANE) >> 4),
-                                       db + (uint64_t)((b * OZ_B_PLANE) >> 4), idesc_i8(a, b),
-                                       (kb > 0 || a > 0) ? 1u : 0u);
-                            }
-                        }
+                        const uint32_t dacc = tmem_base + (uint32_t)(buf * OZ_PASS_Q * OZ_BN);
+                        if (ps == 0) oz_issue<NS, 0>(dacc, da, db, kb > 0);
+                        else oz_issue<NS, npass - 1>(dacc, da, db, kb > 0);
                         tc::mma_commit(&empty[st]);  // frees the stage once these MMAs finish
                     }
                     if (!ok) break;
@@ -320,67 +343,60 @@ ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
             tc::mma_commit(mma_done);
             if (!tc::mbar_wait(mma_done, 0, budget)) oz_fail(info);
         }
-    } else {
+    } else if (warp >= 4) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(OZ_REGS_EPI));
         // --------------------------------------------------------------- epilogue
-        // C's tile is staged in shared memory (cs, rows of 129 doubles) by
-        // cp.async while the tile's first pass runs on the tensor cores, and
-        // written back once after its last pass, both with one coalesced row
-        // segment of 32 columns per warp instruction (element i * 256 + e of
-        // the tile for thread e). Two warps per TMEM lane quarter, 64 columns
-        // (two chunks of 32) each: per pass and chunk, drain the pass's
-        // accumulators into FP64 (Horner in 256), scale, and subtract from
-        // this lane's row of cs. TMEM is released after the second chunk's
-        // drain, so the next pass's MMAs overlap that chunk's arithmetic.
+        // Two warps per TMEM lane quarter, 64 columns each. The tensor cores wait
+        // from a pass's last MMA until its accumulators are drained, so that comes
+        // first and alone: into FP64 (Horner in 256), a row and 64 columns per
+        // lane in registers, the next 8 columns' loads in flight while 8 are
+        // converted. The rest runs beside the next pass's MMAs: 8 columns at a
+        // time go through the warp's stage to the lanes that hold those entries of
+        // C in 64-byte row segments, which scale, subtract and store them. An entry
+        // of C belongs to the same lane in every pass; C's lines are brought into
+        // L2 while the tile's first pass runs.
+        // Cycles of a tile (6 planes, k = 1024): 96k, of which the MMAs wait 8k for
+        // the drain and 9k for operands; 136k with the drain, the scaling and C's
+        // update in one loop, 33k of them waiting for it.
         const int qw = warp & 3;
-        const int half = (warp - 2) >> 2;
-        const int e = threadIdx.x - 64;           // 0 .. 255
-        const int rl = qw * 32 + lane;            // this lane's row of the tile
-        double *csr = cs + rl * OZ_CPITCH;
+        const int half = (warp - 4) >> 2;
+        double *stage = cstage + (warp - 4) * OZ_WARP_STAGE;
+        double *colf = stage + 32 * OZ_CHUNK, *colsum = colf + 64;
+        double *rowf = colsum + 64, *rowsum = rowf + 32;
+        const int sr0 = lane >> 3, sc0 = lane & 7;
         int lp = 0;
-        uint32_t nsync = 0;
         bool ok = true;
-        // every epilogue thread arrives; bounded wait, so a warp that gave up
-        // cannot hold the others
-        auto epi_sync = [&]() -> bool {
-            tc::mbar_arrive(epi_bar);
-            const bool r = tc::mbar_wait(epi_bar, nsync & 1, budget);
-            ++nsync;
-            return r;
-        };
-        auto tile_elem = [&](int i, int r0, int c0, int &r, int &c, size_t &g) -> bool {
-            const int idx = i * (OZ_EPI_WARPS * 32) + e;
-            r = idx >> 7;
-            c = idx & (OZ_BN - 1);
-            const int gr = r0 + r, gc = c0 + c;
-            g = (size_t)gr * p.ldc + gc;
-            return gr < p.m && gc <= gr && (p.strip_cols == 0 || gc < p.strip_cols);
-        };
-        auto prefetch = [&](int r0, int c0) {
-            for (int i = 0; i < OZ_BM * OZ_BN / (OZ_EPI_WARPS * 32); ++i) {
-                int r, c;
-                size_t g;
-                if (tile_elem(i, r0, c0, r, c, g)) cp_async8(cs + r * OZ_CPITCH + c, C + g);
-            }
-            cp_async_commit();
-        };
         int row0 = 0, col0 = 0;
-        long long t = oz_next_tile(blockIdx.x, p, row0, col0);
-        if (t < p.ntiles) prefetch(row0, col0);
-        while (t < p.ntiles && ok) {
-            const int grow = row0 + rl;
-            const int er = grow < p.m ? exps[p.p_row0 + grow] : 0;
-            const double sr = grow < p.m ? rsum[p.p_row0 + grow] : 0.0;
-            const double rowf = oz_pow2_factor(er);
-            if (e < OZ_BN) {  // the tile's column data; read after the tile-start barrier
-                const int gc = col0 + e;
-                const int ec = gc < p.m ? exps[p.p_row0 + gc] : 0;
-                colf[e] = oz_pow2_factor(ec);
-                cs[e * OZ_CPITCH + OZ_BN] = gc < p.m ? rsum[p.p_row0 + gc] : 0.0;
+        for (long long t = oz_next_tile(blockIdx.x, p, row0, col0); t < p.ntiles && ok;
+             t = oz_next_tile(t + gridDim.x, p, row0, col0)) {
+            const int wrow = row0 + qw * 32, wcol = col0 + half * 64;  // the warp's part of C
+            double *cbase = C + (size_t)(wrow + sr0) * p.ldc + wcol + sc0;
+            // entry i of chunk ch: row 4 i + sr0, column 8 ch + sc0
+            auto inside = [&](int i, int ch) {
+                const int gr = wrow + 4 * i + sr0, gc = wcol + OZ_CHUNK * ch + sc0;
+                return gr < p.m && gc <= gr && (p.strip_cols == 0 || gc < p.strip_cols);
+            };
+            {   // the 512-byte row segment of each lane's row
+                const int gr = wrow + lane;
+                if (gr < p.m && wcol <= gr)
+                    for (int c = 0; c < 64; c += 16)
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(
+                            C + (size_t)gr * p.ldc + min(wcol + c, p.m - 1)));
             }
-            for (int ps = 0; ps < p.npass && ok; ++ps, ++lp) {
-                int q0, q1;
-                oz_pass(p, ps, q0, q1);
-                const bool last = ps == p.npass - 1;
+            // data of the warp's 64 columns and 32 rows: 2^(e + 1) (0 where the
+            // exact scaling needs ldexp) and the digit sums S
+            bool plain = true;
+            for (int c = lane; c < 96; c += 32) {
+                const int g = c < 64 ? wcol + c : wrow + c - 64;
+                const double f = oz_pow2_factor(g < p.m ? exps[p.p_row0 + g] : 0);
+                plain = plain && f != 0.0;
+                (c < 64 ? colf + c : rowf + c - 64)[0] = f;
+                (c < 64 ? colsum + c : rowsum + c - 64)[0] = g < p.m ? rsum[p.p_row0 + g] : 0.0;
+            }
+            plain = __all_sync(0xffffffffu, plain);
+            for (int ps = 0; ps < npass; ++ps, ++lp) {
+                const int q1 = oz_pass_end(NS, ps), nq = q1 - ps * OZ_PASS_Q;
+                const bool last = ps == npass - 1;
                 // Horner over diagonals q0 .. q1-1 carries 256^(q1-1-q): scale by 256^-(q1+1)
                 const double pbias = __longlong_as_double((long long)(1023 - 8 * (q1 + 1)) << 52);
                 const int buf = lp % OZ_TMEM_BUFS;
@@ -390,74 +406,83 @@ ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
                     break;
                 }
                 tc::fence_after_sync();
-                if (ps == 0) {  // the tile's C has landed in cs (every thread's copies)
-                    cp_async_wait_all();
-                    if (!epi_sync()) {
-                        oz_fail(info);
-                        ok = false;
-                        break;
+                const uint32_t tbase = tmem_base + ((uint32_t)(qw * 32) << 16) +
+                                       (uint32_t)(buf * OZ_PASS_Q * OZ_BN + half * 64);
+                double acc[64];
+                {
+                    uint32_t v[OZ_PASS_Q][OZ_CHUNK];
+                    auto load = [&](int cb) {
+#pragma unroll
+                        for (int q = 0; q < OZ_PASS_Q; ++q)
+                            if (q < nq) tc::tmem_ld8_async(tbase + (uint32_t)(q * OZ_BN + cb), v[q]);
+                    };
+                    load(0);
+#pragma unroll
+                    for (int cb = 0; cb < 64; cb += OZ_CHUNK) {
+                        tc::tmem_ld_wait();
+#pragma unroll
+                        for (int q = 0; q < OZ_PASS_Q; ++q) {
+                            if (q < nq) {
+#pragma unroll
+                                for (int j = 0; j < OZ_CHUNK; ++j) {
+                                    const double x = oz_double(tc::after_ld_wait(v[q][j]));
+                                    acc[cb + j] = q ? fma(acc[cb + j], 256.0, x) : x;
+                                }
+                            }
+                        }
+                        if (cb + OZ_CHUNK < 64) load(cb + OZ_CHUNK);
                     }
                 }
-                for (int cc = 0; cc < 2; ++cc) {
-                    const int cb = half * 64 + cc * 32;  // chunk's first column in the tile
-                    double acc[32];
+                tc::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&tmem_empty[buf]);  // the buffer is free
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) acc[j] = 0.0;
-                    for (int q = q0; q < q1; ++q) {
-                        uint32_t v[32];
-                        tc::tmem_ld32(tmem_base + ((uint32_t)(qw * 32) << 16) +
-                                          (uint32_t)((buf * OZ_PASS_Q + q - q0) * OZ_BN + cb), v);
+                for (int ch = 0; ch < 64 / OZ_CHUNK; ++ch) {
+                    const int cb = ch * OZ_CHUNK;
 #pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            acc[j] = fma(acc[j], 256.0, (double)(int)v[j]);
-                    }
-                    if (cc == 1) {
-                        tc::fence_before_sync();
-                        __syncwarp();
-                        if (lane == 0) tc::mbar_arrive(&tmem_empty[buf]);  // the buffer is free
-                    }
+                    for (int c = 0; c < OZ_CHUNK; c += 2)
+                        *reinterpret_cast<double2 *>(&stage[oz_stage_at(lane, c)]) =
+                            make_double2(acc[cb + c], acc[cb + c + 1]);
+                    __syncwarp();
                     // last pass: (acc 256^-(s+1) + c' (S_r + S_c) + k c'^2) 2^(e_r + e_c + 2),
                     // earlier passes: acc 256^-(q1+1) 2^(e_r + e_c + 2); fixed order, no
                     // contraction. Both power-of-two scalings are exact multiplications
                     // (core * 2^(e_r+1) is normal), so the result is ldexp's, rounded once.
+                    auto core_of = [&](int r) {
+                        const double core = __dmul_rn(stage[oz_stage_at(r, sc0)], pbias);
+                        return last ? __dadd_rn(__dadd_rn(core, __dmul_rn(p.zp_c,
+                                                                          __dadd_rn(rowsum[r],
+                                                                                    colsum[cb + sc0]))),
+                                                p.zp_kc2)
+                                    : core;
+                    };
+                    double *cc = cbase + cb;
+                    if (plain) {
+                        const double f = colf[cb + sc0];
+                        double cv[8];
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const double f = colf[cb + j];
-                        double core = __dmul_rn(acc[j], pbias);
-                        if (last)
-                            core = __dadd_rn(
-                                __dadd_rn(core, __dmul_rn(p.zp_c,
-                                                          __dadd_rn(sr, cs[(cb + j) * OZ_CPITCH + OZ_BN]))),
-                                p.zp_kc2);
-                        double v;
-                        if (rowf != 0.0 && f != 0.0) {
-                            v = __dmul_rn(__dmul_rn(core, rowf), f);
-                        } else {  // a non-finite row or column, or an exponent outside +-500
-                            const int gc = col0 + cb + j;
-                            const int ec = gc < p.m ? exps[p.p_row0 + gc] : 0;
-                            v = (er == OZ_NONFINITE || ec == OZ_NONFINITE)
-                                    ? __longlong_as_double(0x7ff8000000000000LL)
-                                    : ldexp(core, er + ec + 2);
+                        for (int i = 0; i < 8; ++i)
+                            cv[i] = inside(i, ch) ? cc[(size_t)(4 * i) * p.ldc] : 0.0;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const int r = 4 * i + sr0;
+                            const double v = __dmul_rn(__dmul_rn(core_of(r), rowf[r]), f);
+                            if (inside(i, ch)) cc[(size_t)(4 * i) * p.ldc] = __dsub_rn(cv[i], v);
                         }
-                        csr[cb + j] = __dsub_rn(csr[cb + j], v);
+                    } else {  // a non-finite row or column, or an exponent outside +-500
+#pragma unroll 1
+                        for (int i = 0; i < 8; ++i) {
+                            if (!inside(i, ch)) continue;
+                            const int r = 4 * i + sr0;
+                            double *e = cc + (size_t)(4 * i) * p.ldc;
+                            *e = __dsub_rn(*e, oz_scale_far(core_of(r), exps[p.p_row0 + wrow + r],
+                                                            exps[p.p_row0 + wcol + cb + sc0]));
+                        }
                     }
+                    __syncwarp();
                 }
             }
-            if (!ok) break;
-            if (!epi_sync()) {  // every pass's subtraction is in cs
-                oz_fail(info);
-                break;
-            }
-            for (int i = 0; i < OZ_BM * OZ_BN / (OZ_EPI_WARPS * 32); ++i) {
-                int r, c;
-                size_t g;
-                if (tile_elem(i, row0, col0, r, c, g)) C[g] = cs[r * OZ_CPITCH + c];
-            }
-            // the next tile's C into the elements this thread has just written back
-            t = oz_next_tile(t + gridDim.x, p, row0, col0);
-            if (t < p.ntiles) prefetch(row0, col0);
         }
-        cp_async_wait_all();  // no copy lands after the CTA has left
     }
     tc::fence_before_sync();
     __syncthreads();
@@ -569,7 +594,7 @@ int make_plane_map(CUtensorMap *map, const int8_t *base, int rows, long long ldp
     const cuuint32_t estride[3] = {1, 1, 1};
     CUresult res = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<int8_t *>(base), gdim,
                       gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                      CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                      CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (res != CUDA_SUCCESS) {
         set_error("ozaki: cuTensorMapEncodeTiled failed (%d)", (int)res);
@@ -578,20 +603,45 @@ int make_plane_map(CUtensorMap *map, const int8_t *base, int rows, long long ldp
     return FMLB_OK;
 }
 
-// Deepest operand ring (<= OZ_MAX_STAGES) whose shared memory fits a CTA.
-// (two stages at 6 planes, one at 7 or 8 beside the 129 KB C tile).
+// Deepest operand ring (<= OZ_MAX_STAGES) whose shared memory fits a CTA
+// (three stages up to 4 planes, two at 5 or 6, one at 7 or 8).
 int oz_stages(int ns) {
     const int sb = ns * (OZ_A_PLANE + OZ_B_PLANE);
-    const int room = OZ_SMEM_LIMIT - OZ_CTILE_BYTES - OZ_COLF_BYTES - OZ_BAR_BYTES - OZ_ALIGN;
+    const int room = OZ_SMEM_LIMIT - OZ_CSTAGE_BYTES - OZ_BAR_BYTES - OZ_ALIGN;
     return std::max(1, std::min(OZ_MAX_STAGES, room / sb));
 }
 
 size_t oz_smem_bytes(int ns) {
-    return (size_t)oz_stages(ns) * ns * (OZ_A_PLANE + OZ_B_PLANE) + OZ_CTILE_BYTES +
-           OZ_COLF_BYTES + OZ_BAR_BYTES + OZ_ALIGN;
+    return (size_t)oz_stages(ns) * ns * (OZ_A_PLANE + OZ_B_PLANE) + OZ_CSTAGE_BYTES +
+           OZ_BAR_BYTES + OZ_ALIGN;
 }
 
 thread_local tc::TestHooks t_hooks = {0, 0};
+
+template <int NS>
+int launch_oz(const OzMaps &maps, const OzakiSlices &s, const OzParams &p, double *C, int *info,
+              int grid, size_t smem, long long budget, cudaStream_t st) {
+    static_assert(NS <= OZAKI_MAX_SLICES, "digit planes");
+    static int attr_dev = -1;
+    int dev = 0;
+    FMLB_TRY(cuda_status(cudaGetDevice(&dev), "ozaki: cudaGetDevice"));
+    if (attr_dev != dev) {
+        FMLB_TRY(cuda_status(cudaFuncSetAttribute(ozaki_syrk_kernel<NS>,
+                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  OZ_SMEM_LIMIT),
+                             "ozaki: smem attribute"));
+        cudaFuncAttributes fa;
+        FMLB_TRY(cuda_status(cudaFuncGetAttributes(&fa, ozaki_syrk_kernel<NS>),
+                             "ozaki: kernel attributes"));
+        if (fa.numRegs != OZ_REGS) {  // setmaxnreg.inc would wait for registers it cannot get
+            set_error("ozaki: built with %d registers a thread instead of %d", fa.numRegs, OZ_REGS);
+            return FMLB_ENOTSUP;
+        }
+        attr_dev = dev;
+    }
+    ozaki_syrk_kernel<NS><<<grid, OZ_THREADS, smem, st>>>(maps, s.exps, s.rsum, p, C, info, budget);
+    return launch_status("ozaki_syrk_kernel");
+}
 
 }  // namespace
 
@@ -615,30 +665,26 @@ int ozaki_syrk(double *C, long long ldc, int m, const OzakiSlices &s, int p_row0
                int *info, cudaStream_t st) {
     if (m <= 0) return FMLB_OK;
     FMLB_REQUIRE(s.ns >= 1 && s.ns <= OZAKI_MAX_SLICES, "ozaki: 1..%d slices", OZAKI_MAX_SLICES);
-    FMLB_REQUIRE(s.kp % OZ_KB == 0 && s.kp <= 8192, "ozaki: k must be a multiple of 32, <= 8192");
+    FMLB_REQUIRE(s.kp % OZ_MMA_K == 0 && s.kp <= 8192, "ozaki: k must be a multiple of 32, <= 8192");
     FMLB_REQUIRE(p_row0 >= 0 && p_row0 + m <= s.rows, "ozaki: rows outside the slice buffer");
     // boxes of 128 rows and the planes each pass reads (planes 0 .. q1-1 for
     // its last diagonal q1-1)
     OzMaps maps;
     memset(&maps, 0, sizeof maps);
-    const int npass = (s.ns + OZ_PASS_Q - 1) / OZ_PASS_Q;
-    for (int ps = 0; ps < npass; ++ps)
+    for (int ps = 0; ps < oz_passes(s.ns); ++ps)
         FMLB_TRY(make_plane_map(&maps.m[ps], s.planes, s.rows, s.ldpl, s.kp, s.pstride,
-                                std::min(s.ns, (ps + 1) * OZ_PASS_Q), OZ_BM));
+                                oz_pass_end(s.ns, ps), OZ_BM));
     OzParams p;
     p.m = m;
     p.p_row0 = p_row0;
-    p.ns = s.ns;
-    p.nkb = s.kp / OZ_KB;
+    p.nkb = ceil_div(s.kp, OZ_KB);  // past kp the copies fill with zeros
     p.strip_cols = strip_cols > 0 ? std::min(strip_cols, m) : 0;
     const long long Tr = ceil_div(m, OZ_BM);
     p.strip_tiles = p.strip_cols > 0 ? ceil_div(p.strip_cols, OZ_BN) : 0;
     const long long nband = ceil_div(Tr, OZ_BAND);
     p.ntiles = p.strip_tiles ? nband * OZ_BAND * p.strip_tiles
                              : (long long)OZ_GROUP * nband * (nband + 1) / 2;
-    p.npass = npass;
     p.ldc = ldc;
-    p.exp_bias = -8 * (s.ns + 1);
     double zc = ldexp(1.0, -8 * s.ns - 1);  // half an ulp of the last digit
     for (int t = 2; t <= s.ns; ++t) zc += ldexp(128.0, -8 * t);
     p.zp_c = zc;
@@ -647,24 +693,21 @@ int ozaki_syrk(double *C, long long ldc, int m, const OzakiSlices &s, int p_row0
     p.skip_loads = hooks.skip_loads;
     p.stages = oz_stages(s.ns);
     const size_t smem = oz_smem_bytes(s.ns);
-    static int attr_dev = -1;
-    int dev = 0;
-    FMLB_TRY(cuda_status(cudaGetDevice(&dev), "ozaki: cudaGetDevice"));
-    if (attr_dev != dev) {
-        FMLB_TRY(cuda_status(cudaFuncSetAttribute(ozaki_syrk_kernel,
-                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  OZ_SMEM_LIMIT),
-                             "ozaki: smem attribute"));
-        attr_dev = dev;
-    }
     // four tiles per CTA: CTAs retire while the update runs, so the
     // factorisation's high-priority panel chain gets SMs (a persistent grid
     // held every SM until the update ended and serialised the lookahead)
     const int grid = (int)std::min<long long>(
         p.ntiles, std::max<long long>(sm_count(), (p.ntiles + 3) / 4));
-    ozaki_syrk_kernel<<<grid, OZ_THREADS, smem, st>>>(maps, s.exps, s.rsum, p, C, info,
-                                                       hooks.wait_budget);
-    return launch_status("ozaki_syrk_kernel");
+    switch (s.ns) {
+        case 1: return launch_oz<1>(maps, s, p, C, info, grid, smem, hooks.wait_budget, st);
+        case 2: return launch_oz<2>(maps, s, p, C, info, grid, smem, hooks.wait_budget, st);
+        case 3: return launch_oz<3>(maps, s, p, C, info, grid, smem, hooks.wait_budget, st);
+        case 4: return launch_oz<4>(maps, s, p, C, info, grid, smem, hooks.wait_budget, st);
+        case 5: return launch_oz<5>(maps, s, p, C, info, grid, smem, hooks.wait_budget, st);
+        case 6: return launch_oz<6>(maps, s, p, C, info, grid, smem, hooks.wait_budget, st);
+        case 7: return launch_oz<7>(maps, s, p, C, info, grid, smem, hooks.wait_budget, st);
+        default: return launch_oz<8>(maps, s, p, C, info, grid, smem, hooks.wait_budget, st);
+    }
 }
 
 size_t ozaki_slice_bytes(int rows, int kp, int ns) {
@@ -672,7 +715,7 @@ size_t ozaki_slice_bytes(int rows, int kp, int ns) {
 }
 
 int ozaki_bind(void *ws, int rows, int kp, int ns, OzakiSlices &s) {
-    FMLB_REQUIRE(kp % OZ_KB == 0, "ozaki: padded k must be a multiple of 32");
+    FMLB_REQUIRE(kp % OZ_MMA_K == 0, "ozaki: padded k must be a multiple of 32");
     char *p = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(ws) + 255) & ~(uintptr_t)255);
     s.planes = reinterpret_cast<int8_t *>(p);
     s.rows = rows;

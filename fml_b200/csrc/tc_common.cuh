@@ -127,6 +127,24 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
+// 8 consecutive 32-bit TMEM columns of this thread's lane. Asynchronous: the
+// values may be used after tmem_ld_wait(), through after_ld_wait(), which keeps
+// the compiler from moving a use above the wait.
+__device__ __forceinline__ void tmem_ld8_async(uint32_t taddr, uint32_t (&v)[8]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+          "=r"(v[7])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld_wait() {
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ uint32_t after_ld_wait(uint32_t v) {
+    asm volatile("" : "+r"(v));
+    return v;
+}
+
 // ---- host ---------------------------------------------------------------------
 // Test hooks of the tensor-core kernels, per host thread (fmlb_tc_test_hooks):
 // the clock-cycle budget of every mbarrier wait and a switch that makes the
