@@ -21,6 +21,7 @@
 // Every mbarrier wait is bounded; a wait that runs out records an error code
 // in *status and the CTA winds down instead of hanging, after its own copies
 // and MMAs in flight have finished.
+#include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <math.h>
@@ -443,11 +444,13 @@ __global__ void split_center_kernel(const double *__restrict__ X, int n, int ldx
     }
 }
 
-// column means of X (n rows): a CTA per 32 columns, 32 row groups of one warp
-// each (row r to group r mod 32, coalesced 32-column segments), the groups'
-// partial sums combined by a fixed shared-memory tree
-constexpr int CM_ROWG = 32;
-__global__ void __launch_bounds__(32 * CM_ROWG)
+// column means of X (n rows): a cluster of CM_PARTS CTAs per 32 columns, 32 row
+// groups of one warp in each CTA (row r to group r mod (32 CM_PARTS), coalesced
+// 32-column segments), the groups' partial sums combined by a fixed
+// shared-memory tree and the CTAs' in rank order. One CTA per 32 columns kept 14
+// of the SMs busy at d = 435 (70 us for 16384 rows).
+constexpr int CM_ROWG = 32, CM_PARTS = 8;
+__global__ void __cluster_dims__(1, CM_PARTS, 1) __launch_bounds__(32 * CM_ROWG)
 column_mean_kernel(const double *__restrict__ X, int n, int ldx, int d, double *__restrict__ mu) {
     __shared__ double part[CM_ROWG][33];
     const int c = threadIdx.x, g = threadIdx.y;
@@ -455,7 +458,8 @@ column_mean_kernel(const double *__restrict__ X, int n, int ldx, int d, double *
     double s = 0.0;
     if (k < d) {
 #pragma unroll 8
-        for (int i = g; i < n; i += CM_ROWG) s += X[(size_t)i * ldx + k];
+        for (int i = blockIdx.y * CM_ROWG + g; i < n; i += CM_PARTS * CM_ROWG)
+            s += X[(size_t)i * ldx + k];
     }
     part[g][c] = s;
     __syncthreads();
@@ -463,7 +467,14 @@ column_mean_kernel(const double *__restrict__ X, int n, int ldx, int d, double *
         if (g < h) part[g][c] += part[g + h][c];
         __syncthreads();
     }
-    if (g == 0 && k < d) mu[k] = n ? part[0][c] / n : 0.0;
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    cluster.sync();
+    if (blockIdx.y == 0 && g == 0 && k < d) {
+        double v = 0.0;
+        for (int p = 0; p < CM_PARTS; ++p) v += *cluster.map_shared_rank(&part[0][c], p);
+        mu[k] = n ? v / n : 0.0;
+    }
+    cluster.sync();  // no CTA leaves while its sums are read
 }
 
 // ---- host: tensor maps --------------------------------------------------------
@@ -525,8 +536,8 @@ extern "C" int fmlb_column_mean_f64(const double *X, int n, int ldx, int d, doub
                                     void *stream) {
     using namespace fmlb;
     FMLB_REQUIRE(n >= 0 && d >= 1 && ldx >= d && mu, "fmlb_column_mean_f64: bad arguments");
-    column_mean_kernel<<<ceil_div(d, 32), dim3(32, CM_ROWG), 0, FMLB_STREAM(stream)>>>(X, n, ldx,
-                                                                                  d, mu);
+    column_mean_kernel<<<dim3(ceil_div(d, 32), CM_PARTS), dim3(32, CM_ROWG), 0,
+                         FMLB_STREAM(stream)>>>(X, n, ldx, d, mu);
     return launch_status("column_mean_kernel");
 }
 
