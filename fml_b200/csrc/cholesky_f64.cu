@@ -51,6 +51,22 @@ __device__ __forceinline__ void pdl_launch_dependents() {
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+__device__ __forceinline__ void cp_async_16(void *smem, const void *gmem, int src_bytes) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem),
+                 "r"(src_bytes));
+}
+__device__ __forceinline__ void cp_async_8(void *smem, const void *gmem, int src_bytes) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem),
+                 "r"(src_bytes));
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
+}
+
 // ---- 1. diagonal block ----------------------------------------------------
 // The 128 x 128 block is factored in four 32-column steps. In step J one warp
 // factors and inverts the 32 x 32 diagonal sub-block in registers with warp
@@ -142,14 +158,14 @@ potf2_block_kernel(double *__restrict__ A, long long lda, int k0, int kn,
     if (failed(info)) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, tq = lane & 3;  // fragment row / k (A, B), row / column pair (C)
-    for (int t = tid; t < NB * NB; t += TPB) {
+    for (int t = tid; t < NB * NB; t += TPB) {  // all loads in flight together
         const int r = t >> 7, c = t & (NB - 1);
-        double v = 0.0;
-        if (r < kn && c <= r) v = A[(size_t)(k0 + r) * lda + (k0 + c)];
-        else if (r == c) v = 1.0;  // identity padding past kn keeps the block SPD
-        L[r][c] = v;
+        if (r < kn && c <= r) cp_async_8(&L[r][c], A + (size_t)(k0 + r) * lda + (k0 + c), 8);
+        else L[r][c] = r == c ? 1.0 : 0.0;  // identity padding past kn keeps the block SPD
     }
     if (tid == 0) bad = 0;
+    cp_async_commit();
+    cp_async_wait<0>();
     __syncthreads();
     for (int J = 0; J < NSB; ++J) {
         const int b0 = J * SB, r0 = b0 + SB;
@@ -235,15 +251,17 @@ panel_trsm_kernel(double *__restrict__ A, long long lda, int n, int k0,
     for (int t = tid; t < NB * NB; t += TPB) {
         const int r = t / NB, c = t % NB, R = r / SB, C = c / SB;
         if (C <= R)
-            blocks[(R * (R + 1) / 2 + C) * TRSM_BLK + (r % SB) * LDW + c % SB] =
-                C == R ? Linv[t] : A[(size_t)(k0 + r) * lda + k0 + c];
+            cp_async_8(&blocks[(R * (R + 1) / 2 + C) * TRSM_BLK + (r % SB) * LDW + c % SB],
+                       C == R ? Linv + t : A + (size_t)(k0 + r) * lda + k0 + c, 8);
     }
     const int m = (warp & 3) * 8, h = (warp >> 2) * 16;  // rows m.., columns h.. of each block
     for (int r0 = k0 + NB + blockIdx.x * TRSM_ROWS; r0 < n; r0 += gridDim.x * TRSM_ROWS) {
         for (int t = tid; t < TRSM_ROWS * NB; t += TPB) {
             const int r = t / NB, c = t % NB;
-            X[r][c] = r0 + r < n ? A[(size_t)(r0 + r) * lda + k0 + c] : 0.0;
+            cp_async_8(&X[r][c], A + (size_t)min(r0 + r, n - 1) * lda + k0 + c, r0 + r < n ? 8 : 0);
         }
+        cp_async_commit();
+        cp_async_wait<0>();
         for (int J = 0; J < NSB; ++J) {
             const double *row = blocks + J * (J + 1) / 2 * TRSM_BLK + (h + g) * LDW + tq;
             __syncthreads();
@@ -307,15 +325,19 @@ block_inverse_kernel(const double *__restrict__ A, long long lda, int n, double 
     const int g = lane >> 2, tq = lane & 3;
     for (int t = tid; t < NB * NB; t += TPB) {
         const int r = t >> 7, c = t & (NB - 1);
-        V[r][c] = c / SB == r / SB ? Li[t] : 0.0;
+        if (c / SB == r / SB) cp_async_8(&V[r][c], Li + t, 8);
+        else V[r][c] = 0.0;
     }
     for (int I = 1; I < NSB; ++I) {
         // T: block row I of L, then sum_K L_IK inv(L)_KJ in its place
         __syncthreads();
         for (int t = tid; t < SB * I * SB; t += TPB) {
             const int r = t / (I * SB), c = t % (I * SB);
-            T[r][c] = I * SB + r < kn ? A[(size_t)(k0 + I * SB + r) * lda + k0 + c] : 0.0;
+            const bool in = I * SB + r < kn;
+            cp_async_8(&T[r][c], in ? A + (size_t)(k0 + I * SB + r) * lda + k0 + c : A, in ? 8 : 0);
         }
+        cp_async_commit();
+        cp_async_wait<0>();
         __syncthreads();
         double o[6][2];  // 8 x 8 tiles of the (32 x 32 I) block row, 16 I of them over 8 warps
         for (int pass = 0; pass < 2; ++pass) {
@@ -400,22 +422,6 @@ constexpr int SY_STAGE_DOUBLES = (SY_TM + SY_TN) * SY_LD;
 constexpr int SY_CLD = SY_TN + 8;  // row pitch of the epilogue's C tile in shared memory
 static_assert(SY_TM * SY_CLD <= SY_STAGES * SY_STAGE_DOUBLES, "C tile must fit in the stages");
 constexpr size_t kSyrkSmem = (size_t)SY_STAGES * SY_STAGE_DOUBLES * sizeof(double);
-
-__device__ __forceinline__ void cp_async_16(void *smem, const void *gmem, int src_bytes) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem),
-                 "r"(src_bytes));
-}
-__device__ __forceinline__ void cp_async_8(void *smem, const void *gmem, int src_bytes) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem),
-                 "r"(src_bytes));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
-}
 
 // Loads rows [row0, row0+ROWS) x k-columns [kc0, kc0+16) of P into a ROWS x
 // SY_LD stage buffer; out-of-range rows / columns are zero-filled.
