@@ -94,15 +94,16 @@ __device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
 // r holds row r of the block (a) and column r of the inverse (v) in registers;
 // the column steps are unrolled by template recursion, so every register index
 // is a constant. A step scales column J by 1 / sqrt(pivot) and then, from one
-// shuffle per entry L[c][J], updates both the rest of the block and the
-// inverse's forward substitution (right-looking): two independent FMA streams
-// that cover each other's and the next pivot's latency. Entries above the
-// diagonal hold values that nothing reads.
+// broadcast per entry L[c][J], updates both the rest of the block and the
+// inverse's forward substitution (right-looking): two independent FMA streams.
+// The next pivot goes ahead of them by shuffles, so its reciprocal root is
+// formed beside them; the other entries of the column are broadcast through
+// shared memory (two to a load, where a shuffle takes two instructions each).
+// Entries above the diagonal hold values that nothing reads.
 template <int J>
 struct WarpFactorInvert32 {
-    __device__ __forceinline__ static void run(double (&a)[SB], double (&v)[SB], int lane,
-                                               int &fail) {
-        const double piv = __shfl_sync(0xffffffffu, a[J], J);
+    __device__ __forceinline__ static void run(double (&a)[SB], double (&v)[SB], double piv,
+                                               double *col, int lane, int &fail) {
         if (!(piv > 0.0) && !fail) fail = J + 1;  // later columns are NaN and not stored
         const double inv = rsqrt(piv);
         double root = piv * inv;  // sqrt(piv), corrected once
@@ -110,24 +111,40 @@ struct WarpFactorInvert32 {
         a[J] = lane == J ? root : a[J] * inv;
         v[J] *= inv;
         const double lij = a[J], vj = v[J];
-#pragma unroll
-        for (int c = J + 1; c < SB; ++c) {
-            const double lcj = __shfl_sync(0xffffffffu, lij, c);  // L[c][J]
-            a[c] = fma(-lij, lcj, a[c]);
-            v[c] = fma(-lcj, vj, v[c]);
+        double *mine = col + (J & 1) * SB;  // two buffers: one barrier a step
+        mine[lane] = lij;
+        double next = 0.0;
+        if (J + 1 < SB) {
+            const double l1 = __shfl_sync(0xffffffffu, lij, J + 1);
+            a[(J + 1) % SB] = fma(-lij, l1, a[(J + 1) % SB]);
+            v[(J + 1) % SB] = fma(-l1, vj, v[(J + 1) % SB]);
+            next = __shfl_sync(0xffffffffu, a[(J + 1) % SB], J + 1);
         }
-        WarpFactorInvert32<J + 1>::run(a, v, lane, fail);
+        __syncwarp();
+#pragma unroll
+        for (int c = (J + 2) & ~1; c < SB; c += 2) {
+            const double2 l = *reinterpret_cast<const double2 *>(mine + c);  // L[c][J], L[c+1][J]
+            if (c > J + 1) {
+                a[c] = fma(-lij, l.x, a[c]);
+                v[c] = fma(-l.x, vj, v[c]);
+            }
+            a[c + 1] = fma(-lij, l.y, a[c + 1]);
+            v[c + 1] = fma(-l.y, vj, v[c + 1]);
+        }
+        WarpFactorInvert32<J + 1>::run(a, v, next, col, lane, fail);
     }
 };
 template <>
 struct WarpFactorInvert32<SB> {
-    __device__ __forceinline__ static void run(double (&)[SB], double (&)[SB], int, int &) {}
+    __device__ __forceinline__ static void run(double (&)[SB], double (&)[SB], double, double *,
+                                               int, int &) {}
 };
 
 // Factors the sub-block at L[b0.., b0..] in place and writes its inverse into W
 // (row-major, zeros above the diagonal). Returns the 1-based failing column or
 // 0 (the same value in every lane).
-__device__ __forceinline__ int warp_potrf_inv32(double (*L)[LDL], int b0, double (*W)[LDW]) {
+__device__ __forceinline__ int warp_potrf_inv32(double (*L)[LDL], int b0, double (*W)[LDW],
+                                                double *col) {
     const int lane = threadIdx.x & 31;
     double a[SB], v[SB];
 #pragma unroll
@@ -136,7 +153,7 @@ __device__ __forceinline__ int warp_potrf_inv32(double (*L)[LDL], int b0, double
         v[c] = c == lane ? 1.0 : 0.0;
     }
     int fail = 0;
-    WarpFactorInvert32<0>::run(a, v, lane, fail);
+    WarpFactorInvert32<0>::run(a, v, __shfl_sync(0xffffffffu, a[0], 0), col, lane, fail);
     if (fail) return fail;
 #pragma unroll
     for (int c = 0; c < SB; ++c) {
@@ -154,6 +171,7 @@ potf2_block_kernel(double *__restrict__ A, long long lda, int k0, int kn,
     double(*L)[LDL] = reinterpret_cast<double(*)[LDL]>(potf2_smem);
     double(*W)[LDW] = reinterpret_cast<double(*)[LDW]>(potf2_smem + NB * LDL);
     __shared__ int bad;
+    __shared__ __align__(16) double col[2 * SB];
     pdl_wait();
     if (failed(info)) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -170,7 +188,7 @@ potf2_block_kernel(double *__restrict__ A, long long lda, int k0, int kn,
     for (int J = 0; J < NSB; ++J) {
         const int b0 = J * SB, r0 = b0 + SB;
         if (warp == 0) {
-            const int f = warp_potrf_inv32(L, b0, W);
+            const int f = warp_potrf_inv32(L, b0, W, col);
             if (f && lane == 0) bad = b0 + f;
         }
         __syncthreads();
