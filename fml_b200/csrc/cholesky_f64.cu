@@ -1130,7 +1130,10 @@ static int panel_factor(double *A, long long lda, int n, int k0, double *Li, int
 
 // Factor the outer panel of columns [K0, K0 + width) on stream st: per inner
 // panel of NB columns, the diagonal block and the panel solve (all rows below),
-// then the update of the rest of the outer panel's columns by that inner panel.
+// then an update inside the outer panel. The updates are those of recursive
+// halving: after j inner panels, the last s = lowest set bit of j of them
+// update the next s, so half of the work runs with k = width / 2 and a quarter
+// with k = width / 4 (28 and 24 TFLOP/s) instead of all of it with k = NB (17).
 static int factor_outer_panel(double *A, long long lda, int n, int K0, int width, double *Linv,
                               int *info, cudaStream_t st) {
     using namespace fmlb;
@@ -1140,9 +1143,11 @@ static int factor_outer_panel(double *A, long long lda, int n, int K0, int width
                               k0 > K0));
         const size_t b = (size_t)(k0 + NB);
         const int rem = end - (int)b;
-        if (rem > 0)
-            FMLB_TRY(launch_syrk(A + b * lda + b, lda, n - (int)b, A + b * lda + k0, lda, NB, info,
-                                 st, rem, true));
+        if (rem > 0) {
+            const int j = (int)(b - K0) / NB, s = (j & -j) * NB;
+            FMLB_TRY(launch_syrk(A + b * lda + b, lda, n - (int)b, A + b * lda + b - s, lda, s, info,
+                                 st, std::min(s, rem), true));
+        }
     }
     return FMLB_OK;
 }
