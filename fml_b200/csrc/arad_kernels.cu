@@ -95,6 +95,32 @@ SetWs carve(char *&p, int nm, int amax) {
     return w;
 }
 
+// exp(x) for the terms inside the window, x in [-16, 0] (the reduction holds to
+// -700): x = k ln2 + r with ln2 in two parts, exp(r) by the polynomial of degree
+// 11 that interpolates it at the Chebyshev nodes of [-ln2/2, ln2/2] (relative
+// error 1.5e-17; coefficients computed in 60 digits and rounded), the exponent
+// added as an integer. Within 0.9 ulp (0.26 on average); half the instructions of the general
+// function, which has to look after every argument.
+__device__ __forceinline__ double exp_window(double x) {
+    const double magic = 6755399441055744.0;  // 1.5 * 2^52: rounds to an integer
+    const double kd = fma(x, 1.4426950408889634, magic);
+    const int k = __double2loint(kd);
+    const double n = kd - magic;
+    const double r = fma(n, -2.3190468138462996e-17, fma(n, -0.6931471805599453, x));
+    const double r2 = r * r;
+    double e = fma(2.7632715071632255e-07, r2, 2.4801485278370062e-05);
+    double o = fma(2.5110095611886237e-08, r2, 2.7557240761739257e-06);
+    e = fma(e, r2, 0.0013888888952505406);
+    o = fma(o, r2, 0.00019841269890193705);
+    e = fma(e, r2, 0.04166666666648738);
+    o = fma(o, r2, 0.008333333333319546);
+    e = fma(e, r2, 0.5000000000000019);
+    o = fma(o, r2, 0.1666666666666668);
+    const double q = fma(o, r, e);
+    const double p = fma(fma(q, r, 1.0), r, 1.0);
+    return __hiloint2double(__double2hiint(p) + (k << 20), __double2loint(p));
+}
+
 // atomic_distl2 in FP64, reference order (farad_kernels.f90:58-88).
 // x = descriptor of one atom (5, amax); xi = its sine factors.
 __device__ double distl2_f64(const double *x1, const double *xi1, int n1, const double *x2,
@@ -110,7 +136,7 @@ __device__ double distl2_f64(const double *x1, const double *xi1, int n1, const 
             const double dr = __dsub_rn(r2, r1);
             const double t = __dmul_rn(dr, dr);
             if (t < P.maxg2) {
-                double d = __dmul_rn(__dmul_rn(exp(__dmul_rn(t, P.inv_width)), e1), xi2[m2]);
+                double d = __dmul_rn(__dmul_rn(exp_window(__dmul_rn(t, P.inv_width)), e1), xi2[m2]);
                 const double dp = __dsub_rn(p1, x2[amax + m2]);
                 const double dg = __dsub_rn(g1, x2[2 * amax + m2]);
                 const double st = __ddiv_rn(
@@ -956,27 +982,38 @@ arad_fast_pair_kernel(SetWs w1, const int *__restrict__ N1, int nm1, SetWs w2,
 // operations. At sigma 0.1 the exponent carries l2 / sigma^2 = 100 l2, and sums
 // in any other order leave the 1e-12 agreement with the reference.
 //
-// Per molecule pair, both molecules staged in shared memory:
+// A CTA takes one molecule I and a few molecules J, as many at a time as its
+// shared memory holds:
 //   1. the run of neighbours m2 of j1 inside the (8 w)^2 window of every
 //      record (i1, m1), walking both ascending lists together (a list that
 //      does not ascend keeps its whole length, and its terms are tested);
-//   2. the atom pairs bucketed by their number of terms, so that the 32 pairs
-//      of a warp have nearly the same number (86 % of the lanes work, against
-//      59 % with loops over m1 and m2 in lockstep);
-//   3. one thread per atom pair walks its runs as one flat loop;
-//   4. the kernel exponentials of every l2 and sigma, summed in a fixed order.
-// Bound by the FP64 pipe: 28 FP64 instructions per term, 16 of them the
-// exponential. The stoichiometric factor comes from the class table, formed by
-// the same operations (two FP64 divisions per term before), and the operands
-// from shared memory (per-lane gathers from global memory before).
-constexpr int F6_TPB = 256, F6_BUCKETS = 64;
-constexpr int F6_WIN = 4096;  // runs held at a time (8 KB): the atoms j1 go in chunks above that
+//   2. the atom pairs ordered by their number of terms, so that the 32 pairs
+//      of a warp have nearly the same number (59 % of the lanes work with loops
+//      over m1 and m2 in lockstep), and by atom j1 among equals, so that its
+//      lanes read the same few records;
+//   3. warps take 32 pairs at a time, longest first; a thread walks the runs of
+//      its pair as one flat loop;
+//   4. the kernel exponentials of every l2 and sigma, a warp per molecule J and
+//      sigma, in a fixed order.
+// 28 FP64 instructions per term, 16 of them the exponential. The stoichiometric
+// factor comes from the class table, formed by the same operations (two FP64
+// divisions per term before), and the operands from shared memory (per-lane
+// gathers from global memory before), whose pipe is now as busy as the issue
+// slots. One J at a time and 256 threads left half of the warps waiting for the
+// one with the longest pairs.
+constexpr int F6_TPB = 512;
+constexpr int F6_AP = 1024;    // atom pairs at a time (a pair of the largest molecules)
+constexpr int F6_WIN = 12288;  // runs at a time (24 KB): the atoms j1 go in chunks above that
+constexpr int F6_JA = 128, F6_JM = 16;  // atoms and molecules J at a time
+constexpr int F6_BUCKETS = 32, F6_CHUNKS = F6_AP / 32;
 constexpr int F6_SST = FC_MAXC + 1;
+static_assert(FC_MAXA * FC_MAXA <= F6_AP && FC_MAXA <= F6_JA, "one pair of molecules fits");
+static_assert(F6_JM <= F6_TPB / 32 && F6_JM < 32, "a warp per molecule J, a lane each");
 
 struct F64Side {
     double2 *A, *B;    // records by atom: (r, sine factor), (cos, sin)
     double *self;
-    int *off;          // record offsets of the atoms
+    int *off, *end;    // records of the atoms
     int *acls, *asc;
     unsigned char *C;  // class of each record
 };
@@ -984,87 +1021,103 @@ struct F64View {
     F64Side i, j;
     double *l2;           // l2 of every atom pair
     double *st;           // stoichiometric table, row stride F6_SST
-    double *red;          // (F6_TPB / 32) * MAXSIG
     int *tot;             // terms of every atom pair
-    int *bucket;          // F6_BUCKETS + 1
+    int *rank;            // F6_BUCKETS x F6_CHUNKS
+    int *jatom, *jrec;    // first atom and record of each molecule J, and the ends
+    int *ctl;             // molecules J, largest atom count, next 32 pairs
     unsigned short *win;  // F6_WIN: [m1][atom pair] first neighbour | length << 8
     unsigned short *perm; // atom pairs by number of terms
 };
 
 __host__ __device__ inline int f64_pad(int n) { return (n + 7) & ~7; }
+// records of the molecules J at a time: about four of average size
+__host__ __device__ inline int f64_pool(int amax) {
+    return f64_pad(amax * amax) > 1072 ? f64_pad(amax * amax) : 1072;
+}
 inline size_t f64_smem_bytes(int amax) {
-    const size_t R = (size_t)f64_pad(amax * amax);
-    return R * 4 * sizeof(double2) +
-           (R + FC_MAXC * F6_SST + (F6_TPB / 32) * MAXSIG + 2 * FC_MAXA) * sizeof(double) +
-           (R + F6_BUCKETS + 8 + 2 * (3 * FC_MAXA + 8)) * sizeof(int) +
-           (F6_WIN + R) * sizeof(unsigned short) + 2 * R;
+    const size_t R = (size_t)f64_pad(amax * amax), RJ = (size_t)f64_pool(amax);
+    return (R + RJ) * 2 * sizeof(double2) +
+           (F6_AP + FC_MAXC * F6_SST + FC_MAXA + F6_JA) * sizeof(double) +
+           (F6_AP + F6_BUCKETS * F6_CHUNKS + 2 * (F6_JM + 2) + 4 + 4 * (FC_MAXA + F6_JA)) *
+               sizeof(int) +
+           (F6_WIN + F6_AP) * sizeof(unsigned short) + R + RJ;
 }
 // the self kernel: one side and the table
 inline size_t f64_self_smem_bytes(int amax) {
     const size_t R = (size_t)f64_pad(amax * amax);
     return R * 2 * sizeof(double2) + (FC_MAXC * F6_SST + FC_MAXA) * sizeof(double) +
-           (3 * FC_MAXA + 8) * sizeof(int) + R;
+           4 * FC_MAXA * sizeof(int) + R;
+}
+
+__device__ __forceinline__ int *f64_atoms(F64Side &s, int *q, int atoms) {
+    s.off = q;
+    s.end = q + atoms;
+    s.acls = q + 2 * atoms;
+    s.asc = q + 3 * atoms;
+    return q + 4 * atoms;
 }
 
 __device__ __forceinline__ F64View f64_view(unsigned char *p, int amax) {
-    const int R = f64_pad(amax * amax);
+    const int R = f64_pad(amax * amax), RJ = f64_pool(amax);
     F64View v;
     v.i.A = reinterpret_cast<double2 *>(p);
     v.i.B = v.i.A + R;
     v.j.A = v.i.B + R;
-    v.j.B = v.j.A + R;
-    v.l2 = reinterpret_cast<double *>(v.j.B + R);
-    v.st = v.l2 + R;
-    v.red = v.st + FC_MAXC * F6_SST;
-    v.i.self = v.red + (F6_TPB / 32) * MAXSIG;
+    v.j.B = v.j.A + RJ;
+    v.l2 = reinterpret_cast<double *>(v.j.B + RJ);
+    v.st = v.l2 + F6_AP;
+    v.i.self = v.st + FC_MAXC * F6_SST;
     v.j.self = v.i.self + FC_MAXA;
-    v.tot = reinterpret_cast<int *>(v.j.self + FC_MAXA);
-    v.bucket = v.tot + R;
-    int *q = v.bucket + F6_BUCKETS + 8;
-    for (F64Side *s : {&v.i, &v.j}) {
-        s->off = q;
-        s->acls = q + FC_MAXA + 8;
-        s->asc = s->acls + FC_MAXA;
-        q += 3 * FC_MAXA + 8;
-    }
+    v.tot = reinterpret_cast<int *>(v.j.self + F6_JA);
+    v.rank = v.tot + F6_AP;
+    v.jatom = v.rank + F6_BUCKETS * F6_CHUNKS;
+    v.jrec = v.jatom + F6_JM + 2;
+    v.ctl = v.jrec + F6_JM + 2;
+    int *q = f64_atoms(v.i, v.ctl + 4, FC_MAXA);
+    q = f64_atoms(v.j, q, F6_JA);
     v.win = reinterpret_cast<unsigned short *>(q);
     v.perm = v.win + F6_WIN;
-    v.i.C = reinterpret_cast<unsigned char *>(v.perm + R);
+    v.i.C = reinterpret_cast<unsigned char *>(v.perm + F6_AP);
     v.j.C = v.i.C + R;
     return v;
 }
 
-// Whole CTA (of any size >= 32): molecule m's records and atoms. Synchronises
-// between the offsets and the records; the caller synchronises after.
-__device__ void f64_load(const F64Side &s, const double *__restrict__ X, const SetWs &w, int m,
-                         int amax, int n, bool use_self) {
-    const size_t mol = (size_t)m * amax;
-    if (threadIdx.x < 32) {
-        const int a = threadIdx.x;
-        const int cnt = a < n ? w.nnb[mol + a] : 0;
-        int incl = cnt;
-        for (int d = 1; d < 32; d <<= 1) {
-            const int o = __shfl_up_sync(0xffffffffu, incl, d);
-            if (a >= d) incl += o;
-        }
-        s.off[a] = incl - cnt;
-        if (a == 31) s.off[32] = incl;
+// One warp: the record ranges of molecule m's n atoms, from entry `atom` of the
+// side's lists and record `rec` on.
+__device__ __forceinline__ void f64_offsets(const F64Side &s, const SetWs &w, int m, int amax, int n,
+                                            int atom, int rec) {
+    const int a = threadIdx.x & 31;
+    const int cnt = a < n ? w.nnb[(size_t)m * amax + a] : 0;
+    int incl = cnt;
+    for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, incl, d);
+        if (a >= d) incl += o;
     }
-    __syncthreads();
+    if (a < n) {
+        s.off[atom + a] = rec + incl - cnt;
+        s.end[atom + a] = rec + incl;
+    }
+}
+
+// Whole CTA (of any size): molecule m's records and atoms, its ranges being set.
+__device__ __forceinline__ void f64_load(const F64Side &s, const double *__restrict__ X,
+                                         const SetWs &w, int m, int amax, int n, int atom,
+                                         bool use_self) {
+    const size_t mol = (size_t)m * amax;
     for (int t = threadIdx.x; t < n * amax; t += blockDim.x) {
         const int a = t / amax, k = t - a * amax;
-        const int beg = s.off[a];
-        if (k < s.off[a + 1] - beg) {
+        const int at = s.off[atom + a] + k;
+        if (at < s.end[atom + a]) {
             const double *x = X + (mol + a) * 5 * amax + k;
-            s.A[beg + k] = make_double2(x[0], w.xi[(mol + a) * amax + k]);
-            s.B[beg + k] = make_double2(x[3 * amax], x[4 * amax]);
-            s.C[beg + k] = (unsigned char)w.cls[(mol + a) * amax + k];
+            s.A[at] = make_double2(x[0], w.xi[(mol + a) * amax + k]);
+            s.B[at] = make_double2(x[3 * amax], x[4 * amax]);
+            s.C[at] = (unsigned char)w.cls[(mol + a) * amax + k];
         }
     }
     for (int a = threadIdx.x; a < n; a += blockDim.x) {
-        s.self[a] = use_self ? w.self[mol + a] : 0.0;
-        s.acls[a] = w.acls[mol + a];
-        s.asc[a] = w.asc[mol + a];
+        s.self[atom + a] = use_self ? w.self[mol + a] : 0.0;
+        s.acls[atom + a] = w.acls[mol + a];
+        s.asc[atom + a] = w.asc[mol + a];
     }
 }
 
@@ -1077,7 +1130,7 @@ __device__ __forceinline__ void f64_load_table(double *st, const ClassInfo *ci) 
 __device__ __forceinline__ double f64_term(double t, double inv_width, const double2 &A1,
                                            const double2 &B1, const double2 &A2, const double2 &B2,
                                            double st) {
-    double d = __dmul_rn(__dmul_rn(exp(__dmul_rn(t, inv_width)), A1.y), A2.y);
+    double d = __dmul_rn(__dmul_rn(exp_window(__dmul_rn(t, inv_width)), A1.y), A2.y);
     d = __dmul_rn(d, st);
     const double ang = __dadd_rn(__dadd_rn(1.0, __dmul_rn(B1.x, B2.x)), __dmul_rn(B1.y, B2.y));
     return __dmul_rn(d, ang);
@@ -1097,20 +1150,20 @@ arad_f64_self_kernel(const double *__restrict__ X, SetWs w, const int *__restric
     s.B = s.A + R;
     double *st = reinterpret_cast<double *>(s.B + R);
     s.self = st + FC_MAXC * F6_SST;
-    s.off = reinterpret_cast<int *>(s.self + FC_MAXA);
-    s.acls = s.off + FC_MAXA + 8;
-    s.asc = s.acls + FC_MAXA;
-    s.C = reinterpret_cast<unsigned char *>(s.asc + FC_MAXA);
+    s.C = reinterpret_cast<unsigned char *>(
+        f64_atoms(s, reinterpret_cast<int *>(s.self + FC_MAXA), FC_MAXA));
     const int n = min(max(N[m], 0), amax), a = threadIdx.x;
     f64_load_table(st, ci);
-    f64_load(s, X, w, m, amax, n, false);
+    f64_offsets(s, w, m, amax, n, 0, 0);
+    __syncthreads();
+    f64_load(s, X, w, m, amax, n, 0, false);
     __syncthreads();
     if (a >= n) return;
     double sum = 0.0;
-    for (int k1 = s.off[a]; k1 < s.off[a + 1]; ++k1) {
+    for (int k1 = s.off[a]; k1 < s.end[a]; ++k1) {
         const double2 A1 = s.A[k1], B1 = s.B[k1];
         const double *strow = st + s.C[k1] * F6_SST;
-        for (int k2 = s.off[a]; k2 < s.off[a + 1]; ++k2) {
+        for (int k2 = s.off[a]; k2 < s.end[a]; ++k2) {
             const double2 A2 = s.A[k2];
             const double dr = __dsub_rn(A2.x, A1.x);
             const double t = __dmul_rn(dr, dr);
@@ -1122,8 +1175,8 @@ arad_f64_self_kernel(const double *__restrict__ X, SetWs w, const int *__restric
 }
 
 // Sum of atom pair ap = (i1, j1) of a chunk of nap over its runs, in (m1, m2)
-// order. kTest: some list
-// of J does not ascend, so terms outside the window occur in the runs.
+// order. kTest: some list of J does not ascend, so terms outside the window
+// occur in the runs.
 template <bool kTest>
 __device__ __forceinline__ double f64_pair_sum(const F64View &v, int i1, int j1, int ap, int nap,
                                                const AradParams &P) {
@@ -1156,94 +1209,146 @@ __device__ __forceinline__ double f64_pair_sum(const F64View &v, int i1, int j1,
     return sum;
 }
 
-// bm x bm molecule block per CTA.
-__global__ void __launch_bounds__(F6_TPB, 4)
+// Molecule I = blockIdx / nbj against the bj molecules J of block blockIdx % nbj.
+__global__ void __launch_bounds__(F6_TPB, 2)
 arad_f64_pair_kernel(const double *__restrict__ X1, SetWs w1, const int *__restrict__ N1, int nm1,
                      const double *__restrict__ X2, SetWs w2, const int *__restrict__ N2, int nm2,
                      int amax, AradParams P, const ClassInfo *ci,
-                     const __grid_constant__ SigmaTable sig, int nsig, int symmetric, int bm,
+                     const __grid_constant__ SigmaTable sig, int nsig, int symmetric, int bj,
                      double *__restrict__ K) {
     extern __shared__ __align__(16) unsigned char fc_smem_raw[];
     if (ci->flag) return;
+    const int nbj = (nm2 + bj - 1) / bj;
+    const int I = (int)(blockIdx.x / nbj), jb = (int)(blockIdx.x % nbj);
+    const int jend = min(nm2, (jb + 1) * bj);
+    if (symmetric && jend <= I) return;  // below the diagonal
     const F64View v = f64_view(fc_smem_raw, amax);
-    int bi, bj;
-    pair_block(blockIdx.x, symmetric, (nm2 + bm - 1) / bm, bi, bj);
-    f64_load_table(v.st, ci);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int il = 0; il < bm; ++il) {
-        const int I = bi * bm + il;
-        if (I >= nm1) break;
-        const int nI = min(max(N1[I], 0), amax);
-        __syncthreads();  // the previous pair is done with shared memory
-        f64_load(v.i, X1, w1, I, amax, nI, true);
-        for (int jl = 0; jl < bm; ++jl) {
-            const int J = bj * bm + jl;
-            if (J >= nm2) break;
-            if (symmetric && J < I) continue;
-            const int nJ = min(max(N2[J], 0), amax);
+    const int nI = min(max(N1[I], 0), amax);
+    f64_load_table(v.st, ci);
+    if (warp == 1) f64_offsets(v.i, w1, I, amax, nI, 0, 0);
+    __syncthreads();
+    f64_load(v.i, X1, w1, I, amax, nI, 0, true);
+    int J0 = symmetric ? max(jb * bj, I) : jb * bj;
+    while (J0 < jend) {
+        // as many molecules J as fit (the first always does); a lane each
+        if (warp == 0) {
+            const bool in = lane < F6_JM && J0 + lane < jend;
+            const int n = in ? min(max(N2[J0 + lane], 0), amax) : 0;
+            int atoms = n, recs = n * n;
+            for (int d = 1; d < 32; d <<= 1) {
+                const int oa = __shfl_up_sync(0xffffffffu, atoms, d);
+                const int orc = __shfl_up_sync(0xffffffffu, recs, d);
+                if (lane >= d) {
+                    atoms += oa;
+                    recs += orc;
+                }
+            }
+            const bool fits = in && atoms * nI <= F6_AP && atoms <= F6_JA && recs <= f64_pool(amax);
+            const int nj = __ffs(~__ballot_sync(0xffffffffu, fits || lane == 0)) - 1;
+            int big = lane < nj ? n : 0;
+            for (int d = 16; d; d >>= 1) big = max(big, __shfl_xor_sync(0xffffffffu, big, d));
+            if (lane <= nj) {
+                v.jatom[lane] = atoms - n;
+                v.jrec[lane] = recs - n * n;
+            }
+            if (lane == 0) {
+                v.ctl[0] = nj;
+                v.ctl[1] = big;
+            }
+        }
+        __syncthreads();
+        const int nj = v.ctl[0], big = v.ctl[1], natom = v.jatom[nj];
+        if (warp < nj)
+            f64_offsets(v.j, w2, J0 + warp, amax, v.jatom[warp + 1] - v.jatom[warp],
+                        v.jatom[warp], v.jrec[warp]);
+        __syncthreads();
+        for (int b = 0; b < nj; ++b)
+            f64_load(v.j, X2, w2, J0 + b, amax, v.jatom[b + 1] - v.jatom[b], v.jatom[b], true);
+        const int jstep = nI > 0 ? F6_WIN / (nI * nI) : F6_JA;
+        for (int j0 = 0; j0 < natom; j0 += jstep) {
+            const int jn = min(jstep, natom - j0), nap = nI * jn;
+            for (int t = tid; t < F6_BUCKETS * F6_CHUNKS; t += F6_TPB) v.rank[t] = 0;
+            if (tid == 0) v.ctl[2] = 0;
             __syncthreads();
-            f64_load(v.j, X2, w2, J, amax, nJ, true);
-            const int jstep = nI > 0 ? F6_WIN / (nI * nI) : FC_MAXA;
-            for (int j0 = 0; j0 < nJ; j0 += jstep) {
-                const int jn = min(jstep, nJ - j0), nap = nI * jn;
-                if (tid < F6_BUCKETS) v.bucket[tid] = 0;
-                __syncthreads();
-                // 1. the runs; atom pair ap = (j1 - j0) nI + i1, a thread each. Both
-                // ends of the window only move up while r1 ascends.
-                for (int ap = tid; ap < nap; ap += F6_TPB) {
-                    const int jq = ap / nI, i1 = ap - jq * nI, j1 = j0 + jq;
-                    const double2 *J2 = v.j.A + v.j.off[j1];
-                    const int cnt = v.j.off[j1 + 1] - v.j.off[j1], k1 = v.i.off[i1];
-                    const bool ascends = v.j.asc[j1] != 0;
-                    int lo = 0, hi = ascends ? 0 : cnt, total = 0;
-                    double before = 0.0;
-                    for (int m1 = 0; m1 < v.i.off[i1 + 1] - k1; ++m1) {
-                        const double r1 = v.i.A[k1 + m1].x;
-                        if (ascends) {
-                            if (!(r1 >= before)) lo = hi = 0;
-                            before = r1;
-                            while (lo < cnt) {  // to the first neighbour not below the window
-                                const double dr = __dsub_rn(J2[lo].x, r1);
-                                if (!(dr < 0.0) || __dmul_rn(dr, dr) < P.maxg2) break;
-                                ++lo;
-                            }
-                            hi = max(hi, lo);
-                            while (hi < cnt) {  // to the first neighbour above it
-                                const double dr = __dsub_rn(J2[hi].x, r1);
-                                if (!(dr < 0.0) && !(__dmul_rn(dr, dr) < P.maxg2)) break;
-                                ++hi;
-                            }
+            // 1. the runs; atom pair ap = (j1 - j0) nI + i1, a thread each. Both
+            // ends of the window only move up while r1 ascends.
+            for (int ap = tid; ap < nap; ap += F6_TPB) {
+                const int jq = ap / nI, i1 = ap - jq * nI, j1 = j0 + jq;
+                const double2 *J2 = v.j.A + v.j.off[j1];
+                const int cnt = v.j.end[j1] - v.j.off[j1], k1 = v.i.off[i1];
+                const bool ascends = v.j.asc[j1] != 0;
+                int lo = 0, hi = ascends ? 0 : cnt, total = 0;
+                double before = 0.0;
+                for (int m1 = 0; m1 < v.i.end[i1] - k1; ++m1) {
+                    const double r1 = v.i.A[k1 + m1].x;
+                    if (ascends) {
+                        if (!(r1 >= before)) lo = hi = 0;
+                        before = r1;
+                        while (lo < cnt) {  // to the first neighbour not below the window
+                            const double dr = __dsub_rn(J2[lo].x, r1);
+                            if (!(dr < 0.0) || __dmul_rn(dr, dr) < P.maxg2) break;
+                            ++lo;
                         }
-                        v.win[m1 * nap + ap] = (unsigned short)(lo | ((hi - lo) << 8));
-                        total += hi - lo;
+                        hi = max(hi, lo);
+                        while (hi < cnt) {  // to the first neighbour above it
+                            const double dr = __dsub_rn(J2[hi].x, r1);
+                            if (!(dr < 0.0) && !(__dmul_rn(dr, dr) < P.maxg2)) break;
+                            ++hi;
+                        }
                     }
-                    v.tot[ap] = total;
+                    v.win[m1 * nap + ap] = (unsigned short)(lo | ((hi - lo) << 8));
+                    total += hi - lo;
                 }
-                const bool test = __syncthreads_or(tid < jn && !v.j.asc[j0 + tid]);
-                // 2. atom pairs by number of terms, largest first (which lane
-                // takes a pair does not change its sum)
-                auto bucket_of = [&](int ap) {
-                    return F6_BUCKETS - 1 -
-                           min(F6_BUCKETS - 1, v.tot[ap] * F6_BUCKETS / (nI * nJ));
-                };
-                for (int t = tid; t < nap; t += F6_TPB) atomicAdd(&v.bucket[bucket_of(t)], 1);
-                __syncthreads();
-                if (warp == 0) {  // exclusive prefix over the 64 buckets
-                    const int b0 = v.bucket[2 * lane], b1 = v.bucket[2 * lane + 1];
-                    int incl = b0 + b1;
-                    for (int d = 1; d < 32; d <<= 1) {
-                        const int o = __shfl_up_sync(0xffffffffu, incl, d);
-                        if (lane >= d) incl += o;
-                    }
-                    v.bucket[2 * lane] = incl - b0 - b1;
-                    v.bucket[2 * lane + 1] = incl - b1;
+                v.tot[ap] = total;
+            }
+            const bool test = __syncthreads_or(tid < jn && !v.j.asc[j0 + tid]);
+            // 2. the order: per 32 pairs the count of each bucket (most terms
+            // first), an exclusive prefix over buckets and 32s, then the places
+            int bucket[F6_AP / F6_TPB], place[F6_AP / F6_TPB];
+#pragma unroll
+            for (int q = 0; q < F6_AP / F6_TPB; ++q) {
+                const int ap = tid + q * F6_TPB;
+                const bool in = ap < nap;
+                bucket[q] = in ? F6_BUCKETS - 1 -
+                                     min(F6_BUCKETS - 1, v.tot[ap] * F6_BUCKETS / (nI * big))
+                               : F6_BUCKETS;
+                const unsigned same = __match_any_sync(0xffffffffu, bucket[q]);
+                place[q] = __popc(same & ((1u << lane) - 1));
+                if (in && place[q] == 0) v.rank[bucket[q] * F6_CHUNKS + (ap >> 5)] = __popc(same);
+            }
+            __syncthreads();
+            static_assert(F6_BUCKETS * F6_CHUNKS == 2 * F6_TPB, "two entries per thread");
+            {
+                const int c0 = v.rank[2 * tid], c1 = v.rank[2 * tid + 1];
+                int incl = c0 + c1;
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int o = __shfl_up_sync(0xffffffffu, incl, d);
+                    if (lane >= d) incl += o;
                 }
+                __shared__ int part[F6_TPB / 32];
+                if (lane == 31) part[warp] = incl;
                 __syncthreads();
-                for (int t = tid; t < nap; t += F6_TPB)
-                    v.perm[atomicAdd(&v.bucket[bucket_of(t)], 1)] = (unsigned short)t;
-                __syncthreads();
-                // 3. the sums and l2
-                for (int t = tid; t < nap; t += F6_TPB) {
+                int before = 0;
+                for (int q = 0; q < warp; ++q) before += part[q];
+                v.rank[2 * tid] = before + incl - c0 - c1;
+                v.rank[2 * tid + 1] = before + incl - c1;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < F6_AP / F6_TPB; ++q) {
+                const int ap = tid + q * F6_TPB;
+                if (ap < nap)
+                    v.perm[v.rank[bucket[q] * F6_CHUNKS + (ap >> 5)] + place[q]] =
+                        (unsigned short)ap;
+            }
+            __syncthreads();
+            // 3. the sums and l2 (which warp takes a pair does not change its sum)
+            for (;;) {
+                int t = lane == 0 ? atomicAdd(&v.ctl[2], 32) : 0;
+                t = __shfl_sync(0xffffffffu, t, 0) + lane;
+                if (t - lane >= nap) break;
+                if (t < nap) {
                     const int ap = v.perm[t], jq = ap / nI, i1 = ap - jq * nI, j1 = j0 + jq;
                     const double S = test ? f64_pair_sum<true>(v, i1, j1, ap, nap, P)
                                           : f64_pair_sum<false>(v, i1, j1, ap, nap, P);
@@ -1253,31 +1358,30 @@ arad_f64_pair_kernel(const double *__restrict__ X1, SetWs w1, const int *__restr
                     if (fabs(l2) < P.eps) l2 = 0.0;  // farad_kernels.f90:594
                     v.l2[j0 * nI + ap] = l2;
                 }
-                __syncthreads();
-            }
-            const int nall = nI * nJ;
-            // 4. the kernel exponentials
-            for (int s = 0; s < nsig; ++s) {
-                double e = 0.0;
-                for (int t = tid; t < nall; t += F6_TPB) e += exp(v.l2[t] * sig.inv_sigma2[s]);
-                for (int o = 16; o; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-                if (lane == 0) v.red[warp * MAXSIG + s] = e;
+                __syncwarp();
             }
             __syncthreads();
-            if (tid < nsig) {
-                double e = 0.0;
-                for (int q = 0; q < F6_TPB / 32; ++q) e += v.red[q * MAXSIG + tid];
-                K[((size_t)tid * nm1 + I) * nm2 + J] = e;
-                if (symmetric) K[((size_t)tid * nm1 + J) * nm2 + I] = e;
+        }
+        // 4. the kernel exponentials, a warp per molecule J and sigma
+        for (int q = warp; q < nj * nsig; q += F6_TPB / 32) {
+            const int b = q / nsig, s = q - b * nsig, J = J0 + b;
+            const int beg = v.jatom[b] * nI, end = v.jatom[b + 1] * nI;
+            double e = 0.0;
+            for (int t = beg + lane; t < end; t += 32) e += exp(v.l2[t] * sig.inv_sigma2[s]);
+            for (int o = 16; o; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+            if (lane == 0) {
+                K[((size_t)s * nm1 + I) * nm2 + J] = e;
+                if (symmetric) K[((size_t)s * nm1 + J) * nm2 + I] = e;
             }
         }
+        __syncthreads();  // the next molecules overwrite these
+        J0 += nj;
     }
 }
 
-// Molecule block of the FP64 pair kernel: 2 x 2 once the blocks fill the GPU
-// several times over (each molecule is then staged for two pairs), else one
-// pair per CTA.
-inline int f64_block(long long npairs) { return npairs >= (1LL << 13) ? 2 : 1; }
+// Molecules J of a CTA: four, about what its shared memory holds at a time, once
+// such blocks fill the GPU several times over.
+inline int f64_block(long long npairs) { return npairs >= (1LL << 13) ? 4 : 1; }
 
 // The fast kernels' shared memory is dynamic (above the 48 KB static limit);
 // the attribute is set once per device.
@@ -1549,12 +1653,11 @@ static int arad_kernels_impl(const double *X1, const double *Z1, const int *N1, 
         double *Ks = K + (size_t)s0 * nm1 * nm2;
         if (precision == 0) {
             if (try_fast) {
-                const int bm = f64_block(npairs);
-                const long long nbi = ceil_div(nm1, bm), nbj = ceil_div(nm2, bm);
-                const long long nblk = symmetric ? nbi * (nbi + 1) / 2 : nbi * nbj;
+                const int bj = f64_block(npairs);
+                const long long nblk = (long long)nm1 * ceil_div(nm2, bj);
                 FMLB_REQUIRE(nblk < (1LL << 31), "fmlb_arad_kernels: too many molecule blocks");
                 arad_f64_pair_kernel<<<(unsigned)nblk, F6_TPB, f64_smem_bytes(amax), st>>>(
-                    X1, w1, N1, nm1, X2, w2, N2, nm2, amax, P, ci, sig, ns, symmetric, bm, Ks);
+                    X1, w1, N1, nm1, X2, w2, N2, nm2, amax, P, ci, sig, ns, symmetric, bj, Ks);
                 FMLB_TRY(launch_status("arad_f64_pair_kernel"));
             }
             arad_pair_kernel<true><<<blocks, tpb, 0, st>>>(X1, Z1, N1, w1, nm1, X2, Z2, N2, w2, nm2,
