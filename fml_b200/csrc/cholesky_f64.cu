@@ -1229,8 +1229,11 @@ extern "C" int fmlb_potrf_f64(double *A, long long lda, int n, void *work, int *
 extern "C" size_t fmlb_potrf_ozaki_workspace_bytes(int n, int nslices) {
     if (n <= 0 || nslices <= 0) return 256;
     const int W = outer_width(n);
-    return (fmlb_potrf_workspace_bytes(n) + 255) / 256 * 256 +
-           fmlb::ozaki_slice_bytes(n, W, nslices);
+    // a multiple of 256, so that workspaces laid side by side stay aligned (the
+    // digit data of an odd n ends on 4 bytes, and a second workspace right behind
+    // it held its doubles misaligned)
+    return ((fmlb_potrf_workspace_bytes(n) + 255) / 256 * 256 +
+            fmlb::ozaki_slice_bytes(n, W, nslices) + 255) / 256 * 256;
 }
 
 extern "C" int fmlb_potrf_ozaki_f64(double *A, long long lda, int n, int nslices, void *work,
