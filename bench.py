@@ -1182,7 +1182,7 @@ class PlainLoop:
                     arad_launches(False, "fp64", st["amax"], 1) + 1
             else:
                 c += 1 + 2
-            c += 1 + potrf_launches(n) + 2 * -(-n // 128)
+            c += 1 + potrf_launches(n) + 2
         return c
 
     def run(self):

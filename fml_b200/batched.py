@@ -329,7 +329,7 @@ class BatchedKRR:
             r = self.recs[i]
             n = int(r["n"])
             count += (1 if int(r["kind"]) == 0 else 0) + 1 + potrf_launches(n) + \
-                2 * -(-n // 128) + (1 if int(r["nt"]) else 0)
+                2 + (1 if int(r["nt"]) else 0)
             if int(r["kind"]) == 0 and int(r["nt"]):
                 count += 1  # the prediction's chunk reduction
         return count

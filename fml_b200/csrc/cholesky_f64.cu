@@ -43,9 +43,7 @@ __device__ __forceinline__ bool failed(const int *info) {
 // completed and its writes are visible, so every read of data that kernel
 // may write comes after it. The panel chain (diagonal block, panel solve,
 // update inside the outer panel) signals its dependent only at its end, so
-// the next kernel's CTAs do not sit on SMs the concurrent bulk update needs;
-// the solve's step kernels signal at their start and read their rows of the
-// factor, which no step writes, before waiting.
+// the next kernel's CTAs do not sit on SMs the concurrent bulk update needs.
 __device__ __forceinline__ void pdl_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
@@ -655,217 +653,194 @@ int launch_syrk(double *C, long long ldc, int m, const double *P, long long ldp,
 }
 
 // ---- 4. triangular solves with the factor (potrs) ---------------------------
-// Right-looking, one launch per 128-block column and direction. Every thread
-// block reads its rows (forward) or columns (backward) of the factor once,
-// coalesced; the block that owns the next diagonal block also applies that
-// block's stored inverse, so the next launch starts from a finished
-// sub-vector. All reductions run in a fixed order (deterministic).
-constexpr int SOLVE_WARPS = TPB / 32;
+// One launch per direction. A CTA takes one block of 128 unknowns, in the order
+// of the substitution by a ticket, and sums the contributions of the blocks
+// before it as they appear:
+//   forward   y_k = Linv_k (b_k - sum_{j < k} L_kj y_j)
+//   backward  x_k = Linv_k^T (y_k - sum_{j > k} L_jk^T x_j)
+// The next 128 x 128 block of the factor is loaded into registers before its
+// vector block is waited for. A vector block is its own flag: the vector is
+// filled with a bit pattern that no result has, and a reader polls each value
+// until it is another. A CTA waits only for blocks that CTAs with lower tickets,
+// started before it, own, so the first unfinished block can always proceed. All
+// sums run in a fixed order (deterministic).
+//
+// Bound by the chain of n / 128 blocks per direction: one block's value through
+// L2, 128 x 128 products with it and with the block inverse (kept in shared
+// memory), about 1.5 us; a launch per block and direction took 6.5 us.
+constexpr int SV_WARPS = TPB / 32, SV_ROWS = NB / SV_WARPS;  // 8 warps of 16 rows
+constexpr size_t kSolveSmem = ((size_t)NB * NB + (size_t)SV_WARPS * NB + 3 * NB) * sizeof(double);
+constexpr size_t kSolveCounterBytes = 2 * sizeof(unsigned);  // behind y in the workspace
+constexpr unsigned long long kSolveUnset = ~0ull;   // what a byte-wise fill with 0xff leaves
+constexpr long long kSolveBudget = 4000000000LL;    // clock cycles of a wait (~2 s)
 
-constexpr int FWD_ROWS = 32;   // rows per thread block past the next diagonal block
-constexpr int BWD_COLS = 32;   // columns per thread block before the previous one
-
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+// The value at p once it is set; NaN when the wait runs out (the solution then
+// holds NaN from there on).
+__device__ __forceinline__ double solve_wait(const double *p) {
+    const long long t0 = clock64();
+    for (;;) {
+        unsigned long long u;
+        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(u) : "l"(p) : "memory");
+        if (u != kSolveUnset) return __longlong_as_double((long long)u);
+        if (clock64() - t0 > kSolveBudget) return __longlong_as_double(0x7ff8000000000000LL);
+    }
+}
+__device__ __forceinline__ void solve_publish(double *p, double v) {
+    unsigned long long u = (unsigned long long)__double_as_longlong(v);
+    if (u == kSolveUnset) u = 0x7ff8000000000000ull;  // a NaN like any other
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(u) : "memory");
 }
 
-// out[t] = sum_{c <= t} Linv[t][c] in[c], t < kn (lower-triangular block
-// inverse, row-major 128 x 128); warp per row, four rows in flight per warp.
-__device__ __forceinline__ void tri_lower_apply(const double *__restrict__ Linv,
-                                                const double *in, double *out, int kn) {
+// This CTA's place in the order (the counter starts at 0xffffffff).
+__device__ __forceinline__ int solve_ticket(unsigned *counter) {
+    __shared__ int place;
+    if (threadIdx.x == 0) place = (int)(atomicAdd(counter, 1u) + 1u);
+    __syncthreads();
+    return place;
+}
+
+// The block inverse (zeros above the diagonal) into shared memory, asynchronously.
+__device__ __forceinline__ void solve_load_inverse(double *Li, const double *__restrict__ Linv) {
+    for (int t = threadIdx.x; t < NB * NB; t += TPB) cp_async_8(Li + t, Linv + t, 8);
+    cp_async_commit();
+}
+
+// Rows warp * 16 .. + 15 of a 128 x 128 block, columns lane + 32 i: rows past
+// `rows` and columns past `cols` as zeros.
+__device__ __forceinline__ void solve_load_rows(double (&lv)[SV_ROWS][NB / 32],
+                                                const double *__restrict__ block, long long lda,
+                                                int rows, int cols) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int t0 = warp; t0 < kn; t0 += 4 * SOLVE_WARPS) {
-        double s[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int t = t0 + q * SOLVE_WARPS;
-            s[q] = 0.0;
+    for (int r = 0; r < SV_ROWS; ++r)
 #pragma unroll
-            for (int i = 0; i < NB / 32; ++i) {
-                const int c = lane + 32 * i;
-                if (t < kn && c <= t) s[q] = fma(Linv[t * NB + c], in[c], s[q]);
-            }
+        for (int i = 0; i < NB / 32; ++i) {
+            const int row = warp * SV_ROWS + r, c = lane + 32 * i;
+            lv[r][i] = row < rows && c < cols ? block[(size_t)row * lda + c] : 0.0;
         }
+}
+
+// Sums of a[0 .. 15] over the warp's lanes: lane l returns that of a[l / 2].
+__device__ __forceinline__ double warp_sums16(double (&a)[SV_ROWS]) {
+    const int lane = threadIdx.x & 31;
+    static_assert(SV_ROWS == 16, "four halvings");
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const double v = warp_sum(s[q]);
-            const int t = t0 + q * SOLVE_WARPS;
-            if (lane == 0 && t < kn) out[t] = v;
+    for (int m = 8; m >= 1; m >>= 1) {
+        const bool up = lane & (2 * m);
+#pragma unroll
+        for (int q = 0; q < m; ++q) {
+            const double give = up ? a[q] : a[q + m], keep = up ? a[q + m] : a[q];
+            a[q] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * m);
         }
     }
+    return a[0] + __shfl_xor_sync(0xffffffffu, a[0], 1);
 }
 
-// out[t] = sum_{r >= t} Linv[r][t] in[r], t < kn (the transposed inverse);
-// thread t with 2 row halves reduced through shared memory.
-__device__ __forceinline__ void tri_upper_apply(const double *__restrict__ Linv,
-                                                const double *in, double *out, int kn,
-                                                double *red) {
-    const int t = threadIdx.x & (NB - 1), h = threadIdx.x >> 7;  // TPB = 2 NB
-    double s = 0.0;
-    if (t < kn) {
-        const int r1 = min(kn, (h + 1) * (NB / 2));
-#pragma unroll 32
-        for (int r = h * (NB / 2); r < r1; ++r)
-            if (r >= t) s = fma(Linv[r * NB + t], in[r], s);
-    }
-    red[threadIdx.x] = s;
-    __syncthreads();
-    if (h == 0 && t < kn) out[t] = red[t] + red[t + NB];
-}
-
-// y[0..kn) = Linv_0 x[0..kn)
-__global__ void __launch_bounds__(TPB)
-solve_first_forward_kernel(const double *__restrict__ Linv0, const double *__restrict__ x,
-                           double *__restrict__ y, int kn) {
-    tri_lower_apply(Linv0, x, y, kn);
-}
-
-// x[k0..k0+kn) = Linv_k^T y[k0..k0+kn)
-__global__ void __launch_bounds__(TPB)
-solve_first_backward_kernel(const double *__restrict__ Linvk, const double *__restrict__ y,
-                            double *__restrict__ x, int kn) {
-    __shared__ double red[TPB];
-    pdl_launch_dependents();
-    pdl_wait();
-    tri_upper_apply(Linvk, y, x, kn, red);
-}
-
-// L2 prefetch of a 128 x 128 block (the next diagonal block's inverse), so
-// that the owner block's final step reads it from L2
-__device__ __forceinline__ void prefetch_block_l2(const double *p) {
-    for (int t = threadIdx.x; t < NB * NB / 16; t += blockDim.x)  // one 128-byte line each
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(p + (size_t)t * 16));
-}
-
-// Forward step for block column k (y_k final): x[r] -= L[r, k0:k0+kn] y_k for
-// r >= k0 + kn. Thread block 0 owns the next diagonal block and then writes
-// y_{k+1} = Linv_{k+1} x_{k+1}. Every lane reads its four entries of y_k
-// directly, so a warp's row loads, y_k loads and x loads all go out together;
-// each warp keeps eight rows in flight.
-__global__ void __launch_bounds__(TPB)
-forward_step_kernel(const double *__restrict__ L, long long lda, int n, int k0, int kn,
-                    const double *__restrict__ LinvNext, double *__restrict__ x,
-                    double *__restrict__ y) {
-    __shared__ double xn[NB];
+__global__ void __launch_bounds__(TPB, 1)
+solve_forward_kernel(const double *__restrict__ L, long long lda, int n,
+                     const double *__restrict__ Linv, const double *__restrict__ b,
+                     double *y, unsigned *counter) {
+    extern __shared__ __align__(16) double sv_smem[];
+    double *Li = sv_smem, *v = Li + NB * NB, *yb = v + NB;  // yb: two blocks
+    const int k = solve_ticket(counter), k0 = k * NB, kn = min(NB, n - k0);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const bool owner = blockIdx.x == 0;
-    pdl_launch_dependents();
-    if (owner && LinvNext != nullptr) prefetch_block_l2(LinvNext);
-    double ykr[NB / 32];
-    bool waited = false;
-    const int nb0 = k0 + kn;
-    int rb, re;
-    if (owner) {
-        rb = nb0;
-        re = min(n, nb0 + NB);
-    } else {
-        rb = nb0 + NB + (blockIdx.x - 1) * FWD_ROWS;
-        re = min(n, rb + FWD_ROWS);
-    }
-    constexpr int G = 8;  // rows per warp in flight
-    for (int r0 = rb + warp; r0 < re; r0 += G * SOLVE_WARPS) {
-        double s[G], xr[G], lv[G][NB / 32];
+    solve_load_inverse(Li, Linv + (size_t)k * NB * NB);
+    const double *rows = L + (size_t)k0 * lda;
+    double lv[SV_ROWS][NB / 32], acc[SV_ROWS];
 #pragma unroll
-        for (int q = 0; q < G; ++q) {  // the factor's rows: not written by any step
-            const int r = r0 + q * SOLVE_WARPS;
-            const bool ok = r < re;
-            const double *row = L + (size_t)min(r, n - 1) * lda + k0;
-#pragma unroll
-            for (int i = 0; i < NB / 32; ++i) {
-                const int c = lane + 32 * i;
-                lv[q][i] = (ok && c < kn) ? row[c] : 0.0;
-            }
-        }
-        if (!waited) {
-            pdl_wait();
-            waited = true;
-#pragma unroll
-            for (int i = 0; i < NB / 32; ++i) {
-                const int c = lane + 32 * i;
-                ykr[i] = c < kn ? y[k0 + c] : 0.0;
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < G; ++q) {
-            const int r = r0 + q * SOLVE_WARPS;
-            const bool ok = r < re;
-            s[q] = 0.0;
-            xr[q] = (ok && lane == 0) ? x[r] : 0.0;
-#pragma unroll
-            for (int i = 0; i < NB / 32; ++i) {
-                const int c = lane + 32 * i;
-                if (ok && c < kn) s[q] = fma(lv[q][i], ykr[i], s[q]);
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < G; ++q) {
-            const double sq = warp_sum(s[q]);
-            const int r = r0 + q * SOLVE_WARPS;
-            if (lane == 0 && r < re) {
-                const double v = xr[q] - sq;
-                x[r] = v;
-                if (owner) xn[r - nb0] = v;
-            }
-        }
-    }
-    if (!waited) pdl_wait();
-    if (owner && LinvNext != nullptr) {
+    for (int r = 0; r < SV_ROWS; ++r) acc[r] = 0.0;
+    if (k > 0) solve_load_rows(lv, rows, lda, kn, NB);
+    for (int j = 0; j < k; ++j) {
+        double *yj = yb + (j & 1) * NB;
+        if (tid < NB) yj[tid] = solve_wait(y + j * NB + tid);
         __syncthreads();
-        tri_lower_apply(LinvNext, xn, y + nb0, re - rb);
+#pragma unroll
+        for (int i = 0; i < NB / 32; ++i) {
+            const double yv = yj[lane + 32 * i];
+#pragma unroll
+            for (int r = 0; r < SV_ROWS; ++r) acc[r] = fma(lv[r][i], yv, acc[r]);
+        }
+        if (j + 1 < k) solve_load_rows(lv, rows + (j + 1) * NB, lda, kn, NB);
     }
+    const int row = warp * SV_ROWS + (lane >> 1);
+    const double bk = row < kn ? b[k0 + row] : 0.0;
+    double s = warp_sums16(acc);
+    if ((lane & 1) == 0) v[row] = bk - s;
+    cp_async_wait<0>();
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < SV_ROWS; ++r) {
+        double p = 0.0;
+#pragma unroll
+        for (int i = 0; i < NB / 32; ++i)
+            p = fma(Li[(warp * SV_ROWS + r) * NB + lane + 32 * i], v[lane + 32 * i], p);
+        acc[r] = p;
+    }
+    s = warp_sums16(acc);
+    if ((lane & 1) == 0 && row < kn) solve_publish(y + k0 + row, s);
 }
 
-// Backward step for block column k (x_k final): y[j] -= sum_r L[k0 + r, j]
-// x_k[r] for j < k0. Thread block 0 owns the previous diagonal block's 128
-// columns (2 row halves per column) and then writes x_{k-1} = Linv_{k-1}^T
-// y_{k-1}; the others own 32 columns each (8 row groups per column). Partial
-// sums are added in a fixed order.
-__global__ void __launch_bounds__(TPB)
-backward_step_kernel(const double *__restrict__ L, long long lda, int k0, int kn,
-                     const double *__restrict__ LinvPrev, double *__restrict__ y,
-                     double *__restrict__ x) {
-    __shared__ double xk[NB];
-    __shared__ double yp[NB];
-    __shared__ double red[TPB];
-    const int tid = threadIdx.x;
-    const bool owner = blockIdx.x == 0;
-    pdl_launch_dependents();
-    if (owner) prefetch_block_l2(LinvPrev);
-    pdl_wait();
-    if (tid < NB) xk[tid] = tid < kn ? x[k0 + tid] : 0.0;
+// Columns of the warps' partial sums p[i] (columns lane + 32 i), added in warp
+// order: thread c < 128 returns column c's.
+__device__ __forceinline__ double solve_column_sums(double *part, const double (&p)[NB / 32]) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+#pragma unroll
+    for (int i = 0; i < NB / 32; ++i) part[warp * NB + lane + 32 * i] = p[i];
     __syncthreads();
-    const int pb = k0 - NB;  // first column of the previous diagonal block (k0 >= NB here)
-    const int W = owner ? NB : BWD_COLS;          // columns of this thread block
-    const int G = TPB / W;                        // row groups per column
-    const int rows_per = NB / G;
-    const int cb = owner ? pb : (blockIdx.x - 1) * BWD_COLS;
-    const int ce = owner ? k0 : min(pb, cb + BWD_COLS);
-    const int col = tid % W, g = tid / W;
-    const int j = cb + col;
     double s = 0.0;
-    if (j < ce) {
-        const int rbeg = g * rows_per;
-#pragma unroll 32
-        for (int rr = 0; rr < rows_per; ++rr) {
-            const int r = rbeg + rr;
-            if (r < kn) s = fma(L[(size_t)(k0 + r) * lda + j], xk[r], s);
-        }
-    }
-    red[tid] = s;
-    __syncthreads();
-    if (g == 0 && j < ce) {
-        double t = 0.0;
-        for (int q = 0; q < G; ++q) t += red[q * W + col];
-        const double v = y[j] - t;
-        y[j] = v;
-        if (owner) yp[col] = v;
-    }
-    if (owner) {
+    if (tid < NB)
+#pragma unroll
+        for (int w = 0; w < SV_WARPS; ++w) s += part[w * NB + tid];
+    return s;
+}
+
+__global__ void __launch_bounds__(TPB, 1)
+solve_backward_kernel(const double *__restrict__ L, long long lda, int n,
+                      const double *__restrict__ Linv, const double *__restrict__ y, double *x,
+                      unsigned *counter) {
+    extern __shared__ __align__(16) double sv_smem[];
+    double *Li = sv_smem, *v = Li + NB * NB, *xb = v + NB, *part = xb + 2 * NB;
+    const int nblk = (n + NB - 1) / NB;
+    const int k = nblk - 1 - solve_ticket(counter), k0 = k * NB, kn = min(NB, n - k0);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    solve_load_inverse(Li, Linv + (size_t)k * NB * NB);
+    double lv[SV_ROWS][NB / 32], acc[2][NB / 32];
+#pragma unroll
+    for (int i = 0; i < NB / 32; ++i) acc[0][i] = acc[1][i] = 0.0;
+    if (k < nblk - 1)
+        solve_load_rows(lv, L + (size_t)(nblk - 1) * NB * lda + k0, lda, n - (nblk - 1) * NB, NB);
+    for (int j = nblk - 1; j > k; --j) {
+        double *xj = xb + (j & 1) * NB;
+        if (tid < NB) xj[tid] = j * NB + tid < n ? solve_wait(x + j * NB + tid) : 0.0;
         __syncthreads();
-        tri_upper_apply(LinvPrev, yp, x + pb, NB, red);
+#pragma unroll
+        for (int r = 0; r < SV_ROWS; ++r) {
+            const double xv = xj[warp * SV_ROWS + r];
+#pragma unroll
+            for (int i = 0; i < NB / 32; ++i) acc[r & 1][i] = fma(lv[r][i], xv, acc[r & 1][i]);
+        }
+        if (j - 1 > k) solve_load_rows(lv, L + (size_t)(j - 1) * NB * lda + k0, lda, NB, NB);
     }
+    double p[NB / 32];
+#pragma unroll
+    for (int i = 0; i < NB / 32; ++i) p[i] = acc[0][i] + acc[1][i];
+    double s = solve_column_sums(part, p);
+    if (tid < NB) v[tid] = tid < kn ? y[k0 + tid] - s : 0.0;
+    cp_async_wait<0>();
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NB / 32; ++i) acc[0][i] = acc[1][i] = 0.0;
+#pragma unroll
+    for (int r = 0; r < SV_ROWS; ++r) {
+        const double vr = v[warp * SV_ROWS + r];
+#pragma unroll
+        for (int i = 0; i < NB / 32; ++i)
+            acc[r & 1][i] = fma(Li[(warp * SV_ROWS + r) * NB + lane + 32 * i], vr, acc[r & 1][i]);
+    }
+#pragma unroll
+    for (int i = 0; i < NB / 32; ++i) p[i] = acc[0][i] + acc[1][i];
+    s = solve_column_sums(part, p);
+    if (tid < kn) solve_publish(x + k0 + tid, s);
 }
 
 // ---- 5. inverse from the factor (potri) ------------------------------------
@@ -1041,6 +1016,12 @@ int set_smem_attrs() {
     FMLB_TRY(cuda_status(cudaFuncSetAttribute(block_inverse_kernel,
                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)kBlockInvSmem), "block inverse smem attribute"));
+    FMLB_TRY(cuda_status(cudaFuncSetAttribute(solve_forward_kernel,
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)kSolveSmem), "solve smem attribute"));
+    FMLB_TRY(cuda_status(cudaFuncSetAttribute(solve_backward_kernel,
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)kSolveSmem), "solve smem attribute"));
     attr_dev = dev;
     return FMLB_OK;
 }
@@ -1052,7 +1033,7 @@ extern "C" size_t fmlb_potrf_workspace_bytes(int n) {
     if (n <= 0) return 256;
     const size_t nblk = (size_t)(n + fmlb::NB - 1) / fmlb::NB;
     return nblk * fmlb::NB * fmlb::NB * sizeof(double) +
-           ((size_t)n * sizeof(double) + 255) / 256 * 256;
+           ((size_t)n * sizeof(double) + fmlb::kSolveCounterBytes + 255) / 256 * 256;
 }
 
 // Per host thread, device and caller stream: the high-priority stream that
@@ -1266,34 +1247,22 @@ extern "C" int fmlb_potrs_f64(const double *L, long long lda, int n, const void 
     FMLB_REQUIRE(n >= 0 && lda >= n, "fmlb_potrs_f64: bad n=%d / lda=%lld", n, lda);
     if (n == 0) return FMLB_OK;
     FMLB_REQUIRE(L && work && x, "fmlb_potrs_f64: null pointer");
+    FMLB_TRY(set_smem_attrs());
     const double *Linv = static_cast<const double *>(work);
     const size_t nblk = (size_t)(n + NB - 1) / NB;
-    // y lives after the inverted blocks in the workspace (written by potrs only)
+    // y and the two counters live after the inverted blocks in the workspace
+    // (written by potrs only)
     double *y = const_cast<double *>(Linv + nblk * NB * NB);
-    solve_first_forward_kernel<<<1, TPB, 0, st>>>(Linv, x, y, std::min(NB, n));
-    FMLB_TRY(launch_status("solve_first_forward_kernel"));
-    for (int k0 = 0, kb = 0; k0 + NB < n; k0 += NB, ++kb) {
-        const int rest = n - k0 - NB;  // rows past this block column
-        const int grid = 1 + ceil_div(std::max(0, rest - NB), FWD_ROWS);
-        FMLB_TRY(launch_maybe_pdl(true, forward_step_kernel, dim3(grid), dim3(TPB), 0, st,
-                                  "forward_step_kernel", L, lda, n, k0, (int)NB,
-                                  (const double *)(Linv + (size_t)(kb + 1) * NB * NB), x, y));
-    }
-    {
-        const int kb = (int)nblk - 1, k0 = kb * NB;
-        FMLB_TRY(launch_maybe_pdl(true, solve_first_backward_kernel, dim3(1), dim3(TPB), 0, st,
-                                  "solve_first_backward_kernel",
-                                  (const double *)(Linv + (size_t)kb * NB * NB),
-                                  (const double *)(y + k0), x + k0, n - k0));
-    }
-    for (int kb = (int)nblk - 1; kb >= 1; --kb) {
-        const int k0 = kb * NB, kn = std::min(NB, n - k0);
-        const int grid = 1 + ceil_div(k0 - NB, BWD_COLS);
-        FMLB_TRY(launch_maybe_pdl(true, backward_step_kernel, dim3(grid), dim3(TPB), 0, st,
-                                  "backward_step_kernel", L, lda, k0, kn,
-                                  (const double *)(Linv + (size_t)(kb - 1) * NB * NB), y, x));
-    }
-    return FMLB_OK;
+    unsigned *counters = reinterpret_cast<unsigned *>(y + n);
+    FMLB_TRY(cuda_status(cudaMemsetAsync(y, 0xff, (size_t)n * sizeof(double) + kSolveCounterBytes,
+                                         st), "fmlb_potrs_f64: fill"));
+    solve_forward_kernel<<<(unsigned)nblk, TPB, kSolveSmem, st>>>(L, lda, n, Linv, x, y, counters);
+    FMLB_TRY(launch_status("solve_forward_kernel"));
+    FMLB_TRY(cuda_status(cudaMemsetAsync(x, 0xff, (size_t)n * sizeof(double), st),
+                         "fmlb_potrs_f64: fill"));
+    solve_backward_kernel<<<(unsigned)nblk, TPB, kSolveSmem, st>>>(L, lda, n, Linv, y, x,
+                                                                  counters + 1);
+    return launch_status("solve_backward_kernel");
 }
 
 extern "C" int fmlb_syrk_lower_f64(double *C, long long ldc, int m, const double *P,

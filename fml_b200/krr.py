@@ -112,9 +112,8 @@ class KRRPipeline:
 
     def launches_per_run(self):
         """Kernel launches of one ``run`` (mirrors the loops in the C library)."""
-        nblk = -(-self.n_train // PANEL)
         potrf = potrf_launches(self.n_train, self.factor == "ozaki")
-        potrs = 2 * nblk
+        potrs = 2  # one launch per direction
         per_sigma = 1 + potrf + potrs
         per_sigma += 1  # the kept diagonal
         if self.refine > 0:  # per step 3 residual + 2 norm + potrs + update, final residual

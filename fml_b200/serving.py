@@ -365,7 +365,7 @@ class KRRServer:
                     g.capture_end()
                 g.replay()
             graphs.append(g)
-        self._count(1 + potrf_launches(n) + 2 * -(-n // 128))
+        self._count(1 + potrf_launches(n) + 2)
         return L, work, info, alpha
 
     def _build_version(self, m, charges, coords, offsets, y, stream, old=None, old_nmol=0,
