@@ -46,8 +46,9 @@ struct SetWs {
     signed char *cls;     // (nm, amax, amax) element class of each neighbour (fast path)
     signed char *acls;    // (nm, amax)       element class of each atom (fast path)
     float *selff;         // (nm, amax)       self terms (fast path)
-    float4 *spk;          // (nm, amax, amax) records of each molecule sorted by r (paired path)
-    int *smeta;           // (nm, amax, amax) atom | class << 16 | 1 << 24 of each sorted record
+    float4 *spk;          // (nm, slots) records of each molecule by r, 64 to a group (paired path)
+    unsigned short *smeta;  // (nm, slots)   atom | class << 8 | used << 15 of each
+    float2 *band;         // (nm, slots / 64) lowest and highest r of each group
     int *nrec;            // (nm)             records per molecule
 };
 
@@ -66,14 +67,24 @@ struct ClassInfo {
 
 __host__ __device__ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
+// The FP32 pair kernel takes BD_REC records of molecule I at a time: the slots of
+// nm molecules' records, each molecule's a multiple of that.
+constexpr int BD_REC = 64;
+__host__ __device__ inline int band_stride(int amax) {
+    return (amax * amax + BD_REC - 1) / BD_REC * BD_REC;
+}
+inline size_t band_slots(int nm, int amax) { return (size_t)nm * band_stride(amax); }
+
 size_t set_ws_bytes(int nm, int amax) {
     const size_t a2 = (size_t)nm * amax * amax, a1 = (size_t)nm * amax;
     return align256(a1 * sizeof(int)) + align256(a2 * sizeof(double)) +
            align256(a1 * sizeof(double)) + align256(a2 * sizeof(float4)) +
            align256(a2 * sizeof(float2)) + align256(a1 * sizeof(float)) + align256(a2) +
-           align256(a1) + align256(a1 * sizeof(float)) + align256(a2 * sizeof(float4)) +
-           align256(a2 * sizeof(int)) + align256((size_t)nm * sizeof(int)) +
-           align256(a1);
+           align256(a1) + align256(a1 * sizeof(float)) +
+           align256(band_slots(nm, amax) * sizeof(float4)) +
+           align256(band_slots(nm, amax) * sizeof(unsigned short)) +
+           align256(band_slots(nm, amax) / BD_REC * sizeof(float2)) +
+           align256((size_t)nm * sizeof(int)) + align256(a1);
 }
 
 SetWs carve(char *&p, int nm, int amax) {
@@ -88,8 +99,10 @@ SetWs carve(char *&p, int nm, int amax) {
     w.cls = reinterpret_cast<signed char *>(p); p += align256(a2);
     w.acls = reinterpret_cast<signed char *>(p); p += align256(a1);
     w.selff = reinterpret_cast<float *>(p); p += align256(a1 * sizeof(float));
-    w.spk = reinterpret_cast<float4 *>(p); p += align256(a2 * sizeof(float4));
-    w.smeta = reinterpret_cast<int *>(p); p += align256(a2 * sizeof(int));
+    const size_t slots = band_slots(nm, amax);
+    w.spk = reinterpret_cast<float4 *>(p); p += align256(slots * sizeof(float4));
+    w.smeta = reinterpret_cast<unsigned short *>(p); p += align256(slots * sizeof(unsigned short));
+    w.band = reinterpret_cast<float2 *>(p); p += align256(slots / BD_REC * sizeof(float2));
     w.nrec = reinterpret_cast<int *>(p); p += align256((size_t)nm * sizeof(int));
     w.asc = reinterpret_cast<signed char *>(p); p += align256(a1);
     return w;
@@ -447,32 +460,19 @@ constexpr int FC_PTS = FC_PC * FC_PC + 1;  // pair-table row stride (float2): co
 constexpr int FC_SS = FC_MAXA + 1;         // S row stride: lanes adding to different atoms i1
                                            // of one column j1 hit different banks
 
+// Scalar path (more classes): one molecule pair at a time.
 struct FastSmem {
     float4 recI[FC_MAXREC];      // molecule I, dense by atom, 32 records per pass
     int metaI[FC_MAXREC];        // atom | seg_start << 8 | cls << 16 | active << 24 | tail << 25
     float selfI[FC_MAXA];
     int aclsI[FC_MAXA];
-    union {
-        struct {
-            float4 rec[FC_MAXREC];       // molecule J, dense by atom
-            signed char cls[FC_MAXREC];  // element class of each record of J
-        } s;
-        struct {
-            float4 a[FC_MAXREC / 2];     // (r0, r1, xi0, xi1) per record pair
-            float4 b[FC_MAXREC / 2];     // (xc0, xc1, xs0, xs1)
-            int k[FC_MAXREC / 2];        // cls0 * FC_PC + cls1: column of the pair table
-        } p;
-    } J;
-    int offJ[FC_MAXA + 1];       // record offsets (scalar path) or pair offsets (paired path)
+    float4 recJ[FC_MAXREC];      // molecule J, dense by atom
+    signed char clsJ[FC_MAXREC];  // element class of each record of J
+    int offJ[FC_MAXA + 1];       // record offsets
     float selfJ[FC_MAXA];
     int aclsJ[FC_MAXA];
     float stoch[FC_MAXC * FC_SST];  // row stride 17: lanes of different classes hit distinct banks
-    float2 pt[FC_PC * FC_PTS];   // pt[c1][ca * FC_PC + cb] = (stoch(c1, ca), stoch(c1, cb))
-    union {
-        float f[FC_MAXA * FC_SS];      // scalar path: S(i1, j1), row stride FC_SS
-        long long q[FC_MAXA * FC_SS];  // paired path: S(i1, j1) in fixed point (2^-32 units)
-    } S;
-    float passLo[FC_MAXREC / 32], passHi[FC_MAXREC / 32];  // r band of each I pass (paired)
+    float S[FC_MAXA * FC_SS];       // S(i1, j1), row stride FC_SS
     float red[FC_WARPS][FC_MAXSIG];
     int npassI, nI, nJ;
 };
@@ -548,145 +548,13 @@ __device__ void fast_load_J(FastSmem &sm, const SetWs &w, int J, int amax, int n
         if (k < sm.offJ[a + 1] - sm.offJ[a]) {
             const int d = sm.offJ[a] + k;
             const size_t src = ((size_t)J * amax + a) * amax + k;
-            sm.J.s.rec[d] = w.pk[src];
-            sm.J.s.cls[d] = w.cls[src];
+            sm.recJ[d] = w.pk[src];
+            sm.clsJ[d] = w.cls[src];
         }
     }
     for (int a = threadIdx.x; a < nJ; a += blockDim.x) {
         sm.selfJ[a] = use_self ? w.selff[(size_t)J * amax + a] : 0.0f;
         sm.aclsJ[a] = w.acls[(size_t)J * amax + a];
-    }
-}
-
-// Molecule J in record pairs (paired path). Whole CTA; the caller synchronises
-// before the records are read.
-__device__ void fast_load_J_pairs(FastSmem &sm, const SetWs &w, int J, int amax, int nJ,
-                                  bool use_self) {
-    if (threadIdx.x < 32) {  // exclusive prefix of the padded pair counts (nJ <= 32)
-        const int a = threadIdx.x;
-        const int np = a < nJ ? (w.nnb[(size_t)J * amax + a] + 1) >> 1 : 0;
-        int incl = np;
-        for (int d = 1; d < 32; d <<= 1) {
-            const int o = __shfl_up_sync(0xffffffffu, incl, d);
-            if (a >= d) incl += o;
-        }
-        sm.offJ[a] = incl - np;
-        if (a == 31) {
-            sm.offJ[32] = incl;
-            sm.nJ = nJ;
-        }
-    }
-    __syncthreads();
-    const int hp = (amax + 1) >> 1;
-    for (int t = threadIdx.x; t < nJ * hp; t += blockDim.x) {
-        const int a = t / hp, q = t - a * hp;
-        const int beg = sm.offJ[a];
-        if (q < sm.offJ[a + 1] - beg) {
-            const size_t base = (size_t)J * amax + a;
-            const int cnt = w.nnb[base];
-            const size_t src = base * amax + 2 * q;
-            const float4 r0 = w.pk[src];
-            const int c0 = w.cls[src];
-            float4 r1 = make_float4(1.0e18f, 0.0f, 0.0f, 0.0f);
-            int c1 = 0;
-            if (2 * q + 1 < cnt) {
-                r1 = w.pk[src + 1];
-                c1 = w.cls[src + 1];
-            }
-            sm.J.p.a[beg + q] = make_float4(r0.x, r1.x, r0.y, r1.y);
-            sm.J.p.b[beg + q] = make_float4(r0.z, r1.z, r0.w, r1.w);
-            sm.J.p.k[beg + q] = c0 * FC_PC + c1;
-        }
-    }
-    for (int a = threadIdx.x; a < nJ; a += blockDim.x) {
-        sm.selfJ[a] = use_self ? w.selff[(size_t)J * amax + a] : 0.0f;
-        sm.aclsJ[a] = w.acls[(size_t)J * amax + a];
-    }
-}
-
-__device__ __forceinline__ float set_lt(float a, float b) {  // 1.0f if a < b, else 0.0f
-    float r;
-    asm("set.lt.f32.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
-
-// Paired work item over molecule I in radius bands: lane = one record of
-// pass p and one of pass p + 1 (records of I sorted by r, 32 per pass),
-// against the record pairs of atom j1 of J, two records per step with packed
-// FP32x2 arithmetic; each J record pair is loaded once for four
-// neighbour-pair evaluations. Every term is computed with the same operations
-// as in fast_item. Records of j1 outside the (8w)^2 window of every lane of
-// the two passes (j1's records are sorted by r) are skipped, and terms outside
-// a record's own window are masked: both are exactly zero. The lane's sums are
-// added to S(i1, j1) in 2^-32 fixed point, so the result does not depend on
-// the order of the additions.
-__device__ __forceinline__ void fast_item_band2(FastSmem &sm, int p, int j1, float maxg2s,
-                                                float wd) {
-    const int lane = threadIdx.x & 31;
-    const bool two = p + 1 < sm.npassI;
-    const float4 u0 = sm.recI[p * 32 + lane];
-    const int meta0 = sm.metaI[p * 32 + lane];
-    const float4 u1 = two ? sm.recI[(p + 1) * 32 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const int meta1 = two ? sm.metaI[(p + 1) * 32 + lane] : 0;
-    const float2 *ptrow0 = sm.pt + ((meta0 >> 16) & 0xff) * FC_PTS;
-    const float2 *ptrow1 = sm.pt + ((meta1 >> 16) & 0xff) * FC_PTS;
-    const float2 nux0 = make_float2(-u0.x, -u0.x), uy0 = make_float2(u0.y, u0.y),
-                 uz0 = make_float2(u0.z, u0.z), uw0 = make_float2(u0.w, u0.w);
-    const float2 nux1 = make_float2(-u1.x, -u1.x), uy1 = make_float2(u1.y, u1.y),
-                 uz1 = make_float2(u1.z, u1.z), uw1 = make_float2(u1.w, u1.w);
-    const int beg = sm.offJ[j1], end = sm.offJ[j1 + 1];
-    const float lo = sm.passLo[p] - wd, hi = sm.passHi[two ? p + 1 : p] + wd;
-    bool below = false, before = false;
-    if (beg + lane < end) {
-        const float4 A = sm.J.p.a[beg + lane];
-        below = !(A.y > lo);
-        before = A.x < hi;
-    }
-    const int mb = beg + __popc(__ballot_sync(0xffffffffu, below));
-    const int me = beg + __popc(__ballot_sync(0xffffffffu, before));
-    float2 acc0 = make_float2(0.0f, 0.0f), acc1 = make_float2(0.0f, 0.0f);
-#pragma unroll 2
-    for (int m = mb; m < me; ++m) {
-        const float4 A = sm.J.p.a[m];
-        const float4 B = sm.J.p.b[m];
-        const int k = sm.J.p.k[m];
-        const float2 st0 = ptrow0[k], st1 = ptrow1[k];
-        const float2 rj = make_float2(A.x, A.y), xj = make_float2(A.z, A.w);
-        const float2 cj = make_float2(B.x, B.y), sj = make_float2(B.z, B.w);
-        {
-            const float2 dr = __fadd2_rn(rj, nux0);
-            const float2 t = __fmul2_rn(dr, dr);
-            float e0, e1;
-            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(-t.x));
-            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(-t.y));
-            const float2 g = __ffma2_rn(sj, uw0, __ffma2_rn(cj, uz0, __fmul2_rn(xj, uy0)));
-            const float2 win = make_float2(set_lt(t.x, maxg2s), set_lt(t.y, maxg2s));
-            const float2 eg = __fmul2_rn(__fmul2_rn(make_float2(e0, e1), st0), win);
-            acc0 = __ffma2_rn(eg, g, acc0);
-        }
-        {
-            const float2 dr = __fadd2_rn(rj, nux1);
-            const float2 t = __fmul2_rn(dr, dr);
-            float e0, e1;
-            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(-t.x));
-            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(-t.y));
-            const float2 g = __ffma2_rn(sj, uw1, __ffma2_rn(cj, uz1, __fmul2_rn(xj, uy1)));
-            const float2 win = make_float2(set_lt(t.x, maxg2s), set_lt(t.y, maxg2s));
-            const float2 eg = __fmul2_rn(__fmul2_rn(make_float2(e0, e1), st1), win);
-            acc1 = __ffma2_rn(eg, g, acc1);
-        }
-    }
-    if ((meta0 >> 24) & 1) {
-        const long long f = __float2ll_rn((acc0.x + acc0.y) * 4294967296.0f);
-        if (f)
-            atomicAdd(reinterpret_cast<unsigned long long *>(&sm.S.q[(meta0 & 0xff) * FC_SS + j1]),
-                      (unsigned long long)f);
-    }
-    if ((meta1 >> 24) & 1) {
-        const long long f = __float2ll_rn((acc1.x + acc1.y) * 4294967296.0f);
-        if (f)
-            atomicAdd(reinterpret_cast<unsigned long long *>(&sm.S.q[(meta1 & 0xff) * FC_SS + j1]),
-                      (unsigned long long)f);
     }
 }
 
@@ -703,13 +571,13 @@ __device__ __forceinline__ void fast_item(FastSmem &sm, int p, int j1, float max
     float acc = 0.0f;
 #pragma unroll 4
     for (int m2 = beg; m2 < end; ++m2) {
-        const float4 q = sm.J.s.rec[m2];
+        const float4 q = sm.recJ[m2];
         const float dr = q.x - u.x;
         const float t = dr * dr;
         float e;
         asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-t));
         const float g = fmaf(u.w, q.w, fmaf(u.z, q.z, u.y * q.y));
-        const float eg = e * strow[sm.J.s.cls[m2]];
+        const float eg = e * strow[sm.clsJ[m2]];
         if (t < maxg2s) acc = fmaf(eg, g, acc);
     }
     const int seg = (meta >> 8) & 0xff;
@@ -719,79 +587,22 @@ __device__ __forceinline__ void fast_item(FastSmem &sm, int p, int j1, float max
         const float o = __shfl_up_sync(0xffffffffu, v, d);
         if (lane - d >= seg) v += o;
     }
-    if ((meta >> 25) & 1) atomicAdd(&sm.S.f[(meta & 0xff) * FC_SS + j1], v);
+    if ((meta >> 25) & 1) atomicAdd(&sm.S[(meta & 0xff) * FC_SS + j1], v);
 }
 
 // All work items of one molecule pair, S cleared first. Whole CTA.
-__device__ __forceinline__ void fast_pair_sums(FastSmem &sm, int nJ, float maxg2s, bool paired) {
-    if (paired) {
-        for (int t = threadIdx.x; t < FC_MAXA * FC_SS; t += blockDim.x) sm.S.q[t] = 0;
-    } else {
-        for (int t = threadIdx.x; t < FC_MAXA * FC_SS; t += blockDim.x) sm.S.f[t] = 0.0f;
-    }
+__device__ __forceinline__ void fast_pair_sums(FastSmem &sm, int nJ, float maxg2s) {
+    for (int t = threadIdx.x; t < FC_MAXA * FC_SS; t += blockDim.x) sm.S[t] = 0.0f;
     __syncthreads();
     const int warp = threadIdx.x >> 5;
     const int items = sm.npassI * nJ;
-    if (paired) {
-        // skip margin slightly wider than the window: only records whose every
-        // term is masked are skipped
-        const float wd = sqrtf(maxg2s) * 1.0001f;
-        const int items2 = ((sm.npassI + 1) >> 1) * nJ;
-        for (int it = warp; it < items2; it += FC_WARPS)
-            fast_item_band2(sm, 2 * (it / nJ), it % nJ, maxg2s, wd);
-    } else {
-        for (int it = warp; it < items; it += FC_WARPS) fast_item(sm, it / nJ, it % nJ, maxg2s);
-    }
+    for (int it = warp; it < items; it += FC_WARPS) fast_item(sm, it / nJ, it % nJ, maxg2s);
     __syncthreads();
 }
 
-__device__ __forceinline__ float s_value(const FastSmem &sm, int idx, bool paired) {
-    return paired ? (float)((double)sm.S.q[idx] * 2.3283064365386963e-10) : sm.S.f[idx];
-}
-
-// Molecule I for the paired path: its records sorted by r (prepared once per
-// set by arad_sort_records_kernel), 32 per pass, with the r band of each
-// pass. Whole CTA; the caller synchronises before the records are read.
-__device__ void fast_load_I_band(FastSmem &sm, const SetWs &w, int I, int amax, int nI,
-                                 bool use_self) {
-    const int nrec = w.nrec[I];
-    const int npass = (nrec + 31) / 32;
-    const size_t base = (size_t)I * amax * amax;
-    for (int slot = threadIdx.x; slot < npass * 32; slot += blockDim.x) {
-        if (slot < nrec) {
-            sm.recI[slot] = w.spk[base + slot];
-            sm.metaI[slot] = w.smeta[base + slot];
-        } else {
-            sm.recI[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
-            sm.metaI[slot] = 0;  // inactive
-        }
-    }
-    for (int p = threadIdx.x; p < npass; p += blockDim.x) {
-        sm.passLo[p] = w.spk[base + 32 * p].x;
-        sm.passHi[p] = w.spk[base + min(32 * p + 31, nrec - 1)].x;
-    }
-    for (int a = threadIdx.x; a < nI; a += blockDim.x) {
-        sm.selfI[a] = use_self ? w.selff[(size_t)I * amax + a] : 0.0f;
-        sm.aclsI[a] = w.acls[(size_t)I * amax + a];
-    }
-    if (threadIdx.x == 0) {
-        sm.npassI = npass;
-        sm.nI = nI;
-    }
-}
-
-// Class tables of the CTA: the stoichiometric table (row stride FC_SST) and,
-// for the paired path, the pair table.
-__device__ __forceinline__ void fast_load_tables(FastSmem &sm, const ClassInfo *ci, bool paired) {
+__device__ __forceinline__ void load_stoch(float *stoch, const ClassInfo *ci) {
     for (int t = threadIdx.x; t < FC_MAXC * FC_MAXC; t += blockDim.x)
-        sm.stoch[(t / FC_MAXC) * FC_SST + t % FC_MAXC] = ci->stoch[t];
-    if (paired)
-        for (int t = threadIdx.x; t < FC_PC * FC_PC * FC_PC; t += blockDim.x) {
-            const int c1 = t / (FC_PC * FC_PC), k = t % (FC_PC * FC_PC);
-            const int ca = k / FC_PC, cb = k % FC_PC;
-            sm.pt[c1 * FC_PTS + k] =
-                make_float2(ci->stoch[c1 * FC_MAXC + ca], ci->stoch[c1 * FC_MAXC + cb]);
-        }
+        stoch[(t / FC_MAXC) * FC_SST + t % FC_MAXC] = ci->stoch[t];
 }
 
 __device__ __forceinline__ void pair_block(long long t, int symmetric, int nbj, int &bi, int &bj) {
@@ -860,58 +671,446 @@ arad_sort_records_kernel(SetWs w, const int *__restrict__ N, int nm, int amax,
             }
             __syncthreads();
         }
-    const size_t base = (size_t)I * amax * amax;
+    // Inside a group of 64 two records of one atom go to one lane, as far as they
+    // come in twos: the lane then adds to S once instead of twice. Twos take the
+    // lanes in the order in which they are completed, then the atoms' odd records
+    // in the order of the atoms; slots past them stay unused.
+    const size_t base = (size_t)I * band_stride(amax);
+    const int slots = (nrec + BD_REC - 1) / BD_REC * BD_REC;
+    for (int t = threadIdx.x; t < slots; t += blockDim.x) {
+        w.spk[base + t] = make_float4(0.f, 0.f, 0.f, 0.f);
+        w.smeta[base + t] = 0;
+    }
+    __syncthreads();
     for (int t = threadIdx.x; t < nrec; t += blockDim.x) {
-        const int idx = (int)(key[t] & 0xffffffffu), a = idx / FC_MAXA, k = idx % FC_MAXA;
+        const int beg = t / BD_REC * BD_REC, end = min(beg + BD_REC, nrec);
+        const auto atom = [&](int q) { return (int)(key[q] & 0xffffffffu) / FC_MAXA; };
+        const int a = atom(t), k = (int)(key[t] & 0xffffffffu) % FC_MAXA;
+        int rank = 0, same = 0;  // among the group's records of this atom
+        for (int q = beg; q < end; ++q) {
+            rank += q < t && atom(q) == a;
+            same += atom(q) == a;
+        }
+        const bool one = (same & 1) && rank == same - 1;
+        int done = t;  // where t's two is completed
+        if (one)
+            done = end;
+        else if (!(rank & 1))
+            while (atom(++done) != a) {}
+        int twos = 0;  // completed before that
+        unsigned odd = 0;
+        for (int q = beg; q < end; ++q) {
+            const unsigned bit = 1u << atom(q);
+            twos += q < done && (odd & bit);
+            odd ^= bit;
+        }
+        const int ones = __popc(odd & ((1u << a) - 1));
+        const int slot = one ? twos + (ones >> 1) + 32 * (ones & 1) : twos + 32 * (rank & 1);
         const size_t src = ((size_t)I * amax + a) * amax + k;
-        w.spk[base + t] = w.pk[src];
-        w.smeta[base + t] = a | ((int)w.cls[src] << 16) | (1 << 24);
+        const float4 rec = w.pk[src];
+        w.spk[base + beg + slot] = rec;
+        w.smeta[base + beg + slot] = (unsigned short)(a | ((int)w.cls[src] << 8) | (1 << 15));
+        float2 *band = w.band + base / BD_REC + t / BD_REC;
+        if (t == beg) band->x = rec.x;
+        if (t == end - 1) band->y = rec.x;
     }
     if (threadIdx.x == 0) w.nrec[I] = nrec;
 }
 
-// Self terms S(a, a) through the same passes, scan and partial sums as the
-// pair kernel, so that l2 = s + s - 2 S cancels exactly for an atom with itself.
-__global__ void __launch_bounds__(FC_WARPS * 32)
+// ---- the paired path's pair sums ---------------------------------------------
+// A CTA takes tiles of FC_BM molecules I and J, as many J at a time as its shared
+// memory holds beside the records of one I:
+//   1. for each group of 64 records of I and each atom j1 the range of j1's
+//      record pairs inside the group's band widened by the (8 w)^2 window;
+//   2. a warp keeps a group's records in registers, two to a lane, and walks the
+//      atoms j1: each record pair of j1 is loaded once for four evaluations.
+//      Terms outside a record's own window are masked, so that what is skipped
+//      and what is masked are both exactly zero;
+//   3. a lane's sums are added to S(i1, j1) in 2^-32 fixed point: the result does
+//      not depend on the order of the additions. 64 bits as two 32-bit words
+//      with a carry: the 64-bit shared-memory atomic is a compare-and-swap loop;
+//   4. the kernel exponentials of every l2 and sigma, in an order that depends on
+//      the two molecules' atoms alone.
+// Bound by the instructions issued: 38 for a step of 2 (128 evaluations, of which 14
+// packed FP32 and 4 exponentials, 8 cycles of their units each), about 45 to add a
+// lane's sums, 5000 per molecule pair outside of the steps. 500 x 3001 molecules of
+// at most 23 atoms, 5 sigmas: 30.3 ms; 39.7 with one J at a time, the ranges found
+// by every warp for itself and the compare-and-swap loop, which took half of the
+// shared memory's cycles.
+constexpr int BD_JA = 96;     // atoms J at a time
+struct BandSmem {
+    float2 pt[FC_PC * FC_PTS];      // pt[c1][ca * FC_PC + cb] = (stoch(c1, ca), stoch(c1, cb))
+    float stoch[FC_MAXC * FC_SST];  // row stride 17: lanes of different classes hit distinct banks
+    float sc[FC_MAXSIG];            // log2 e / sigma^2, negative
+    float selfI[FC_MAXA];
+    float selfJ[BD_JA];
+    float red[FC_BM][FC_WARPS][FC_MAXSIG];
+    int aclsI[FC_MAXA];
+    int nI[FC_BM], recI[FC_BM];     // molecules I of the tile: atoms, records
+    int nJ[FC_BM], pairsJ[FC_BM];   // molecules J of the tile: atoms, record pairs
+    short offJ[BD_JA + 1];          // first record pair of each atom J
+    short atomJ[FC_BM + 1];         // first atom of each molecule J at a time
+    unsigned char aclsJ[BD_JA];
+};
+// four CTAs per SM, with 1 KB for the system and the scalar path's offsets each
+constexpr size_t kBandSmem = 56 * 1024 - 256;
+constexpr size_t kBandArena = kBandSmem - (sizeof(BandSmem) + 15) / 16 * 16;
+
+struct BandArena {
+    float4 *rec;            // molecule I, groups of 64
+    float4 *pair;           // molecules J: (r0, r1, xi0, xi1), (xc0, xc1, xs0, xs1) by turns
+    unsigned *lo, *hi;      // S(i1, j1) in fixed point at j1 * ld + i1
+    unsigned short *meta;   // as SetWs::smeta
+    short2 *win;            // first and past-the-last record pair by group and atom j1
+    unsigned char *pk;      // cls0 * FC_PC + cls1: column of the pair table
+    int ld;                 // odd: lanes adding to different atoms i1 hit different banks
+};
+__host__ __device__ constexpr size_t band_bytes(int recs, int pairs, int atoms, int ld) {
+    return (size_t)recs * 18 + (size_t)pairs * 33 + (size_t)atoms * ld * 8 +
+           (size_t)atoms * (recs / BD_REC) * 4;
+}
+static_assert(band_bytes(FC_MAXREC, FC_MAXREC / 2, FC_MAXA, FC_MAXA + 1) <= kBandArena &&
+              FC_MAXA <= BD_JA && FC_MAXREC / 2 < 32768 && FC_WARPS == FC_BM,
+              "one pair of the largest molecules fits");
+constexpr size_t kFastSmem =
+    sizeof(FastSmem) > kBandSmem ? sizeof(FastSmem) : kBandSmem;  // whichever path the classes decide
+
+__device__ __forceinline__ BandArena band_carve(unsigned char *p, int recs, int pairs, int atoms,
+                                                int ld) {
+    BandArena A;
+    A.rec = reinterpret_cast<float4 *>(p);
+    A.pair = A.rec + recs;
+    A.lo = reinterpret_cast<unsigned *>(A.pair + 2 * pairs);
+    A.hi = A.lo + atoms * ld;
+    A.win = reinterpret_cast<short2 *>(A.hi + atoms * ld);
+    A.meta = reinterpret_cast<unsigned short *>(A.win + atoms * (recs / BD_REC));
+    A.pk = reinterpret_cast<unsigned char *>(A.meta + recs);
+    A.ld = ld;
+    return A;
+}
+
+__device__ __forceinline__ void band_load_tables(BandSmem &sm, const ClassInfo *ci) {
+    load_stoch(sm.stoch, ci);
+    for (int t = threadIdx.x; t < FC_PC * FC_PC * FC_PC; t += blockDim.x) {
+        const int c1 = t / (FC_PC * FC_PC), k = t % (FC_PC * FC_PC);
+        const int ca = k / FC_PC, cb = k % FC_PC;
+        sm.pt[c1 * FC_PTS + k] =
+            make_float2(ci->stoch[c1 * FC_MAXC + ca], ci->stoch[c1 * FC_MAXC + cb]);
+    }
+}
+
+// Sizes of the tile's molecules: warp q takes the q-th of each side.
+__device__ __forceinline__ void band_sizes(BandSmem &sm, const SetWs &w1, const int *N1, int I0,
+                                           int nm1, const SetWs &w2, const int *N2, int J0,
+                                           int nm2, int amax) {
+    const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int I = I0 + q, J = J0 + q;
+    const int nJ = J < nm2 ? min(max(N2[J], 0), amax) : 0;
+    int pairs = lane < nJ ? (w2.nnb[(size_t)J * amax + lane] + 1) >> 1 : 0;
+    for (int o = 16; o; o >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
+    if (lane == 0) {
+        sm.nI[q] = I < nm1 ? min(max(N1[I], 0), amax) : 0;
+        sm.recI[q] = I < nm1 ? w1.nrec[I] : 0;
+        sm.nJ[q] = nJ;
+        sm.pairsJ[q] = pairs;
+    }
+}
+
+// Molecules J .. J + count - 1 (the tile's from j0 on) in record pairs. Whole CTA,
+// with a barrier inside; the caller synchronises before the records are read.
+__device__ __forceinline__ void band_load_J(BandSmem &sm, const BandArena &A, const SetWs &w, int J,
+                                            int j0, int count, int amax, bool use_self) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp < count) {  // offsets: warp q takes the q-th molecule
+        int atoms = 0, beg = 0;
+        for (int q = 0; q < warp; ++q) {
+            atoms += sm.nJ[j0 + q];
+            beg += sm.pairsJ[j0 + q];
+        }
+        const int n = sm.nJ[j0 + warp];
+        const size_t a = (size_t)(J + warp) * amax + lane;
+        const int np = lane < n ? (w.nnb[a] + 1) >> 1 : 0;
+        int incl = np;
+        for (int d = 1; d < 32; d <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += o;
+        }
+        if (lane < n) {
+            sm.offJ[atoms + lane] = (short)(beg + incl - np);
+            sm.selfJ[atoms + lane] = use_self ? w.selff[a] : 0.0f;
+            sm.aclsJ[atoms + lane] = (unsigned char)w.acls[a];
+        }
+        if (lane == 31) {
+            sm.atomJ[warp] = (short)atoms;
+            if (warp == count - 1) {
+                sm.atomJ[count] = (short)(atoms + n);
+                sm.offJ[atoms + n] = (short)(beg + incl);
+            }
+        }
+    }
+    __syncthreads();
+    // 16 threads per atom, a record pair each
+    const int q = threadIdx.x & 15;
+    int m = 0;
+    for (int j = threadIdx.x >> 4; j < sm.atomJ[count]; j += FC_WARPS * 2) {
+        while (j >= sm.atomJ[m + 1]) ++m;
+        const int beg = sm.offJ[j];
+        if (q >= sm.offJ[j + 1] - beg) continue;
+        const size_t base = (size_t)(J + m) * amax + j - sm.atomJ[m], src = base * amax + 2 * q;
+        const float4 r0 = w.pk[src];
+        const int c0 = w.cls[src];
+        float4 r1 = make_float4(1.0e18f, 0.0f, 0.0f, 0.0f);
+        int c1 = 0;
+        if (2 * q + 1 < w.nnb[base]) {
+            r1 = w.pk[src + 1];
+            c1 = w.cls[src + 1];
+        }
+        A.pair[2 * (beg + q)] = make_float4(r0.x, r1.x, r0.y, r1.y);
+        A.pair[2 * (beg + q) + 1] = make_float4(r0.z, r1.z, r0.w, r1.w);
+        A.pk[beg + q] = (unsigned char)(c0 * FC_PC + c1);
+    }
+}
+
+// Molecule I of the tile (the i-th), S cleared, and the ranges of step 1 of its groups with the
+// atoms J (loaded before). Whole CTA; the caller synchronises before use.
+__device__ __forceinline__ void band_load_I(BandSmem &sm, const BandArena &A, const SetWs &w, int I,
+                                            int i, int count, int amax, float wd, bool use_self) {
+    const int nat = sm.atomJ[count], groups = (sm.recI[i] + BD_REC - 1) / BD_REC;
+    const size_t base = (size_t)I * band_stride(amax);
+    for (int t = threadIdx.x; t < groups * BD_REC; t += blockDim.x) {
+        A.rec[t] = w.spk[base + t];
+        A.meta[t] = w.smeta[base + t];
+    }
+    for (int t = threadIdx.x; t < nat * A.ld; t += blockDim.x) A.lo[t] = A.hi[t] = 0;
+    for (int a = threadIdx.x; a < sm.nI[i]; a += blockDim.x) {
+        sm.selfI[a] = use_self ? w.selff[(size_t)I * amax + a] : 0.0f;
+        sm.aclsI[a] = w.acls[(size_t)I * amax + a];
+    }
+    for (int t = threadIdx.x; t < nat * groups; t += blockDim.x) {
+        const int g = t / nat, j = t - g * nat;
+        const float2 band = w.band[base / BD_REC + g];
+        const float lo = band.x - wd, hi = band.y + wd;
+        int below = sm.offJ[j], before = below;
+        for (int q = below, end = sm.offJ[j + 1]; q < end; ++q) {
+            const float2 r = *reinterpret_cast<const float2 *>(A.pair + 2 * q);
+            below += !(r.y > lo);
+            before += r.x < hi;
+        }
+        A.win[t] = make_short2((short)below, (short)before);
+    }
+}
+
+// One record u (its r negated, as pairs of equals) against a record pair.
+struct BandRec {
+    float2 nx, y, z, w;
+    __device__ explicit BandRec(const float4 &u)
+        : nx(make_float2(-u.x, -u.x)), y(make_float2(u.y, u.y)), z(make_float2(u.z, u.z)),
+          w(make_float2(u.w, u.w)) {}
+};
+__device__ __forceinline__ float2 band_terms(const BandRec &u, const float4 &a, const float4 &b,
+                                             float2 st, float maxg2s, float2 acc) {
+    const float2 dr = __fadd2_rn(make_float2(a.x, a.y), u.nx);
+    const float2 t = __fmul2_rn(dr, dr);
+    float e0, e1;  // outside the window exactly zero
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(t.x < maxg2s ? -t.x : -1.0e30f));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(t.y < maxg2s ? -t.y : -1.0e30f));
+    const float2 g = __ffma2_rn(make_float2(b.z, b.w), u.w,
+                                __ffma2_rn(make_float2(b.x, b.y), u.z,
+                                           __fmul2_rn(make_float2(a.z, a.w), u.y)));
+    return __ffma2_rn(__fmul2_rn(make_float2(e0, e1), st), g, acc);
+}
+
+__device__ __forceinline__ void band_add(unsigned *lo, int hi, long long f) {
+    const unsigned l = (unsigned)f;
+    unsigned h = (unsigned)((unsigned long long)f >> 32);
+    h += atomicAdd(lo, l) > ~l;  // the carry
+    if (h) atomicAdd(lo + hi, h);
+}
+
+// Steps 2 and 3 for the atoms J from jfirst on. Whole CTA.
+__device__ __forceinline__ void band_sums(const BandSmem &sm, const BandArena &A, int i, int jfirst,
+                                          int nat, float maxg2s) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int groups = (sm.recI[i] + BD_REC - 1) / BD_REC, hi = (int)(A.hi - A.lo);
+    for (int g = 0; g < groups; ++g) {
+        const BandRec u0(A.rec[g * BD_REC + lane]), u1(A.rec[g * BD_REC + 32 + lane]);
+        const int meta0 = A.meta[g * BD_REC + lane], meta1 = A.meta[g * BD_REC + 32 + lane];
+        const float2 *pt0 = sm.pt + ((meta0 >> 8) & 0x7f) * FC_PTS;
+        const float2 *pt1 = sm.pt + ((meta1 >> 8) & 0x7f) * FC_PTS;
+        unsigned *s0 = A.lo + (meta0 & 0xff), *s1 = A.lo + (meta1 & 0xff);
+        const bool both = ((meta0 ^ meta1) & 0x80ff) == 0;  // two records of one atom
+        // the atoms that are left over after the eights go to other warps in each group
+        for (int j = jfirst + ((warp + 3 * g) & (FC_WARPS - 1)); j < nat; j += FC_WARPS) {
+            const short2 win = A.win[g * nat + j];
+            float2 acc0 = make_float2(0.0f, 0.0f), acc1 = make_float2(0.0f, 0.0f);
+#pragma unroll 2
+            for (int m = win.x; m < win.y; ++m) {
+                const float4 a = A.pair[2 * m], b = A.pair[2 * m + 1];
+                const int k = A.pk[m];
+                acc0 = band_terms(u0, a, b, pt0[k], maxg2s, acc0);
+                acc1 = band_terms(u1, a, b, pt1[k], maxg2s, acc1);
+            }
+            // unused slots: records of zeros, whose sums are zero
+            long long f0 = __float2ll_rn((acc0.x + acc0.y) * 4294967296.0f);
+            const long long f1 = __float2ll_rn((acc1.x + acc1.y) * 4294967296.0f);
+            if (both) f0 += f1;
+            if (f0) band_add(s0 + j * A.ld, hi, f0);
+            if (!both && f1) band_add(s1 + j * A.ld, hi, f1);
+        }
+    }
+}
+
+__device__ __forceinline__ float band_value(const BandArena &A, int idx) {
+    const long long q = (long long)((unsigned long long)A.hi[idx] << 32 | A.lo[idx]);
+    return (float)((double)q * 2.3283064365386963e-10);
+}
+
+// The paired path of a tile: molecules I0 .. and J0 .. (FC_BM of each).
+__device__ __forceinline__ void band_tile(unsigned char *smem, const SetWs &w1, const int *N1,
+                                          int nm1, const SetWs &w2, const int *N2, int nm2, int I0,
+                                          int J0, int amax, float maxg2s, float eps,
+                                          const ClassInfo *ci, const SigmaTable &sig, int nsig,
+                                          int symmetric, double *K) {
+    BandSmem &sm = *reinterpret_cast<BandSmem *>(smem);
+    unsigned char *arena = smem + (sizeof(BandSmem) + 15) / 16 * 16;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float wd = sqrtf(maxg2s) * 1.0001f;  // a little wider than the window
+    band_load_tables(sm, ci);
+#pragma unroll
+    for (int s = 0; s < FC_MAXSIG; ++s)
+        if (threadIdx.x == s && s < nsig)
+            sm.sc[s] = (float)(sig.inv_sigma2[s] * 1.4426950408889634);
+    band_sizes(sm, w1, N1, I0, nm1, w2, N2, J0, nm2, amax);
+    __syncthreads();
+    const int ni = min(FC_BM, nm1 - I0), nj = min(FC_BM, nm2 - J0);
+    int recs = 0, ld = 1;
+    for (int i = 0; i < ni; ++i) {
+        recs = max(recs, (sm.recI[i] + BD_REC - 1) / BD_REC * BD_REC);
+        ld = max(ld, sm.nI[i] | 1);
+    }
+    for (int j0 = 0, count; j0 < nj; j0 += count) {
+        int atoms = sm.nJ[j0], pairs = sm.pairsJ[j0];
+        for (count = 1; j0 + count < nj; ++count) {
+            const int a = atoms + sm.nJ[j0 + count], p = pairs + sm.pairsJ[j0 + count];
+            if (a > BD_JA || band_bytes(recs, p, a, ld) > kBandArena) break;
+            atoms = a;
+            pairs = p;
+        }
+        const BandArena A = band_carve(arena, recs, pairs, atoms, ld);
+        __syncthreads();  // the molecules J before are done with
+        band_load_J(sm, A, w2, J0 + j0, j0, count, amax, true);
+        __syncthreads();
+        for (int i = 0; i < ni; ++i) {
+            const int I = I0 + i, nI = sm.nI[i];
+            const int first = symmetric ? max(0, I - J0 - j0) : 0;  // J >= I
+            if (first >= count) continue;
+            band_load_I(sm, A, w1, I, i, count, amax, wd, true);
+            __syncthreads();
+            band_sums(sm, A, i, sm.atomJ[first], atoms, maxg2s);
+            __syncthreads();
+            for (int m = first; m < count; ++m) {
+                // elements 32 part .. of every 256; which warp takes them does not matter
+                const int part = (warp + 3 * m) & (FC_WARPS - 1);
+                const int j1 = sm.atomJ[m], nJ = sm.atomJ[m + 1] - j1, n = nI * nJ;
+                float kacc[FC_MAXSIG];
+#pragma unroll
+                for (int s = 0; s < FC_MAXSIG; ++s) kacc[s] = 0.0f;
+                const float inv = 1.0f / (float)nJ;
+                for (int t = part * 32 + lane; t < n; t += FC_WARPS * 32) {
+                    const int a = (int)(((float)t + 0.5f) * inv), j = j1 + t - a * nJ;
+                    const float stz = sm.stoch[sm.aclsI[a] * FC_SST + sm.aclsJ[j]];
+                    float l2 = sm.selfI[a] + sm.selfJ[j] -
+                               2.0f * band_value(A, j * A.ld + a) * stz;
+                    if (fabsf(l2) < eps) l2 = 0.0f;  // farad_kernels.f90:594
+#pragma unroll
+                    for (int s = 0; s < FC_MAXSIG; ++s) {
+                        if (s < nsig) {
+                            float e;
+                            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(l2 * sm.sc[s]));
+                            kacc[s] += e;
+                        }
+                    }
+                }
+#pragma unroll
+                for (int s = 0; s < FC_MAXSIG; ++s) {
+                    if (s < nsig) {
+                        float v = kacc[s];
+                        if (part * 32 < n)
+                            for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                        if (lane == 0) sm.red[m][part][s] = v;
+                    }
+                }
+            }
+            __syncthreads();
+            for (int t = threadIdx.x; t < (count - first) * nsig; t += blockDim.x) {
+                const int m = first + t / nsig, s = t % nsig, J = J0 + j0 + m;
+                double v = 0.0;
+                for (int q = 0; q < FC_WARPS; ++q) v += (double)sm.red[m][q][s];
+                K[((size_t)s * nm1 + I) * nm2 + J] = v;
+                if (symmetric) K[((size_t)s * nm1 + J) * nm2 + I] = v;
+            }
+        }
+    }
+}
+
+// Self terms S(a, a) through the pair kernel's passes and sums, so that
+// l2 = s + s - 2 S cancels exactly for an atom with itself.
+__global__ void __launch_bounds__(FC_WARPS * 32, 4)
 arad_fast_self_kernel(SetWs w, const int *__restrict__ N, int nm, int amax, AradParams P,
                       const ClassInfo *ci) {
     extern __shared__ __align__(16) unsigned char fc_smem_raw[];
-    FastSmem &sm = *reinterpret_cast<FastSmem *>(fc_smem_raw);
     if (ci->flag) return;
     const int I = blockIdx.x;
     if (I >= nm) return;
-    const bool paired = ci->ncls <= FC_PC;
-    fast_load_tables(sm, ci, paired);
-    const int nI = min(max(N[I], 0), amax);
-    if (paired) {
-        fast_load_I_band(sm, w, I, amax, nI, false);
-        fast_load_J_pairs(sm, w, I, amax, nI, false);
-    } else {
-        fast_load_I(sm, w, I, amax, nI, false);
-        fast_load_J(sm, w, I, amax, nI, false);
-    }
-    __syncthreads();
     const float maxg2s = (float)(P.maxg2 * fp32_scale(P) * fp32_scale(P));
-    fast_pair_sums(sm, nI, maxg2s, paired);
+    if (ci->ncls <= FC_PC) {
+        BandSmem &sm = *reinterpret_cast<BandSmem *>(fc_smem_raw);
+        band_load_tables(sm, ci);
+        band_sizes(sm, w, N, I, I + 1, w, N, I, I + 1, amax);
+        __syncthreads();
+        const int n = sm.nI[0], recs = (sm.recI[0] + BD_REC - 1) / BD_REC * BD_REC;
+        const BandArena A = band_carve(fc_smem_raw + (sizeof(BandSmem) + 15) / 16 * 16, recs,
+                                       sm.pairsJ[0], n, n | 1);
+        band_load_J(sm, A, w, I, 0, 1, amax, false);
+        __syncthreads();
+        band_load_I(sm, A, w, I, 0, 1, amax, sqrtf(maxg2s) * 1.0001f, false);
+        __syncthreads();
+        band_sums(sm, A, 0, 0, n, maxg2s);
+        __syncthreads();
+        for (int a = threadIdx.x; a < n; a += blockDim.x)
+            w.selff[(size_t)I * amax + a] = band_value(A, a * A.ld + a);
+        return;
+    }
+    FastSmem &sm = *reinterpret_cast<FastSmem *>(fc_smem_raw);
+    load_stoch(sm.stoch, ci);
+    const int nI = min(max(N[I], 0), amax);
+    fast_load_I(sm, w, I, amax, nI, false);
+    fast_load_J(sm, w, I, amax, nI, false);
+    __syncthreads();
+    fast_pair_sums(sm, nI, maxg2s);
     for (int a = threadIdx.x; a < nI; a += blockDim.x)
-        w.selff[(size_t)I * amax + a] = s_value(sm, a * FC_SS + a, paired);
+        w.selff[(size_t)I * amax + a] = sm.S[a * FC_SS + a];
 }
 
-__global__ void __launch_bounds__(FC_WARPS * 32)
+__global__ void __launch_bounds__(FC_WARPS * 32, 4)
 arad_fast_pair_kernel(SetWs w1, const int *__restrict__ N1, int nm1, SetWs w2,
                       const int *__restrict__ N2, int nm2, int amax, AradParams P,
                       const ClassInfo *ci, SigmaTable sig, int nsig, int symmetric,
                       double *__restrict__ K) {
     extern __shared__ __align__(16) unsigned char fc_smem_raw[];
-    FastSmem &sm = *reinterpret_cast<FastSmem *>(fc_smem_raw);
     if (ci->flag) return;
     const int nbj = (nm2 + FC_BM - 1) / FC_BM;
     int bi, bj;
     pair_block(blockIdx.x, symmetric, nbj, bi, bj);
-    const bool paired = ci->ncls <= FC_PC;
-    fast_load_tables(sm, ci, paired);
     const float maxg2s = (float)(P.maxg2 * fp32_scale(P) * fp32_scale(P));
     const float eps = 5.0e-12f;
+    if (ci->ncls <= FC_PC) {
+        band_tile(fc_smem_raw, w1, N1, nm1, w2, N2, nm2, bi * FC_BM, bj * FC_BM, amax, maxg2s, eps,
+                  ci, sig, nsig, symmetric, K);
+        return;
+    }
+    FastSmem &sm = *reinterpret_cast<FastSmem *>(fc_smem_raw);
+    load_stoch(sm.stoch, ci);
     float sc[FC_MAXSIG];
 #pragma unroll
     for (int s = 0; s < FC_MAXSIG; ++s)
@@ -922,22 +1121,16 @@ arad_fast_pair_kernel(SetWs w1, const int *__restrict__ N1, int nm1, SetWs w2,
         if (I >= nm1) break;
         __syncthreads();
         const int nI = min(max(N1[I], 0), amax);
-        if (paired)
-            fast_load_I_band(sm, w1, I, amax, nI, true);
-        else
-            fast_load_I(sm, w1, I, amax, nI, true);
+        fast_load_I(sm, w1, I, amax, nI, true);
         for (int jl = 0; jl < FC_BM; ++jl) {
             const int J = bj * FC_BM + jl;
             if (J >= nm2) break;
             if (symmetric && J < I) continue;
             __syncthreads();
             const int nJ = min(max(N2[J], 0), amax);
-            if (paired)
-                fast_load_J_pairs(sm, w2, J, amax, nJ, true);
-            else
-                fast_load_J(sm, w2, J, amax, nJ, true);
+            fast_load_J(sm, w2, J, amax, nJ, true);
             __syncthreads();
-            fast_pair_sums(sm, nJ, maxg2s, paired);
+            fast_pair_sums(sm, nJ, maxg2s);
             // phase 2: l2 and the kernel exponentials of every atom pair
             float kacc[FC_MAXSIG];
 #pragma unroll
@@ -946,7 +1139,7 @@ arad_fast_pair_kernel(SetWs w1, const int *__restrict__ N1, int nm1, SetWs w2,
                 const int a = t / nJ, j1 = t - a * nJ;
                 const float stz = sm.stoch[sm.aclsI[a] * FC_SST + sm.aclsJ[j1]];
                 float l2 = sm.selfI[a] + sm.selfJ[j1] -
-                           2.0f * s_value(sm, a * FC_SS + j1, paired) * stz;
+                           2.0f * sm.S[a * FC_SS + j1] * stz;
                 if (fabsf(l2) < eps) l2 = 0.0f;  // farad_kernels.f90:594
 #pragma unroll
                 for (int s = 0; s < FC_MAXSIG; ++s) {
@@ -1392,11 +1585,11 @@ int fast_smem_attrs() {
     if (attr_dev == dev) return FMLB_OK;
     FMLB_TRY(cuda_status(cudaFuncSetAttribute(arad_fast_self_kernel,
                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)sizeof(FastSmem)),
+                                              (int)kFastSmem),
                          "fmlb_arad_kernels: self kernel smem attribute"));
     FMLB_TRY(cuda_status(cudaFuncSetAttribute(arad_fast_pair_kernel,
                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)sizeof(FastSmem)),
+                                              (int)kFastSmem),
                          "fmlb_arad_kernels: pair kernel smem attribute"));
     FMLB_TRY(cuda_status(cudaFuncSetAttribute(arad_f64_self_kernel,
                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1627,7 +1820,7 @@ static int arad_kernels_impl(const double *X1, const double *Z1, const int *N1, 
                 s.X, s.Z, s.N, s.nm, amax, ci, s.w);
             if (precision == 1) {
                 arad_sort_records_kernel<<<s.nm, FC_WARPS * 32, 0, st>>>(s.w, s.N, s.nm, amax, ci);
-                arad_fast_self_kernel<<<s.nm, FC_WARPS * 32, sizeof(FastSmem), st>>>(
+                arad_fast_self_kernel<<<s.nm, FC_WARPS * 32, kFastSmem, st>>>(
                     s.w, s.N, s.nm, amax, P, ci);
             } else {
                 arad_f64_self_kernel<<<s.nm, 32, f64_self_smem_bytes(amax), st>>>(
@@ -1668,7 +1861,7 @@ static int arad_kernels_impl(const double *X1, const double *Z1, const int *N1, 
                 const long long nbi = ceil_div(nm1, FC_BM), nbj = ceil_div(nm2, FC_BM);
                 const long long nblk = symmetric ? nbi * (nbi + 1) / 2 : nbi * nbj;
                 FMLB_REQUIRE(nblk < (1LL << 31), "fmlb_arad_kernels: too many molecule blocks");
-                arad_fast_pair_kernel<<<(unsigned)nblk, FC_WARPS * 32, sizeof(FastSmem), st>>>(
+                arad_fast_pair_kernel<<<(unsigned)nblk, FC_WARPS * 32, kFastSmem, st>>>(
                     w1, N1, nm1, w2, N2, nm2, amax, P, ci, sig, ns, symmetric, Ks);
                 FMLB_TRY(launch_status("arad_fast_pair_kernel"));
             }
