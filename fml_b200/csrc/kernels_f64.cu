@@ -5,7 +5,7 @@
 // scale = -0.5/sigma^2) or abs (Laplacian, scale = -1/sigma). Every sigma is
 // emitted from one pass over the descriptors.
 //
-// Tiles of 64 x 64 outputs (16 x 64 for small problems) per 128-thread CTA,
+// Tiles of 64 x 64 outputs (32 x 64 and 16 x 64 for small problems) per 128-thread CTA,
 // dist_tile.cuh. Symmetric mode launches only the tiles on or below the
 // diagonal and writes the mirror through a shared-memory transpose.
 #include <math.h>
@@ -16,44 +16,53 @@
 namespace fmlb {
 namespace {
 
-constexpr int BM = 64, BN = dist::DT_N, TPB = dist::DT_TPB, MAXSIG = 32;
+constexpr int BN = dist::DT_N, TPB = dist::DT_TPB, MAXSIG = 32;
 
-constexpr int kSmallTilesPerSm = 4;  // 16-row tiles per SM up to which they are used
+// Few tiles leave an SM one warp per FP64 unit, which cannot keep it busy: 16-row
+// tiles up to one per SM, 32-row ones up to two 64-row tiles per SM. us on d = 276
+// with 16, 32 and 64 rows: 1 x 1000 19, 23, 68; 128 x 2000 34, 27, 50; 1000 x 1000
+// symmetric 97, 39, 70; 1600 symmetric 222, 85, 84; 2000 x 2000 350, 216, 179.
+constexpr int kSmallTilesPerSm = 1, kHalfTilesPerSm = 2;
 
 struct SigmaScales {
     double s[MAXSIG];
 };
 
+// Tiles of 16 RI x 64. Symmetric: the tiles of the 64 x 64 blocks on or below the
+// diagonal, one or two (RI = 2) to a block.
 template <bool kL1, int RI>
-__global__ void __launch_bounds__(TPB, RI == 4 ? 4 : 8)
+__global__ void __launch_bounds__(TPB, RI == 4 ? 4 : RI == 2 ? 6 : 8)
 distance_kernel_f64(const double *__restrict__ A, int na, int lda, const double *__restrict__ B,
                     int nb, int ldb, int d, const __grid_constant__ SigmaScales sc, int nsig,
                     double *__restrict__ K, long long ldk, long long sstride, int symmetric) {
-    // the stage and (square tiles) the transpose share one buffer
-    constexpr int kT = BN * (BM + 1);
-    __shared__ double smem[RI == 4 && kT > dist::DT_STAGE ? kT : dist::DT_STAGE];
+    // the stage and the transpose share one buffer
+    constexpr int BM = 16 * RI, kT = BN * (BM + 1), kPerBlock = BN / BM;
+    __shared__ double smem[RI > 1 && kT > dist::DT_STAGE ? kT : dist::DT_STAGE];
     double(*T)[BM + 1] = reinterpret_cast<double(*)[BM + 1]>(smem);
 
-    int by, bx;
+    int by, bx, row0;
     if (symmetric) {
-        const long long t = blockIdx.x;
+        const long long t = blockIdx.x / kPerBlock;
         by = (int)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
         while ((long long)by * (by + 1) / 2 > t) --by;
         while ((long long)(by + 1) * (by + 2) / 2 <= t) ++by;
         bx = (int)(t - (long long)by * (by + 1) / 2);
+        row0 = by * BN + blockIdx.x % kPerBlock * BM;
+        if (row0 >= na) return;
     } else {
         bx = blockIdx.x;
         by = blockIdx.y;
+        row0 = by * BM;
     }
-    const int row0 = by * 16 * RI, col0 = bx * BN;
-    const int nr = min(16 * RI, na - row0), nc = min(BN, nb - col0);
+    const int col0 = bx * BN;
+    const int nr = min(BM, na - row0), nc = min(BN, nb - col0);
     double acc[RI][8];
     dist::dist_tile<kL1 ? dist::kAbs : dist::kSquare, RI>(
         acc, smem, [&](int r) { return A + (size_t)(row0 + r) * lda; },
         [&](int c) { return B + (size_t)(col0 + c) * ldb; }, nr, nc, d);
 
     const int r0 = dist::first_row<RI>(), c0 = dist::first_col();
-    const bool mirror = RI == 4 && symmetric && by > bx;
+    const bool mirror = RI > 1 && symmetric && by > bx;
     if (mirror) __syncthreads();  // the stage becomes the transpose
     for (int s = 0; s < nsig; ++s) {
         double *Ks = K + s * sstride;
@@ -103,15 +112,19 @@ int launch_distance(const double *A, int na, int lda, const double *B, int nb, i
             sc.s[s] = kL1 ? -1.0 / sg : -0.5 / (sg * sg);  // fkernels.f90:334 / :367
         }
         double *Ks = K + s0 * sstride;
-        // 64-row tiles, only those on or below the diagonal where symmetric; the
-        // whole matrix in 16-row tiles while that is at most a few tiles per SM
-        // (the k-loop's latency counts there, not the rate)
-        const long long nt = ceil_div(na, BM), ntc = ceil_div(nb, BN);
+        // only the tiles on or below the diagonal where symmetric; the whole matrix
+        // in 16-row tiles, where the k-loop's latency counts and not the work
+        const long long nt = ceil_div(na, BN), ntc = ceil_div(nb, BN);
         const long long nblk = symmetric ? nt * (nt + 1) / 2 : nt * ntc;
         if (4 * nt * ntc <= kSmallTilesPerSm * sm_count()) {
             const dim3 grid((unsigned)ntc, ceil_div(na, 16));
             distance_kernel_f64<kL1, 1><<<grid, TPB, 0, st>>>(A, na, lda, B, nb, ldb, d, sc, ns,
                                                               Ks, ldk, sstride, 0);
+        } else if (nblk <= kHalfTilesPerSm * sm_count()) {
+            const dim3 grid = symmetric ? dim3((unsigned)(2 * nblk))
+                                        : dim3((unsigned)ntc, ceil_div(na, 32));
+            distance_kernel_f64<kL1, 2><<<grid, TPB, 0, st>>>(A, na, lda, B, nb, ldb, d, sc, ns,
+                                                              Ks, ldk, sstride, symmetric);
         } else if (symmetric) {
             FMLB_REQUIRE(nblk < (1LL << 31), "%s: too many tiles", name);
             distance_kernel_f64<kL1, 4><<<(unsigned)nblk, TPB, 0, st>>>(

@@ -39,7 +39,7 @@ __global__ void add_diagonal_kernel(double *A, long long lda, int n, double lam)
 // 16 RI queries x CHUNK training points per cluster. A query's sums are formed
 // in the same order whatever RI and the queries beside it are.
 template <bool kL1, int RI>
-__global__ void __cluster_dims__(1, 1, PARTS) __launch_bounds__(TPB, RI == 4 ? 4 : 8)
+__global__ void __cluster_dims__(1, 1, PARTS) __launch_bounds__(TPB, RI == 4 ? 4 : RI == 2 ? 6 : 8)
 predict_partial_kernel(const double *__restrict__ Q, int nq, int ldq, const double *__restrict__ T,
                        int nt, int ldt, int d, const __grid_constant__ Scales sc, int nsig,
                        const double *__restrict__ alpha, long long lda_alpha,
@@ -96,22 +96,27 @@ predict_partial_kernel(const double *__restrict__ Q, int nq, int ldq, const doub
     cluster.sync();  // no CTA leaves while its sums are read
 }
 
-// The partial sums of every chunk. 16-query tiles while the 64-query ones would
-// not give every SM two.
+// The partial sums of every chunk, in tiles of 16, 32 or 64 queries by the number
+// of CTAs that the largest would give. us for 16, 32, 64 queries, d = 276: 200 x 1000
+// 48, 56, 107; 500 x 1000 72, 74, 107; 1000 x 1000 118, 78, 115; 2000 x 1000 220, 139,
+// 151; 1000 x 2000 220, 140, 130; 2000 x 2000 396, 257, 225.
 int launch_predict_partial(int kind, const double *Xq, int nq, int ldq, const double *Xt, int nt,
                            int ldt, int d, const Scales &sc, int nsigma, const double *alpha,
                            long long lda_alpha, double *partial, cudaStream_t st) {
     const int nsplit = ceil_div(nt, CHUNK);
-    const bool small = (long long)ceil_div(nq, 64) * ceil_div(nt, PART) < 2LL * sm_count();
-    const dim3 grid(ceil_div(nq, small ? 16 : 64), nsplit, PARTS);
+    const long long tiles = (long long)ceil_div(nq, 64) * ceil_div(nt, PART);
+    const int ri = 2 * tiles <= sm_count() ? 1 : 2 * tiles <= 3 * sm_count() ? 2 : 4;
+    const dim3 grid(ceil_div(nq, 16 * ri), nsplit, PARTS);
 #define FMLB_PREDICT(L1, RI)                                                                   \
     predict_partial_kernel<L1, RI><<<grid, TPB, 0, st>>>(Xq, nq, ldq, Xt, nt, ldt, d, sc,     \
                                                          nsigma, alpha, lda_alpha, partial)
     if (kind == 0) {
-        if (small) FMLB_PREDICT(false, 1);
+        if (ri == 1) FMLB_PREDICT(false, 1);
+        else if (ri == 2) FMLB_PREDICT(false, 2);
         else FMLB_PREDICT(false, 4);
     } else {
-        if (small) FMLB_PREDICT(true, 1);
+        if (ri == 1) FMLB_PREDICT(true, 1);
+        else if (ri == 2) FMLB_PREDICT(true, 2);
         else FMLB_PREDICT(true, 4);
     }
 #undef FMLB_PREDICT
