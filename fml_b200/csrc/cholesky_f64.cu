@@ -66,21 +66,25 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 // ---- 1. diagonal block ----------------------------------------------------
-// The 128 x 128 block is factored in four 32-column steps. In step J one warp
-// factors and inverts the 32 x 32 diagonal sub-block in registers with warp
-// shuffles only; the whole CTA then solves the 32-column sub-panel below it
-// (a product with the sub-block's inverse) and updates the rest of the block,
-// both on the FP64 tensor cores. Only the four 32 x 32 inverses are formed
-// here: the panel solve needs no more, and the block inverses of the triangular
-// solves come from block_inverse_kernel, once, for all blocks side by side.
+// The 128 x 128 block is factored in four 32-column steps:
+//   warp 0 factors the 32 x 32 diagonal sub-block in registers, warp 1 follows it
+//   by eight columns with the sub-block's inverse, and the other warps meanwhile
+//   do what is left of the update by the step before;
+//   all warps: the 32-column sub-panel below it (a product with the inverse), then
+//   the update of the next diagonal sub-block, on the FP64 tensor cores.
+// Only the four 32 x 32 inverses are formed here: the panel solve needs no more,
+// and the block inverses of the triangular solves come from block_inverse_kernel,
+// once, for all blocks side by side.
 //
-// Bound by the latency of the 128 serial pivots. With factor and inverse in
-// separate passes, each a shuffle per entry and a division per column, the
-// block products as shared-memory FMA loops and the whole inverse assembled on
-// this path, a block took 190 us.
+// Bound by the latency of the 128 serial pivots, about 190 cycles each. 24 us a
+// block; 36 with the inverse's updates and the whole block's behind the pivots on
+// the one warp's path and the column's stores, with their bank conflicts, among them;
+// 190 with factor and inverse in separate passes and the block products as
+// shared-memory FMA loops.
 constexpr int LDL = NB + 4;  // row pitch: the fragments' rows fall in distinct banks
 constexpr int SB = 32, NSB = NB / SB, LDW = SB + 4;
-constexpr size_t kPotf2Smem = ((size_t)NB * LDL + (size_t)SB * LDW) * sizeof(double);
+constexpr size_t kPotf2Smem =  // the block, two inverses, the sub-block's columns and roots
+    ((size_t)NB * LDL + 2 * (size_t)(SB * LDW + SB * SB + 2 * SB)) * sizeof(double);
 
 __device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -88,117 +92,246 @@ __device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
                  : "d"(a), "d"(b));
 }
 
-// One warp factors the 32 x 32 diagonal sub-block and inverts the factor. Lane
-// r holds row r of the block (a) and column r of the inverse (v) in registers;
-// the column steps are unrolled by template recursion, so every register index
-// is a constant. A step scales column J by 1 / sqrt(pivot) and then, from one
-// broadcast per entry L[c][J], updates both the rest of the block and the
-// inverse's forward substitution (right-looking): two independent FMA streams.
-// The next pivot goes ahead of them by shuffles, so its reciprocal root is
-// formed beside them; the other entries of the column are broadcast through
-// shared memory (two to a load, where a shuffle takes two instructions each).
-// Entries above the diagonal hold values that nothing reads.
-template <int J>
-struct WarpFactorInvert32 {
-    __device__ __forceinline__ static void run(double (&a)[SB], double (&v)[SB], double piv,
-                                               double *col, int lane, int &fail) {
-        if (!(piv > 0.0) && !fail) fail = J + 1;  // later columns are NaN and not stored
-        const double inv = rsqrt(piv);
-        double root = piv * inv;  // sqrt(piv), corrected once
-        root = fma(0.5 * inv, fma(-root, root, piv), root);
-        a[J] = lane == J ? root : a[J] * inv;
-        v[J] *= inv;
-        const double lij = a[J], vj = v[J];
-        double *mine = col + (J & 1) * SB;  // two buffers: one barrier a step
-        mine[lane] = lij;
-        double next = 0.0;
-        if (J + 1 < SB) {
-            const double l1 = __shfl_sync(0xffffffffu, lij, J + 1);
-            a[(J + 1) % SB] = fma(-lij, l1, a[(J + 1) % SB]);
-            v[(J + 1) % SB] = fma(-l1, vj, v[(J + 1) % SB]);
-            next = __shfl_sync(0xffffffffu, a[(J + 1) % SB], J + 1);
-        }
-        __syncwarp();
-#pragma unroll
-        for (int c = (J + 2) & ~1; c < SB; c += 2) {
-            const double2 l = *reinterpret_cast<const double2 *>(mine + c);  // L[c][J], L[c+1][J]
-            if (c > J + 1) {
-                a[c] = fma(-lij, l.x, a[c]);
-                v[c] = fma(-l.x, vj, v[c]);
-            }
-            a[c + 1] = fma(-lij, l.y, a[c + 1]);
-            v[c + 1] = fma(-l.y, vj, v[c + 1]);
-        }
-        WarpFactorInvert32<J + 1>::run(a, v, next, col, lane, fail);
-    }
-};
-template <>
-struct WarpFactorInvert32<SB> {
-    __device__ __forceinline__ static void run(double (&)[SB], double (&)[SB], double, double *,
-                                               int, int &) {}
+// 1 / sqrt(x) for normal x by a third-order step from the hardware's approximation
+// (Householder's method: e = 1 - x y^2, y (1 + e / 2 + 3 e^2 / 8)), without branches.
+__device__ __forceinline__ double rsqrt_normal(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(fma(0.375, e, 0.5), y * e, y);
+}
+
+// Named barriers between warps 0 and 1, one for each eight columns.
+__device__ __forceinline__ void columns_done(int id) {
+    asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory");
+}
+__device__ __forceinline__ void columns_wait(int id) {
+    asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
+}
+
+// What a column step of the sub-block's factorisation hands to the next, the same
+// in every lane: column J's pivot and its reciprocal root, the entry below the pivot
+// (unscaled) and the diagonal entry after that one, both as the steps before J left
+// them.
+struct PotrfStep {
+    double piv, inv, below, diag;
 };
 
-// Factors the sub-block at L[b0.., b0..] in place and writes its inverse into W
-// (row-major, zeros above the diagonal). Returns the 1-based failing column or
-// 0 (the same value in every lane).
-__device__ __forceinline__ int warp_potrf_inv32(double (*L)[LDL], int b0, double (*W)[LDW],
-                                                double *col) {
+// Eight column steps, `WIDTH` columns left at the first: a[c] holds the lane's
+// (row's) entry of column J + c. A step scales column J by inv, stores it and
+// updates the columns after it into the registers one place down. Every lane forms
+// the next pivot by itself from `below` and `diag`, which were broadcast a step
+// ahead, so that a column's chain is the reciprocal root and two operations, with
+// the broadcasts and the updates beside it. The column goes through shared memory
+// (two entries to a load, where a shuffle takes two instructions each). Entries above
+// the diagonal and past the last column hold values that nothing reads.
+template <int WIDTH, bool kCareful>
+__device__ __forceinline__ void potrf_steps(double (&a)[SB], PotrfStep &s, int J0, double *cols,
+                                            double *invs, double &mine) {
     const int lane = threadIdx.x & 31;
-    double a[SB], v[SB];
+#pragma unroll 1
+    for (int q = 0; q < 8; ++q) {
+        const int J = J0 + q;
+        const double lij = a[0] * s.inv, l1 = s.below * s.inv, piv = fma(-l1, l1, s.diag);
+        double *col = cols + J * SB;  // L[J + c][J] at c
+        col[(lane - J) & 31] = lij;
+        invs[J] = s.inv;
+        if (lane == J) mine = s.piv;
+        a[1] = fma(-lij, l1, a[1]);
+        s.below = __shfl_sync(0xffffffffu, a[1], (J + 2) & 31);
+        s.diag = __shfl_sync(0xffffffffu, fma(-lij, lij, a[2]), (J + 2) & 31);
+        __syncwarp();
+        s.piv = piv;
+        s.inv = kCareful ? rsqrt(piv) : rsqrt_normal(piv);
+        a[0] = a[1];
 #pragma unroll
-    for (int c = 0; c < SB; ++c) {
-        a[c] = c <= lane ? L[b0 + lane][b0 + c] : 0.0;
-        v[c] = c == lane ? 1.0 : 0.0;
+        for (int c = 2; c < WIDTH; c += 2) {
+            const double2 l = *reinterpret_cast<const double2 *>(col + c);
+            a[c - 1] = fma(-lij, l.x, a[c]);
+            a[c] = fma(-lij, l.y, a[c + 1 < SB ? c + 1 : c]);
+        }
     }
-    int fail = 0;
-    WarpFactorInvert32<0>::run(a, v, __shfl_sync(0xffffffffu, a[0], 0), col, lane, fail);
-    if (fail) return fail;
+    columns_done(1 + J0 / 8);
+}
+
+// Warp 0: factors the 32 x 32 sub-block at L[b0.., b0..] into cols, with the pivots
+// and their reciprocal roots in pivs and invs. Returns the 1-based failing column, 0
+// or, unless kCareful, -1 (the same in every lane) for a pivot that is not a normal
+// number: the library's reciprocal root then has to be used.
+template <bool kCareful>
+__device__ __forceinline__ int warp_potrf32(double (*L)[LDL], int b0, double *cols, double *invs,
+                                            double *pivs) {
+    const int lane = threadIdx.x & 31;
+    double a[SB];
 #pragma unroll
-    for (int c = 0; c < SB; ++c) {
-        if (c <= lane) L[b0 + lane][b0 + c] = a[c];
-        W[c][lane] = v[c];
+    for (int c = 0; c < SB; ++c) a[c] = c <= lane ? L[b0 + lane][b0 + c] : 0.0;
+    PotrfStep s;
+    s.piv = __shfl_sync(0xffffffffu, a[0], 0);
+    s.inv = rsqrt(s.piv);
+    s.below = __shfl_sync(0xffffffffu, a[0], 1);
+    s.diag = __shfl_sync(0xffffffffu, a[1], 1);
+    double mine = 0.0;
+    static_assert(SB == 32, "four times eight steps");
+    potrf_steps<32, kCareful>(a, s, 0, cols, invs, mine);
+    potrf_steps<24, kCareful>(a, s, 8, cols, invs, mine);
+    potrf_steps<16, kCareful>(a, s, 16, cols, invs, mine);
+    potrf_steps<8, kCareful>(a, s, 24, cols, invs, mine);
+    pivs[lane] = mine;
+    const bool normal = mine >= 2.2250738585072014e-308 && mine <= 1.7976931348623157e308;
+    const unsigned other = __ballot_sync(0xffffffffu, kCareful ? !(mine > 0.0) : !normal);
+    if (!other) return 0;
+    const int first = __ffs(other) - 1;
+    if (!kCareful && __shfl_sync(0xffffffffu, mine, first) > 0.0) return -1;
+    return first + 1;
+}
+
+// Eight row steps of the forward substitution for the inverse: v[c] holds the
+// lane's (column's) entry of row J + c, moved down as above.
+template <int WIDTH>
+__device__ __forceinline__ void inverse_steps(double (&v)[SB], int J0, double (*W)[LDW],
+                                              const double *cols, const double *invs) {
+    const int lane = threadIdx.x & 31;
+    columns_wait(1 + J0 / 8);
+#pragma unroll 1
+    for (int J = J0; J < J0 + 8; ++J) {
+        const double vj = v[0] * invs[J];
+        W[J][lane] = vj;
+#pragma unroll
+        for (int c = 0; c < WIDTH; c += 2) {
+            const double2 l = *reinterpret_cast<const double2 *>(cols + J * SB + c);
+            if (c > 0) v[c - 1] = fma(-l.x, vj, v[c]);
+            v[c] = fma(-l.y, vj, v[c + 1 < SB ? c + 1 : c]);
+        }
     }
-    __syncwarp();
-    return 0;
+}
+
+// Warp 1: the inverse of the sub-block that warp 0 factors, into W (row-major, zeros
+// above the diagonal).
+__device__ __forceinline__ void warp_inverse32(double (*W)[LDW], const double *cols,
+                                               const double *invs) {
+    const int lane = threadIdx.x & 31;
+    double v[SB];
+#pragma unroll
+    for (int c = 0; c < SB; ++c) v[c] = c == lane ? 1.0 : 0.0;
+    inverse_steps<32>(v, 0, W, cols, invs);
+    inverse_steps<24>(v, 8, W, cols, invs);
+    inverse_steps<16>(v, 16, W, cols, invs);
+    inverse_steps<8>(v, 24, W, cols, invs);
+}
+
+// A factored sub-block to its place in the block, its diagonal as the root of the
+// pivot, corrected once, and its inverse to its place in the block inverse: rows
+// `part`, part + parts and so on.
+__device__ __forceinline__ void put_subblock(double (*L)[LDL], double *__restrict__ Linv, int b0,
+                                             const double *step, int part, int parts) {
+    const int lane = threadIdx.x & 31;
+    const double *W = step, *cols = W + SB * LDW, *pivs = cols + SB * SB, *invs = pivs + SB;
+#pragma unroll 4
+    for (int r = part; r < SB; r += parts) {
+        const double piv = pivs[r], inv = invs[r], root = piv * inv;
+        const double v = lane == r ? fma(0.5 * inv, fma(-root, root, piv), root)
+                                   : cols[lane * SB + ((r - lane) & 31)];
+        if (lane <= r) L[b0 + r][b0 + lane] = v;
+        Linv[(size_t)(b0 + r) * NB + b0 + lane] = W[r * LDW + lane];
+    }
+}
+
+// T 8 x 8 tiles of the block side by side: L[m.., c..] -= L[m.., b0..] L[c.., b0..]^T
+template <int T>
+__device__ __forceinline__ void update_tiles(double (*L)[LDL], int m, int c, int b0) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
+    double o[T][4][2];
+#pragma unroll
+    for (int t = 0; t < T; ++t)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) o[t][q][0] = o[t][q][1] = 0.0;
+#pragma unroll
+    for (int k = 0; k < SB; k += 4) {
+        const double x = L[m + g][b0 + k + tq];
+#pragma unroll
+        for (int t = 0; t < T; ++t) dmma_8x8x4(o[t][k / 4 % 4], x, L[c + 8 * t + g][b0 + k + tq]);
+    }
+#pragma unroll
+    for (int t = 0; t < T; ++t)
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+            L[m + g][c + 8 * t + 2 * tq + q] -=
+                (o[t][0][q] + o[t][1][q]) + (o[t][2][q] + o[t][3][q]);
 }
 
 __global__ void __launch_bounds__(TPB, 1)
 potf2_block_kernel(double *__restrict__ A, long long lda, int k0, int kn,
                    double *__restrict__ Linv, int *__restrict__ info) {
-    extern __shared__ double potf2_smem[];
+    extern __shared__ __align__(16) double potf2_smem[];
     double(*L)[LDL] = reinterpret_cast<double(*)[LDL]>(potf2_smem);
-    double(*W)[LDW] = reinterpret_cast<double(*)[LDW]>(potf2_smem + NB * LDL);
+    constexpr int kWarps = TPB / 32, kStep = SB * LDW + SB * SB + 2 * SB;
+    const auto step = [&](int J) {  // two buffers: inverse, columns, pivots, their roots
+        return potf2_smem + NB * LDL + (J & 1) * kStep;
+    };
     __shared__ int bad;
-    __shared__ __align__(16) double col[2 * SB];
-    pdl_wait();
-    if (failed(info)) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, tq = lane & 3;  // fragment row / k (A, B), row / column pair (C)
-    for (int t = tid; t < NB * NB; t += TPB) {  // all loads in flight together
-        const int r = t >> 7, c = t & (NB - 1);
-        if (r < kn && c <= r) cp_async_8(&L[r][c], A + (size_t)(k0 + r) * lda + (k0 + c), 8);
-        else L[r][c] = r == c ? 1.0 : 0.0;  // identity padding past kn keeps the block SPD
-    }
+    double *Ak = A + (size_t)k0 * lda + k0;
+    const bool wide = (uintptr_t)Ak % 16 == 0 && lda % 2 == 0;
     if (tid == 0) bad = 0;
+    pdl_wait();
+    if (wide) {
+        for (int r = warp; r < kn; r += kWarps)  // all loads in flight together
+#pragma unroll
+            for (int c = 2 * lane; c < NB; c += 64)
+                if (c <= r) cp_async_16(&L[r][c], Ak + (size_t)r * lda + c, c < r ? 16 : 8);
+    } else {
+        for (int r = warp; r < kn; r += kWarps)
+#pragma unroll
+            for (int c = lane; c < NB; c += 32)
+                if (c <= r) cp_async_8(&L[r][c], Ak + (size_t)r * lda + c, 8);
+    }
+    for (int r = kn + warp; r < NB; r += kWarps)  // identity past kn keeps the block SPD
+        for (int c = lane; c <= r; c += 32) L[r][c] = r == c ? 1.0 : 0.0;
     cp_async_commit();
+    const bool stop = failed(info);
     cp_async_wait<0>();
+    if (stop) return;
     __syncthreads();
     for (int J = 0; J < NSB; ++J) {
-        const int b0 = J * SB, r0 = b0 + SB;
+        const int b0 = J * SB, r0 = b0 + SB, p0 = b0 - SB;
+        double(*W)[LDW] = reinterpret_cast<double(*)[LDW]>(step(J));
+        double *cols = step(J) + SB * LDW, *pivs = cols + SB * SB, *invs = pivs + SB;
         if (warp == 0) {
-            const int f = warp_potrf_inv32(L, b0, W, col);
-            if (f && lane == 0) bad = b0 + f;
+            const int f = warp_potrf32<false>(L, b0, cols, invs, pivs);
+            if (f && lane == 0) bad = f > 0 ? b0 + f : f;
+        } else if (warp == 1) {
+            warp_inverse32(W, cols, invs);
+        } else if (J > 0 && (warp & 2)) {
+            // the rest of the update by step J - 1, two 8 x 8 tiles at a time (the
+            // second may lie above the diagonal), by the warps that share no
+            // scheduler with warps 0 and 1
+            const int nt = (NB - b0) / 8, turn = (warp & 1) + (warp >> 2) * 2;
+            int item = 0;
+            for (int ti = SB / 8; ti < nt; ++ti)
+                for (int tj = 0; tj <= ti; tj += 2)
+                    if ((item++ & 3) == turn) update_tiles<2>(L, b0 + 8 * ti, b0 + 8 * tj, p0);
+        } else if (J > 0) {
+            put_subblock(L, Linv, p0, step(J - 1), warp & 1, 2);
         }
         __syncthreads();
+        if (bad < 0) {  // a pivot outside the normal numbers
+            __syncthreads();
+            if (warp == 0) {
+                const int f = warp_potrf32<true>(L, b0, cols, invs, pivs);
+                if (lane == 0) bad = f ? b0 + f : 0;
+            } else if (warp == 1) {
+                warp_inverse32(W, cols, invs);
+            }
+            __syncthreads();
+        }
         if (bad) {
             if (tid == 0) atomicCAS(info, 0, k0 + bad);
             return;
         }
-        // the sub-block's inverse to its place in the block inverse
-        for (int t = tid; t < SB * SB; t += TPB)
-            Linv[(size_t)(b0 + t / SB) * NB + b0 + t % SB] = W[t / SB][t % SB];
+        if (J == NSB - 1) break;
         // sub-panel solve, 8 rows per warp and turn: X <- X inv(D)^T
-        for (int m = r0 + warp * 8; m < NB; m += 8 * (TPB / 32)) {
+        for (int m = r0 + warp * 8; m < NB; m += 8 * kWarps) {
             double x[SB / 4], o[SB / 8][2];
 #pragma unroll
             for (int k = 0; k < SB / 4; ++k) x[k] = L[m + g][b0 + 4 * k + tq];
@@ -217,29 +350,21 @@ potf2_block_kernel(double *__restrict__ A, long long lda, int k0, int kn,
             }
         }
         __syncthreads();
-        // update of the rest of the block, 8 x 8 tiles on or below the diagonal
-        const int nt = (NB - r0) / 8;
-        for (int t = warp; t < nt * (nt + 1) / 2; t += TPB / 32) {
-            int ti = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
-            while (ti * (ti + 1) / 2 > t) --ti;
-            while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
-            const int m = r0 + 8 * ti, c = r0 + 8 * (t - ti * (ti + 1) / 2);
-            double o0[2] = {0.0, 0.0}, o1[2] = {0.0, 0.0};
-#pragma unroll
-            for (int k = 0; k < SB; k += 8) {
-                dmma_8x8x4(o0, L[m + g][b0 + k + tq], L[c + g][b0 + k + tq]);
-                dmma_8x8x4(o1, L[m + g][b0 + k + 4 + tq], L[c + g][b0 + k + 4 + tq]);
-            }
-            L[m + g][c + 2 * tq] -= o0[0] + o1[0];
-            L[m + g][c + 2 * tq + 1] -= o0[1] + o1[1];
+        // update of the next diagonal sub-block: its ten tiles on or below the diagonal
+        for (int t = warp; t < 10; t += kWarps) {
+            const int ti = (t > 0) + (t > 2) + (t > 5), tj = t - ti * (ti + 1) / 2;
+            update_tiles<1>(L, r0 + 8 * ti, r0 + 8 * tj, b0);
         }
         __syncthreads();
     }
-    // factor back to global
-    for (int t = tid; t < NB * NB; t += TPB) {
-        const int r = t >> 7, c = t & (NB - 1);
-        if (r < kn && c <= r) A[(size_t)(k0 + r) * lda + (k0 + c)] = L[r][c];
-    }
+    put_subblock(L, Linv, NB - SB, step(NSB - 1), warp, kWarps);
+    __syncthreads();
+    // factor back to global (16-byte stores took 4500 cycles, these 2700)
+#pragma unroll 4
+    for (int r = warp; r < kn; r += kWarps)
+#pragma unroll
+        for (int c = lane; c < NB; c += 32)
+            if (c <= r) Ak[(size_t)r * lda + c] = L[r][c];
     pdl_launch_dependents();
 }
 
