@@ -382,57 +382,88 @@ constexpr size_t kTrsmSmem =
 __global__ void __launch_bounds__(TPB)
 panel_trsm_kernel(double *__restrict__ A, long long lda, int n, int k0,
                   const double *__restrict__ Linv, const int *__restrict__ info) {
-    extern __shared__ double trsm_smem[];
+    extern __shared__ __align__(16) double trsm_smem[];
     double(*X)[LDL] = reinterpret_cast<double(*)[LDL]>(trsm_smem);
     double *blocks = trsm_smem + TRSM_ROWS * LDL;  // (R, C) at R (R + 1) / 2 + C
-    pdl_wait();
-    if (failed(info)) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, tq = lane & 3;
-    for (int t = tid; t < NB * NB; t += TPB) {
-        const int r = t / NB, c = t % NB, R = r / SB, C = c / SB;
-        if (C <= R)
-            cp_async_8(&blocks[(R * (R + 1) / 2 + C) * TRSM_BLK + (r % SB) * LDW + c % SB],
-                       C == R ? Linv + t : A + (size_t)(k0 + r) * lda + k0 + c, 8);
-    }
-    const int m = (warp & 3) * 8, h = (warp >> 2) * 16;  // rows m.., columns h.. of each block
-    for (int r0 = k0 + NB + blockIdx.x * TRSM_ROWS; r0 < n; r0 += gridDim.x * TRSM_ROWS) {
-        for (int t = tid; t < TRSM_ROWS * NB; t += TPB) {
+    const bool wide = ((uintptr_t)A | (uintptr_t)Linv) % 16 == 0 && lda % 2 == 0;
+    pdl_wait();
+    const auto place = [&](int r, int c) {
+        const int R = r / SB, C = c / SB;
+        return blocks + (R * (R + 1) / 2 + C) * TRSM_BLK + (r % SB) * LDW + c % SB;
+    };
+    const double *Ak = A + (size_t)k0 * lda + k0;
+    if (wide) {
+        for (int t = tid; t < NB * NB / 2; t += TPB) {
+            const int r = t / (NB / 2), c = t % (NB / 2) * 2;
+            if (c / SB <= r / SB)
+                cp_async_16(place(r, c), c / SB == r / SB ? Linv + 2 * t : Ak + (size_t)r * lda + c,
+                            16);
+        }
+    } else {
+        for (int t = tid; t < NB * NB; t += TPB) {
             const int r = t / NB, c = t % NB;
-            cp_async_8(&X[r][c], A + (size_t)min(r0 + r, n - 1) * lda + k0 + c, r0 + r < n ? 8 : 0);
+            if (c / SB <= r / SB)
+                cp_async_8(place(r, c), c / SB == r / SB ? Linv + t : Ak + (size_t)r * lda + c, 8);
+        }
+    }
+    const bool stop = failed(info);
+    const int m = (warp & 3) * 8, h = (warp >> 2) * 16;  // rows m.., columns h.. of each block
+    for (int r0 = k0 + NB + blockIdx.x * TRSM_ROWS; r0 < n && !stop;
+         r0 += gridDim.x * TRSM_ROWS) {
+        if (wide) {
+            for (int t = tid; t < TRSM_ROWS * NB / 2; t += TPB) {
+                const int r = t / (NB / 2), c = t % (NB / 2) * 2;
+                cp_async_16(&X[r][c], A + (size_t)min(r0 + r, n - 1) * lda + k0 + c,
+                            r0 + r < n ? 16 : 0);
+            }
+        } else {
+            for (int t = tid; t < TRSM_ROWS * NB; t += TPB) {
+                const int r = t / NB, c = t % NB;
+                cp_async_8(&X[r][c], A + (size_t)min(r0 + r, n - 1) * lda + k0 + c,
+                           r0 + r < n ? 8 : 0);
+            }
         }
         cp_async_commit();
         cp_async_wait<0>();
         for (int J = 0; J < NSB; ++J) {
             const double *row = blocks + J * (J + 1) / 2 * TRSM_BLK + (h + g) * LDW + tq;
             __syncthreads();
-            double o[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+            double o[2][4][2] = {};  // four chains for each 8 x 8 tile
             for (int K = 0; K < J; ++K) {
 #pragma unroll
                 for (int k = 0; k < SB; k += 4) {
                     const double x = X[m + g][K * SB + k + tq];
 #pragma unroll
                     for (int c = 0; c < 2; ++c)
-                        dmma_8x8x4(o[c], x, row[K * TRSM_BLK + 8 * c * LDW + k]);
+                        dmma_8x8x4(o[c][k / 4 % 4], x, row[K * TRSM_BLK + 8 * c * LDW + k]);
                 }
             }
 #pragma unroll
             for (int c = 0; c < 2; ++c)
 #pragma unroll
-                for (int q = 0; q < 2; ++q) X[m + g][J * SB + h + 8 * c + 2 * tq + q] -= o[c][q];
+                for (int q = 0; q < 2; ++q) {
+                    X[m + g][J * SB + h + 8 * c + 2 * tq + q] -=
+                        (o[c][0][q] + o[c][1][q]) + (o[c][2][q] + o[c][3][q]);
+                    o[c][0][q] = o[c][1][q] = 0.0;
+                }
             __syncthreads();
-            o[0][0] = o[0][1] = o[1][0] = o[1][1] = 0.0;
-            for (int k = 0; k < h + 16; k += 4) {  // W_J is lower triangular
-                const double x = X[m + g][J * SB + k + tq];
+            for (int k = 0; k < h + 16; k += 8) {  // W_J is lower triangular
 #pragma unroll
-                for (int c = 0; c < 2; ++c)
-                    dmma_8x8x4(o[c], x, row[J * TRSM_BLK + 8 * c * LDW + k]);
+                for (int e = 0; e < 2; ++e) {
+                    const double x = X[m + g][J * SB + k + 4 * e + tq];
+#pragma unroll
+                    for (int c = 0; c < 2; ++c)
+                        dmma_8x8x4(o[c][e], x, row[J * TRSM_BLK + 8 * c * LDW + k + 4 * e]);
+                }
             }
             __syncthreads();
 #pragma unroll
             for (int c = 0; c < 2; ++c)
 #pragma unroll
-                for (int q = 0; q < 2; ++q) X[m + g][J * SB + h + 8 * c + 2 * tq + q] = o[c][q];
+                for (int q = 0; q < 2; ++q)
+                    X[m + g][J * SB + h + 8 * c + 2 * tq + q] = o[c][0][q] + o[c][1][q];
         }
         __syncthreads();
         for (int t = tid; t < TRSM_ROWS * NB; t += TPB) {
@@ -441,6 +472,7 @@ panel_trsm_kernel(double *__restrict__ A, long long lda, int n, int k0,
         }
         __syncthreads();
     }
+    cp_async_wait<0>();
     pdl_launch_dependents();
 }
 
@@ -610,7 +642,6 @@ syrk_dmma_kernel(double *__restrict__ C, long long ldc, int m, const double *__r
     constexpr int kFr = T::kFr, kFc = T::kFc;  // fragments of a warp: rows, columns
     extern __shared__ __align__(16) double sy_smem[];
     pdl_wait();
-    if (failed(info)) return;
     const long long t = blockIdx.x;
     int by, bx;
     if (strip_tiles > 0) {  // only the first strip_tiles column tiles of every row block
@@ -645,6 +676,10 @@ syrk_dmma_kernel(double *__restrict__ C, long long ldc, int m, const double *__r
         }
         cp_async_commit();
     }
+    if (failed(info)) {  // read while the first stages are on their way
+        cp_async_wait<0>();
+        return;
+    }
     for (int kt = 0; kt < nk; ++kt) {
         cp_async_wait<SY_STAGES - 2>();
         __syncthreads();
@@ -672,7 +707,8 @@ syrk_dmma_kernel(double *__restrict__ C, long long ldc, int m, const double *__r
     }
     cp_async_wait<0>();
     __syncthreads();  // every warp is done with the stage buffers
-    // Epilogue through shared memory: one coalesced pass loads the C tile,
+    // Epilogue through shared memory: one coalesced pass loads the C tile (all of
+    // it in flight at once; loads to registers waited for memory every few rows),
     // the fragments are subtracted there, one coalesced masked pass stores it
     // (keeps the 64 read-modify-writes per thread from serialising).
     double *Cs = sy_smem;  // T::kM x T::kCld doubles, fits in the stage area
@@ -680,15 +716,13 @@ syrk_dmma_kernel(double *__restrict__ C, long long ldc, int m, const double *__r
     for (int e = tid; e < T::kM * (T::kN / 2); e += SY_TPB) {
         const int r = e / (T::kN / 2), c = (e % (T::kN / 2)) * 2;
         const int gr = row0 + r, gc = col0 + c;
-        double v0 = 0.0, v1 = 0.0;
-        if (gr < m) {
-            const double *src = C + (size_t)gr * ldc + gc;
-            if (gc < m) v0 = src[0];
-            if (gc + 1 < m) v1 = src[1];
-        }
-        Cs[r * T::kCld + c] = v0;
-        Cs[r * T::kCld + c + 1] = v1;
+        const double *src = C + (size_t)gr * ldc + gc;
+        const bool in0 = gr < m && gc < m, in1 = gr < m && gc + 1 < m;
+        cp_async_8(Cs + r * T::kCld + c, in0 ? src : C, in0 ? 8 : 0);
+        cp_async_8(Cs + r * T::kCld + c + 1, in1 ? src + 1 : C, in1 ? 8 : 0);
     }
+    cp_async_commit();
+    cp_async_wait<0>();
     __syncthreads();
     // fragment (i, j): rows 8 i + g and columns 8 j + 2 tq + {0, 1} of the warp's tile
 #pragma unroll
