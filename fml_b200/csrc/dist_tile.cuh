@@ -3,7 +3,7 @@
 //
 // A CTA of 128 threads holds a (16 RI) x 64 tile of row pairs, 4 RI rows x 64
 // columns per warp and RI x 8 pairs per thread in registers. Features are
-// staged 8 at a time in shared memory, transposed, by asynchronous copies three
+// staged 8 (or 16) at a time in shared memory, transposed, by asynchronous copies three
 // chunks ahead. Features are added in ascending order by one thread per pair,
 // so a pair's distance does not depend on the tile that it falls in.
 //
@@ -22,9 +22,20 @@
 namespace fmlb {
 namespace dist {
 
-constexpr int DT_TPB = 128, DT_N = 64, DT_K = 8, DT_BUFS = 4;
-constexpr int DT_P = DT_N + 2;                    // row pitch: the transposing copies spread
-constexpr int DT_STAGE = DT_BUFS * 2 * DT_K * DT_P;  // doubles of the stage
+constexpr int DT_TPB = 128, DT_N = 64, DT_BUFS = 4;
+constexpr int DT_P = DT_N + 2;  // row pitch: the transposing copies spread
+
+// Features of a chunk, row pitch of A's part of it, doubles of the stage. Where the
+// tiles are 16 rows high few CTAs run, and the memory's latency per chunk is what
+// they take: 16 features, in a stage that would leave no room for four CTAs.
+template <int RI>
+__host__ __device__ constexpr int chunk() { return RI == 1 ? 16 : 8; }
+template <int RI>
+__host__ __device__ constexpr int pitch_a() { return RI == 1 ? 18 : DT_P; }
+template <int RI>
+__host__ __device__ constexpr int stage_doubles() {
+    return DT_BUFS * chunk<RI>() * (pitch_a<RI>() + DT_P);
+}
 
 enum Op { kSquare = 0, kAbs = 1, kSquareUnfused = 2 };
 
@@ -59,32 +70,34 @@ __device__ __forceinline__ int first_col() {
 template <Op kOp, int RI, typename RowA, typename RowB>
 __device__ __forceinline__ void dist_tile(double (&acc)[RI][8], double *stage, RowA row_a,
                                           RowB row_b, int nr, int nc, int d) {
-    constexpr int kRows = 16 * RI;
+    constexpr int kRows = 16 * RI, kK = chunk<RI>(), kPA = pitch_a<RI>();
+    constexpr int kPass = DT_TPB / kK, kChunk = kK * (kPA + DT_P);
     const int tid = threadIdx.x;
     const int r0 = first_row<RI>(), c0 = first_col();
-    // loader: 8 features of 16 rows a pass
-    const int lk = tid & (DT_K - 1), lr = tid / DT_K;
-    const double *pa[kRows / 16], *pb[DT_N / 16];
+    // loader: the chunk's features of kPass rows a pass
+    const int lk = tid & (kK - 1), lr = tid / kK;
+    const double *pa[kRows / kPass], *pb[DT_N / kPass];
 #pragma unroll
-    for (int q = 0; q < kRows / 16; ++q)
-        pa[q] = lr + 16 * q < nr ? row_a(lr + 16 * q) : nullptr;
+    for (int q = 0; q < kRows / kPass; ++q)
+        pa[q] = lr + kPass * q < nr ? row_a(lr + kPass * q) : nullptr;
 #pragma unroll
-    for (int q = 0; q < DT_N / 16; ++q) pb[q] = lr + 16 * q < nc ? row_b(lr + 16 * q) : nullptr;
+    for (int q = 0; q < DT_N / kPass; ++q)
+        pb[q] = lr + kPass * q < nc ? row_b(lr + kPass * q) : nullptr;
     const double *any = row_b(0);  // a valid address for the zero-filled copies
-    const int nk = (d + DT_K - 1) / DT_K;
+    const int nk = (d + kK - 1) / kK;
     auto copy = [&](int chunk) {
         if (chunk < nk) {
-            double *As = stage + (chunk % DT_BUFS) * 2 * DT_K * DT_P, *Bs = As + DT_K * DT_P;
-            const int f = chunk * DT_K + lk;
+            double *As = stage + (chunk % DT_BUFS) * kChunk, *Bs = As + kK * kPA;
+            const int f = chunk * kK + lk;
 #pragma unroll
-            for (int q = 0; q < kRows / 16; ++q) {
+            for (int q = 0; q < kRows / kPass; ++q) {
                 const bool ok = pa[q] && f < d;
-                copy8_async(As + lk * DT_P + lr + 16 * q, ok ? pa[q] + f : any, ok);
+                copy8_async(As + lk * kPA + lr + kPass * q, ok ? pa[q] + f : any, ok);
             }
 #pragma unroll
-            for (int q = 0; q < DT_N / 16; ++q) {
+            for (int q = 0; q < DT_N / kPass; ++q) {
                 const bool ok = pb[q] && f < d;
-                copy8_async(Bs + lk * DT_P + lr + 16 * q, ok ? pb[q] + f : any, ok);
+                copy8_async(Bs + lk * DT_P + lr + kPass * q, ok ? pb[q] + f : any, ok);
             }
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -102,14 +115,14 @@ __device__ __forceinline__ void dist_tile(double (&acc)[RI][8], double *stage, R
         asm volatile("cp.async.wait_group %0;\n" ::"n"(DT_BUFS - 2) : "memory");
         __syncthreads();  // chunk c has landed, and chunk c - 1 is no longer read
         copy(c + DT_BUFS - 1);
-        const double *As = stage + (c % DT_BUFS) * 2 * DT_K * DT_P + r0;
-        const double *Bs = stage + (c % DT_BUFS) * 2 * DT_K * DT_P + DT_K * DT_P + c0;
+        const double *As = stage + (c % DT_BUFS) * kChunk + r0;
+        const double *Bs = stage + (c % DT_BUFS) * kChunk + kK * kPA + c0;
         if (jn >= 8) {
 #pragma unroll
-            for (int kk = 0; kk < DT_K; ++kk) {
+            for (int kk = 0; kk < kK; ++kk) {
                 double a[RI], b[8];
 #pragma unroll
-                for (int i = 0; i < RI; ++i) a[i] = As[kk * DT_P + 4 * i];
+                for (int i = 0; i < RI; ++i) a[i] = As[kk * kPA + 4 * i];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) b[j] = Bs[kk * DT_P + 8 * j];
 #pragma unroll
@@ -119,10 +132,10 @@ __device__ __forceinline__ void dist_tile(double (&acc)[RI][8], double *stage, R
             }
         } else if (jn > 0) {
 #pragma unroll 2
-            for (int kk = 0; kk < DT_K; ++kk) {
+            for (int kk = 0; kk < kK; ++kk) {
                 double a[RI];
 #pragma unroll
-                for (int i = 0; i < RI; ++i) a[i] = As[kk * DT_P + 4 * i];
+                for (int i = 0; i < RI; ++i) a[i] = As[kk * kPA + 4 * i];
 #pragma unroll
                 for (int j = 0; j < 7; ++j) {
                     if (j < jn) {

@@ -20,7 +20,7 @@ constexpr int BN = dist::DT_N, TPB = dist::DT_TPB, MAXSIG = 32;
 
 // Few tiles leave an SM one warp per FP64 unit, which cannot keep it busy: 16-row
 // tiles up to one per SM, 32-row ones up to two 64-row tiles per SM. us on d = 276
-// with 16, 32 and 64 rows: 1 x 1000 19, 23, 68; 128 x 2000 34, 27, 50; 1000 x 1000
+// with 16, 32 and 64 rows: 1 x 1000 17, 23, 68; 128 x 2000 34, 26, 50; 1000 x 1000
 // symmetric 97, 39, 70; 1600 symmetric 222, 85, 84; 2000 x 2000 350, 216, 179.
 constexpr int kSmallTilesPerSm = 1, kHalfTilesPerSm = 2;
 
@@ -37,7 +37,8 @@ distance_kernel_f64(const double *__restrict__ A, int na, int lda, const double 
                     double *__restrict__ K, long long ldk, long long sstride, int symmetric) {
     // the stage and the transpose share one buffer
     constexpr int BM = 16 * RI, kT = BN * (BM + 1), kPerBlock = BN / BM;
-    __shared__ double smem[RI > 1 && kT > dist::DT_STAGE ? kT : dist::DT_STAGE];
+    constexpr int kStage = dist::stage_doubles<RI>();
+    __shared__ double smem[RI > 1 && kT > kStage ? kT : kStage];
     double(*T)[BM + 1] = reinterpret_cast<double(*)[BM + 1]>(smem);
 
     int by, bx, row0;

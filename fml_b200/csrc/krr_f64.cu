@@ -45,7 +45,7 @@ predict_partial_kernel(const double *__restrict__ Q, int nq, int ldq, const doub
                        const double *__restrict__ alpha, long long lda_alpha,
                        double *__restrict__ partial) {
     constexpr int BM = 16 * RI;
-    __shared__ double stage[dist::DT_STAGE];
+    __shared__ double stage[dist::stage_doubles<RI>()];
     __shared__ double red[MAXSIG][BM];
     const int row0 = blockIdx.x * BM, nr = min(BM, nq - row0);
     const int split = blockIdx.y;
@@ -98,7 +98,7 @@ predict_partial_kernel(const double *__restrict__ Q, int nq, int ldq, const doub
 
 // The partial sums of every chunk, in tiles of 16, 32 or 64 queries by the number
 // of CTAs that the largest would give. us for 16, 32, 64 queries, d = 276: 200 x 1000
-// 48, 56, 107; 500 x 1000 72, 74, 107; 1000 x 1000 118, 78, 115; 2000 x 1000 220, 139,
+// 44, 56, 107; 500 x 1000 66, 74, 107; 1000 x 1000 118, 78, 115; 2000 x 1000 220, 139,
 // 151; 1000 x 2000 220, 140, 130; 2000 x 2000 396, 257, 225.
 int launch_predict_partial(int kind, const double *Xq, int nq, int ldq, const double *Xt, int nt,
                            int ldt, int d, const Scales &sc, int nsigma, const double *alpha,

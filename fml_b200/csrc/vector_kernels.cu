@@ -84,10 +84,10 @@ __global__ void __launch_bounds__(VK_TPB, 4)
 vector_kernels_kernel(const VkSide s1, const VkSide s2, int d, const __grid_constant__ Coefs coef,
                       int nsig, double *__restrict__ K, int *__restrict__ status) {
     extern __shared__ double ksum[];  // [nsig][group1][group2]
-    __shared__ double stage[dist::DT_STAGE];  // of the features, then the distance tile
+    __shared__ double stage[dist::stage_doubles<4>()];  // of the features, then the distance tile
     __shared__ double part[VK_T][VK_MAX_GROUP + 1];
     __shared__ int seg1[VK_MAX_GROUP + 1], seg2[VK_MAX_GROUP + 1], row1[VK_ROWS], row2[VK_ROWS];
-    static_assert(VK_T * VK_P <= dist::DT_STAGE, "the tile fits");
+    static_assert(VK_T * VK_P <= dist::stage_doubles<4>(), "the tile fits");
     double(*D)[VK_P] = reinterpret_cast<double(*)[VK_P]>(stage);
     const int tid = threadIdx.x, warp = tid >> 5;
     const int nb2 = (s2.nm + s2.group - 1) / s2.group;
