@@ -734,7 +734,7 @@ arad_sort_records_kernel(SetWs w, const int *__restrict__ N, int nm, int amax,
 // Bound by the instructions issued: 38 for a step of 2 (128 evaluations, of which 14
 // packed FP32 and 4 exponentials, 8 cycles of their units each), about 45 to add a
 // lane's sums, 5000 per molecule pair outside of the steps. 500 x 3001 molecules of
-// at most 23 atoms, 5 sigmas: 30.3 ms; 39.7 with one J at a time, the ranges found
+// at most 23 atoms, 5 sigmas: 29.7 ms; 39.7 with one J at a time, the ranges found
 // by every warp for itself and the compare-and-swap loop, which took half of the
 // shared memory's cycles.
 constexpr int BD_JA = 96;     // atoms J at a time
