@@ -164,7 +164,13 @@ template <int KIND>
 int launch_vk(VkSide s1, VkSide s2, int d, const Coefs &coef, int nsig, double *K, int *status,
               cudaStream_t st) {
     vk_groups(s1, s2);
-    const size_t smem = sizeof(double) * (size_t)nsig * s1.group * s2.group;  // <= 16 KB
+    // at most 16 KB, but beside 40 KB of static shared memory: with many sigmas the two
+    // pass the 48 KB that a launch gets without the attribute
+    const size_t smem = sizeof(double) * (size_t)nsig * s1.group * s2.group;
+    FMLB_TRY(cuda_status(cudaFuncSetAttribute(vector_kernels_kernel<KIND>,
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)smem),
+                         "cudaFuncSetAttribute"));
     const long long blocks = (long long)ceil_div(s1.nm, s1.group) * ceil_div(s2.nm, s2.group);
     vector_kernels_kernel<KIND><<<(unsigned)blocks, VK_TPB, smem, st>>>(s1, s2, d, coef, nsig, K,
                                                                       status);
