@@ -39,24 +39,24 @@ __global__ void add_diagonal_kernel(double *A, long long lda, int n, double lam)
 // 16 RI queries x CHUNK training points per cluster. A query's sums are formed
 // in the same order whatever RI and the queries beside it are.
 template <bool kL1, int RI>
-__global__ void __cluster_dims__(1, 1, PARTS) __launch_bounds__(TPB, RI == 4 ? 4 : RI == 2 ? 6 : 8)
+__global__ void __cluster_dims__(1, 1, PARTS) __launch_bounds__(TPB, RI == 4 ? 4 : RI == 2 ? 6 : 5)
 predict_partial_kernel(const double *__restrict__ Q, int nq, int ldq, const double *__restrict__ T,
                        int nt, int ldt, int d, const __grid_constant__ Scales sc, int nsig,
                        const double *__restrict__ alpha, long long lda_alpha,
                        double *__restrict__ partial) {
     constexpr int BM = 16 * RI;
-    __shared__ double stage[dist::stage_doubles<RI>()];
+    __shared__ double stage[dist::stage_doubles<RI, 8>()];
     __shared__ double red[MAXSIG][BM];
     const int row0 = blockIdx.x * BM, nr = min(BM, nq - row0);
     const int split = blockIdx.y;
     const int t_begin = split * CHUNK + blockIdx.z * PART, t_end = min(nt, t_begin + PART);
-    const int r0 = dist::first_row<RI>(), c0 = dist::first_col();
+    const int r0 = dist::first_row<RI, 8>(), c0 = dist::first_col<8>();
     for (int t = threadIdx.x; t < nsig * BM; t += TPB) red[t / BM][t % BM] = 0.0;
     // (the first barrier inside dist_tile orders these before their use)
     for (int col0 = t_begin; col0 < t_end; col0 += BN) {
         const int nc = min(BN, t_end - col0);
         double acc[RI][8];
-        dist::dist_tile<kL1 ? dist::kAbs : dist::kSquare, RI>(
+        dist::dist_tile<kL1 ? dist::kAbs : dist::kSquare, true>(
             acc, stage, [&](int r) { return Q + (size_t)(row0 + r) * ldq; },
             [&](int c) { return T + (size_t)(col0 + c) * ldt; }, nr, nc, d);
         for (int s = 0; s < nsig; ++s) {

@@ -84,10 +84,10 @@ __global__ void __launch_bounds__(VK_TPB, 4)
 vector_kernels_kernel(const VkSide s1, const VkSide s2, int d, const __grid_constant__ Coefs coef,
                       int nsig, double *__restrict__ K, int *__restrict__ status) {
     extern __shared__ double ksum[];  // [nsig][group1][group2]
-    __shared__ double stage[dist::stage_doubles<4>()];  // of the features, then the distance tile
+    __shared__ double stage[dist::stage_doubles<4, 8>()];  // features, then the distance tile
     __shared__ double part[VK_T][VK_MAX_GROUP + 1];
     __shared__ int seg1[VK_MAX_GROUP + 1], seg2[VK_MAX_GROUP + 1], row1[VK_ROWS], row2[VK_ROWS];
-    static_assert(VK_T * VK_P <= dist::stage_doubles<4>(), "the tile fits");
+    static_assert(VK_T * VK_P <= dist::stage_doubles<4, 8>(), "the tile fits");
     double(*D)[VK_P] = reinterpret_cast<double(*)[VK_P]>(stage);
     const int tid = threadIdx.x, warp = tid >> 5;
     const int nb2 = (s2.nm + s2.group - 1) / s2.group;
@@ -98,13 +98,13 @@ vector_kernels_kernel(const VkSide s1, const VkSide s2, int d, const __grid_cons
     for (int t = tid; t < nsig * g12; t += VK_TPB) ksum[t] = 0.0;
     __syncthreads();
     const int R1 = seg1[s1.group], R2 = seg2[s2.group];
-    const int tr = dist::first_row<4>(), tc = dist::first_col();
+    const int tr = dist::first_row<4, 8>(), tc = dist::first_col<8>();
 
     for (int r0 = 0; r0 < R1; r0 += VK_T) {
         for (int c0 = 0; c0 < R2; c0 += VK_T) {
             const int nr = min(VK_T, R1 - r0), nc = min(VK_T, R2 - c0);
             double acc[4][8];
-            dist::dist_tile<KIND == 0 ? dist::kSquareUnfused : dist::kAbs, 4>(
+            dist::dist_tile<KIND == 0 ? dist::kSquareUnfused : dist::kAbs, true>(
                 acc, stage, [&](int r) { return s1.X + (size_t)row1[r0 + r] * d; },
                 [&](int c) { return s2.X + (size_t)row2[c0 + c] * d; }, nr, nc, d);
             __syncthreads();  // the stage becomes the distance tile
