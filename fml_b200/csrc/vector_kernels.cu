@@ -146,7 +146,10 @@ vector_kernels_kernel(const VkSide s1, const VkSide s2, int d, const __grid_cons
 
 // Molecules per group: about 80 atoms at the usual fill of a padded row (the
 // tile's unused rows and columns then cost a sixth), fewer while the blocks
-// would not fill the GPU a few times over.
+// would not fill the GPU a few times over. Two blocks per SM are enough where a
+// block is one tile: smaller ones leave more of it empty. us for groups of 1 x 1, 2 x 1
+// and 2 x 2 of 23 atoms, d = 276, one sigma: 30 x 30 molecules 73, 62, -; 40 x 40 105, 95,
+// 76; 60 x 60 (2 x 1, 2 x 2) 159, 122; 74, 113 and 215 us with a CTA per molecule pair.
 void vk_groups(VkSide &s1, VkSide &s2) {
     auto most = [](const VkSide &s) { return std::max(1, std::min(VK_MAX_GROUP, VK_ROWS / s.amax)); };
     s1.group = most(s1);
@@ -154,7 +157,8 @@ void vk_groups(VkSide &s1, VkSide &s2) {
     auto blocks = [&] {
         return (long long)ceil_div(s1.nm, s1.group) * ceil_div(s2.nm, s2.group);
     };
-    while (blocks() < 8LL * sm_count() && (s1.group > 1 || s2.group > 1)) {
+    auto one_tile = [&] { return s1.group * s1.amax <= VK_T && s2.group * s2.amax <= VK_T; };
+    while (blocks() < (one_tile() ? 2LL : 8LL) * sm_count() && (s1.group > 1 || s2.group > 1)) {
         int &g = s1.group >= s2.group ? s1.group : s2.group;
         g = (g + 1) / 2;
     }
