@@ -52,13 +52,15 @@ struct VkSide {
 
 // Atom list of molecules [m0, m0 + group): seg[q] = first list entry of
 // molecule m0 + q, row[] = its rows in X. One whole warp.
-__device__ __forceinline__ void vk_list(const VkSide &s, int m0, int *seg, int *row, int *status) {
+__device__ __forceinline__ void vk_list(const VkSide &s, int m0, int *seg, long long *row,
+                                        int *status) {
     const int lane = threadIdx.x & 31;
-    int n = 0, first = 0;
+    int n = 0;
+    long long first = 0;
     if (lane < s.group && m0 + lane < s.nm) {
         const int m = m0 + lane;
         n = s.O ? s.O[m + 1] - s.O[m] : s.N[m];
-        first = s.O ? s.O[m] : m * s.amax;
+        first = s.O ? s.O[m] : (long long)m * s.amax;
         if (n < 0 || n > s.amax) {  // rejected on the host as well
             if (status) atomicCAS(status, 0, 1);
             n = min(max(n, 0), s.amax);
@@ -71,7 +73,8 @@ __device__ __forceinline__ void vk_list(const VkSide &s, int m0, int *seg, int *
     }
     if (lane <= s.group) seg[lane] = incl - n;
     for (int q = 0; q < s.group; ++q) {
-        const int nq = __shfl_sync(0xffffffffu, n, q), f = __shfl_sync(0xffffffffu, first, q);
+        const int nq = __shfl_sync(0xffffffffu, n, q);
+        const long long f = __shfl_sync(0xffffffffu, first, q);
         const int at = __shfl_sync(0xffffffffu, incl - n, q);
         for (int a = lane; a < nq; a += 32) row[at + a] = f + a;
     }
@@ -86,11 +89,12 @@ vector_kernels_kernel(const VkSide s1, const VkSide s2, int d, const __grid_cons
     extern __shared__ double ksum[];  // [nsig][group1][group2]
     __shared__ double stage[dist::stage_doubles<4, 8>()];  // features, then the distance tile
     __shared__ double part[VK_T][VK_MAX_GROUP + 1];
-    __shared__ int seg1[VK_MAX_GROUP + 1], seg2[VK_MAX_GROUP + 1], row1[VK_ROWS], row2[VK_ROWS];
+    __shared__ int seg1[VK_MAX_GROUP + 1], seg2[VK_MAX_GROUP + 1];
+    __shared__ long long row1[VK_ROWS], row2[VK_ROWS];  // 2^24 molecules x 128 atoms pass 32 bits
     static_assert(VK_T * VK_P <= dist::stage_doubles<4, 8>(), "the tile fits");
     double(*D)[VK_P] = reinterpret_cast<double(*)[VK_P]>(stage);
     const int tid = threadIdx.x, warp = tid >> 5;
-    const int nb2 = (s2.nm + s2.group - 1) / s2.group;
+    const int nb2 = (s2.nm - 1) / s2.group + 1;
     const int m1 = (int)(blockIdx.x / nb2) * s1.group, m2 = (int)(blockIdx.x % nb2) * s2.group;
     const int g12 = s1.group * s2.group;
     if (warp == 0) vk_list(s1, m1, seg1, row1, status);
@@ -105,8 +109,8 @@ vector_kernels_kernel(const VkSide s1, const VkSide s2, int d, const __grid_cons
             const int nr = min(VK_T, R1 - r0), nc = min(VK_T, R2 - c0);
             double acc[4][8];
             dist::dist_tile<KIND == 0 ? dist::kSquareUnfused : dist::kAbs, true>(
-                acc, stage, [&](int r) { return s1.X + (size_t)row1[r0 + r] * d; },
-                [&](int c) { return s2.X + (size_t)row2[c0 + c] * d; }, nr, nc, d);
+                acc, stage, [&](int r) { return s1.X + row1[r0 + r] * d; },
+                [&](int c) { return s2.X + row2[c0 + c] * d; }, nr, nc, d);
             __syncthreads();  // the stage becomes the distance tile
 #pragma unroll
             for (int i = 0; i < 4; ++i)
@@ -168,7 +172,7 @@ template <int KIND>
 int launch_vk(VkSide s1, VkSide s2, int d, const Coefs &coef, int nsig, double *K, int *status,
               cudaStream_t st) {
     vk_groups(s1, s2);
-    // at most 16 KB, but beside 40 KB of static shared memory: with many sigmas the two
+    // at most 16 KB, but beside 41 KB of static shared memory: with many sigmas the two
     // pass the 48 KB that a launch gets without the attribute
     const size_t smem = sizeof(double) * (size_t)nsig * s1.group * s2.group;
     FMLB_TRY(cuda_status(cudaFuncSetAttribute(vector_kernels_kernel<KIND>,
