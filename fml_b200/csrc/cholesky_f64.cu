@@ -26,6 +26,7 @@
 
 #include "common.cuh"
 #include "ozaki.cuh"
+#include "tc_common.cuh"
 
 namespace fmlb {
 namespace {
@@ -851,10 +852,11 @@ __device__ __forceinline__ void solve_publish(double *p, double v) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(u) : "memory");
 }
 
-// This CTA's place in the order (the counter starts at 0xffffffff).
-__device__ __forceinline__ int solve_ticket(unsigned *counter) {
-    __shared__ int place;
-    if (threadIdx.x == 0) place = (int)(atomicAdd(counter, 1u) + 1u);
+// This CTA's place in the order (the counter starts at 0xffffffff). Past the last
+// block, when solves that share a workspace overlap: the CTA has nothing to do.
+__device__ __forceinline__ unsigned solve_ticket(unsigned *counter) {
+    __shared__ unsigned place;
+    if (threadIdx.x == 0) place = atomicAdd(counter, 1u) + 1u;
     __syncthreads();
     return place;
 }
@@ -902,7 +904,9 @@ solve_forward_kernel(const double *__restrict__ L, long long lda, int n,
                      double *y, unsigned *counter) {
     extern __shared__ __align__(16) double sv_smem[];
     double *Li = sv_smem, *v = Li + NB * NB, *yb = v + NB;  // yb: two blocks
-    const int k = solve_ticket(counter), k0 = k * NB, kn = min(NB, n - k0);
+    const unsigned place = solve_ticket(counter);
+    if (place >= (unsigned)(n + NB - 1) / NB) return;
+    const int k = (int)place, k0 = k * NB, kn = min(NB, n - k0);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     solve_load_inverse(Li, Linv + (size_t)k * NB * NB);
     const double *rows = L + (size_t)k0 * lda;
@@ -961,7 +965,9 @@ solve_backward_kernel(const double *__restrict__ L, long long lda, int n,
     extern __shared__ __align__(16) double sv_smem[];
     double *Li = sv_smem, *v = Li + NB * NB, *xb = v + NB, *part = xb + 2 * NB;
     const int nblk = (n + NB - 1) / NB;
-    const int k = nblk - 1 - solve_ticket(counter), k0 = k * NB, kn = min(NB, n - k0);
+    const unsigned place = solve_ticket(counter);
+    if (place >= (unsigned)nblk) return;
+    const int k = nblk - 1 - (int)place, k0 = k * NB, kn = min(NB, n - k0);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     solve_load_inverse(Li, Linv + (size_t)k * NB * NB);
     double lv[SV_ROWS][NB / 32], acc[2][NB / 32];
@@ -1416,12 +1422,12 @@ extern "C" int fmlb_potrs_f64(const double *L, long long lda, int n, const void 
     unsigned *counters = reinterpret_cast<unsigned *>(y + n);
     FMLB_TRY(cuda_status(cudaMemsetAsync(y, 0xff, (size_t)n * sizeof(double) + kSolveCounterBytes,
                                          st), "fmlb_potrs_f64: fill"));
-    solve_forward_kernel<<<(unsigned)nblk, TPB, kSolveSmem, st>>>(L, lda, n, Linv, x, y, counters);
+    const unsigned grid = (unsigned)nblk + (tc::test_hooks().extra_block ? 1 : 0);
+    solve_forward_kernel<<<grid, TPB, kSolveSmem, st>>>(L, lda, n, Linv, x, y, counters);
     FMLB_TRY(launch_status("solve_forward_kernel"));
     FMLB_TRY(cuda_status(cudaMemsetAsync(x, 0xff, (size_t)n * sizeof(double), st),
                          "fmlb_potrs_f64: fill"));
-    solve_backward_kernel<<<(unsigned)nblk, TPB, kSolveSmem, st>>>(L, lda, n, Linv, y, x,
-                                                                  counters + 1);
+    solve_backward_kernel<<<grid, TPB, kSolveSmem, st>>>(L, lda, n, Linv, y, x, counters + 1);
     return launch_status("solve_backward_kernel");
 }
 

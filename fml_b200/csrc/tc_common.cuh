@@ -149,10 +149,11 @@ __device__ __forceinline__ uint32_t after_ld_wait(uint32_t v) {
 // Test hooks of the tensor-core kernels, per host thread (fmlb_tc_test_hooks):
 // the clock-cycle budget of every mbarrier wait and a switch that makes the
 // TMA producer issue no copies, so that the consumers' waits run out with no
-// copy in flight.
+// copy in flight. extra_block: the triangular solves launch a CTA too many.
 struct TestHooks {
     long long wait_budget;
     int skip_loads;
+    int extra_block;
 };
 TestHooks test_hooks();
 
