@@ -833,17 +833,20 @@ constexpr int SV_WARPS = TPB / 32, SV_ROWS = NB / SV_WARPS;  // 8 warps of 16 ro
 constexpr size_t kSolveSmem = ((size_t)NB * NB + (size_t)SV_WARPS * NB + 3 * NB) * sizeof(double);
 constexpr size_t kSolveCounterBytes = 2 * sizeof(unsigned);  // behind y in the workspace
 constexpr unsigned long long kSolveUnset = ~0ull;   // what a byte-wise fill with 0xff leaves
-constexpr long long kSolveBudget = 4000000000LL;    // clock cycles of a wait (~2 s)
 
-// The value at p once it is set; NaN when the wait runs out (the solution then
-// holds NaN from there on).
-__device__ __forceinline__ double solve_wait(const double *p) {
+// The value at p once it is set; NaN when the wait takes more than `budget` clock
+// cycles (the solution then holds NaN from there on), after which the thread's other
+// waits don't wait any more.
+__device__ __forceinline__ double solve_wait(const double *p, long long &budget) {
     const long long t0 = clock64();
     for (;;) {
         unsigned long long u;
         asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(u) : "l"(p) : "memory");
         if (u != kSolveUnset) return __longlong_as_double((long long)u);
-        if (clock64() - t0 > kSolveBudget) return __longlong_as_double(0x7ff8000000000000LL);
+        if (clock64() - t0 > budget) {
+            budget = -1;
+            return __longlong_as_double(0x7ff8000000000000LL);
+        }
     }
 }
 __device__ __forceinline__ void solve_publish(double *p, double v) {
@@ -901,7 +904,7 @@ __device__ __forceinline__ double warp_sums16(double (&a)[SV_ROWS]) {
 __global__ void __launch_bounds__(TPB, 1)
 solve_forward_kernel(const double *__restrict__ L, long long lda, int n,
                      const double *__restrict__ Linv, const double *__restrict__ b,
-                     double *y, unsigned *counter) {
+                     double *y, unsigned *counter, long long budget, int withhold) {
     extern __shared__ __align__(16) double sv_smem[];
     double *Li = sv_smem, *v = Li + NB * NB, *yb = v + NB;  // yb: two blocks
     const unsigned place = solve_ticket(counter);
@@ -916,7 +919,7 @@ solve_forward_kernel(const double *__restrict__ L, long long lda, int n,
     if (k > 0) solve_load_rows(lv, rows, lda, kn, NB);
     for (int j = 0; j < k; ++j) {
         double *yj = yb + (j & 1) * NB;
-        if (tid < NB) yj[tid] = solve_wait(y + j * NB + tid);
+        if (tid < NB) yj[tid] = solve_wait(y + j * NB + tid, budget);
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < NB / 32; ++i) {
@@ -941,7 +944,7 @@ solve_forward_kernel(const double *__restrict__ L, long long lda, int n,
         acc[r] = p;
     }
     s = warp_sums16(acc);
-    if ((lane & 1) == 0 && row < kn) solve_publish(y + k0 + row, s);
+    if ((lane & 1) == 0 && row < kn && !(withhold && k == 0)) solve_publish(y + k0 + row, s);
 }
 
 // Columns of the warps' partial sums p[i] (columns lane + 32 i), added in warp
@@ -961,7 +964,7 @@ __device__ __forceinline__ double solve_column_sums(double *part, const double (
 __global__ void __launch_bounds__(TPB, 1)
 solve_backward_kernel(const double *__restrict__ L, long long lda, int n,
                       const double *__restrict__ Linv, const double *__restrict__ y, double *x,
-                      unsigned *counter) {
+                      unsigned *counter, long long budget, int withhold) {
     extern __shared__ __align__(16) double sv_smem[];
     double *Li = sv_smem, *v = Li + NB * NB, *xb = v + NB, *part = xb + 2 * NB;
     const int nblk = (n + NB - 1) / NB;
@@ -977,7 +980,7 @@ solve_backward_kernel(const double *__restrict__ L, long long lda, int n,
         solve_load_rows(lv, L + (size_t)(nblk - 1) * NB * lda + k0, lda, n - (nblk - 1) * NB, NB);
     for (int j = nblk - 1; j > k; --j) {
         double *xj = xb + (j & 1) * NB;
-        if (tid < NB) xj[tid] = j * NB + tid < n ? solve_wait(x + j * NB + tid) : 0.0;
+        if (tid < NB) xj[tid] = j * NB + tid < n ? solve_wait(x + j * NB + tid, budget) : 0.0;
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < SV_ROWS; ++r) {
@@ -1006,7 +1009,7 @@ solve_backward_kernel(const double *__restrict__ L, long long lda, int n,
 #pragma unroll
     for (int i = 0; i < NB / 32; ++i) p[i] = acc[0][i] + acc[1][i];
     s = solve_column_sums(part, p);
-    if (tid < kn) solve_publish(x + k0 + tid, s);
+    if (tid < kn && !(withhold && k == nblk - 1)) solve_publish(x + k0 + tid, s);
 }
 
 // ---- 5. inverse from the factor (potri) ------------------------------------
@@ -1422,12 +1425,15 @@ extern "C" int fmlb_potrs_f64(const double *L, long long lda, int n, const void 
     unsigned *counters = reinterpret_cast<unsigned *>(y + n);
     FMLB_TRY(cuda_status(cudaMemsetAsync(y, 0xff, (size_t)n * sizeof(double) + kSolveCounterBytes,
                                          st), "fmlb_potrs_f64: fill"));
-    const unsigned grid = (unsigned)nblk + (tc::test_hooks().extra_block ? 1 : 0);
-    solve_forward_kernel<<<grid, TPB, kSolveSmem, st>>>(L, lda, n, Linv, x, y, counters);
+    const tc::TestHooks hooks = tc::test_hooks();
+    const unsigned grid = (unsigned)nblk + (hooks.extra_block ? 1 : 0);
+    solve_forward_kernel<<<grid, TPB, kSolveSmem, st>>>(L, lda, n, Linv, x, y, counters,
+                                                        hooks.wait_budget, hooks.withhold);
     FMLB_TRY(launch_status("solve_forward_kernel"));
     FMLB_TRY(cuda_status(cudaMemsetAsync(x, 0xff, (size_t)n * sizeof(double), st),
                          "fmlb_potrs_f64: fill"));
-    solve_backward_kernel<<<grid, TPB, kSolveSmem, st>>>(L, lda, n, Linv, y, x, counters + 1);
+    solve_backward_kernel<<<grid, TPB, kSolveSmem, st>>>(L, lda, n, Linv, y, x, counters + 1,
+                                                         hooks.wait_budget, hooks.withhold);
     return launch_status("solve_backward_kernel");
 }
 

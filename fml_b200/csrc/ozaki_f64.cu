@@ -616,7 +616,7 @@ size_t oz_smem_bytes(int ns) {
            OZ_BAR_BYTES + OZ_ALIGN;
 }
 
-thread_local tc::TestHooks t_hooks = {0, 0, 0};
+thread_local tc::TestHooks t_hooks = {0, 0, 0, 0};
 
 template <int NS>
 int launch_oz(const OzMaps &maps, const OzakiSlices &s, const OzParams &p, double *C, int *info,
@@ -765,5 +765,6 @@ extern "C" int fmlb_tc_test_hooks(long long wait_cycles, int skip_loads) {
     t_hooks.wait_budget = wait_cycles;
     t_hooks.skip_loads = skip_loads ? 1 : 0;
     t_hooks.extra_block = (skip_loads & 2) != 0;
+    t_hooks.withhold = (skip_loads & 4) != 0;
     return FMLB_OK;
 }

@@ -149,11 +149,13 @@ __device__ __forceinline__ uint32_t after_ld_wait(uint32_t v) {
 // Test hooks of the tensor-core kernels, per host thread (fmlb_tc_test_hooks):
 // the clock-cycle budget of every mbarrier wait and a switch that makes the
 // TMA producer issue no copies, so that the consumers' waits run out with no
-// copy in flight. extra_block: the triangular solves launch a CTA too many.
+// copy in flight. In the triangular solves, whose waits take the same budget:
+// withhold, the first block's values are not published; extra_block, a CTA too many.
 struct TestHooks {
     long long wait_budget;
     int skip_loads;
     int extra_block;
+    int withhold;
 };
 TestHooks test_hooks();
 

@@ -297,7 +297,9 @@ int fmlb_distance_matrix_f64(int kind, const double *A, int na, int lda, const d
  * fmlb_potrs_f64 solves A x = b in place in x (n,) given the factor and work. It
  * keeps an intermediate vector and two counters in work, so one solve at a time may
  * use a workspace: solves that overlap on the GPU need one each (their results are
- * undefined otherwise; no access leaves the buffers).
+ * undefined otherwise; no access leaves the buffers). Its thread blocks wait for one
+ * another's values, about 2 s at most: a wait that runs out leaves NaN in x from there
+ * on, which is the only sign of it (there is no info argument).
  * ---------------------------------------------------------------------- */
 size_t fmlb_potrf_workspace_bytes(int n);
 int fmlb_potrf_f64(double *A, long long lda, int n, void *work, int *info, void *stream);
@@ -360,13 +362,14 @@ int fmlb_syrk_lower_ozaki(double *C, long long ldc, int m, const double *P, long
                           void *stream);
 
 /* Test hooks of the tensor-core kernels (fmlb_gaussian_kernel_tc,
- * fmlb_syrk_lower_ozaki, fmlb_potrf_ozaki_f64) for later launches from the
- * calling host thread: wait_cycles > 0 sets the clock-cycle limit of every
- * device-side mbarrier wait (0 restores the default, about 2 s); skip_loads
+ * fmlb_syrk_lower_ozaki, fmlb_potrf_ozaki_f64) and of fmlb_potrs_f64 for later
+ * launches from the calling host thread: wait_cycles > 0 sets the clock-cycle limit
+ * of every device-side wait (0 restores the default, about 2 s); skip_loads
  * != 0 makes the TMA producer issue no copies, so the waits run out with
  * nothing in flight and the kernel reports FMLB_ETIMEDOUT. skip_loads & 2 also
  * makes fmlb_potrs_f64 launch one thread block more than it has work for (what a
- * solve meets when another one overlaps on its workspace). No reference
+ * solve meets when another one overlaps on its workspace), skip_loads & 4 keeps
+ * its first block's values from the others, so that their waits run out. No reference
  * counterpart (failure-path testing). */
 int fmlb_tc_test_hooks(long long wait_cycles, int skip_loads);
 
