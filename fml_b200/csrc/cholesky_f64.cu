@@ -230,8 +230,9 @@ __device__ __forceinline__ void put_subblock(double (*L)[LDL], double *__restric
 #pragma unroll 4
     for (int r = part; r < SB; r += parts) {
         const double piv = pivs[r], inv = invs[r], root = piv * inv;
-        const double v = lane == r ? fma(0.5 * inv, fma(-root, root, piv), root)
-                                   : cols[lane * SB + ((r - lane) & 31)];
+        // an infinite pivot (its reciprocal root is zero) is its own root
+        const double diag = inv > 0.0 ? fma(0.5 * inv, fma(-root, root, piv), root) : piv;
+        const double v = lane == r ? diag : cols[lane * SB + ((r - lane) & 31)];
         if (lane <= r) L[b0 + r][b0 + lane] = v;
         Linv[(size_t)(b0 + r) * NB + b0 + lane] = W[r * LDW + lane];
     }
