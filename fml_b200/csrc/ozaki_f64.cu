@@ -77,7 +77,8 @@ constexpr int OZ_MAX_STAGES = 8;  // the ring depth is set per launch from share
 constexpr int OZ_THREADS = 384;    // 3 warpgroups: producer and MMA issuer, two of epilogue
 // Registers a thread. The block starts with 168 each (65536 / 384, as the
 // compiler grants them); the first warpgroup gives back what the epilogue takes,
-// which keeps 64 drained columns in registers. The host checks the start.
+// which keeps 64 drained columns in registers. The host checks the start, and runs
+// the form that moves none where the compiler granted another number.
 constexpr int OZ_REGS = 168, OZ_REGS_LOAD = 40, OZ_REGS_EPI = 232;
 static_assert(OZ_REGS_LOAD + 2 * OZ_REGS_EPI <= 3 * OZ_REGS, "the registers of the block");
 constexpr int OZ_EPI_WARPS = 8;
@@ -223,7 +224,7 @@ __device__ __forceinline__ void oz_issue(uint32_t tmem, uint64_t da, uint64_t db
     }
 }
 
-template <int NS>
+template <int NS, bool kMoveRegs>
 __global__ void __launch_bounds__(OZ_THREADS, 1)
 ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
                   const int *__restrict__ exps, const double *__restrict__ rsum, OzParams p,
@@ -266,7 +267,8 @@ ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
 
     // each warpgroup sets its registers inside its own branch: where the two meet
     // the compiler can count on the smaller number only
-    if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(OZ_REGS_LOAD));
+    if (kMoveRegs && warp < 4)
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(OZ_REGS_LOAD));
     if (warp == 0) {
         // ------------------------------------------------------------ producer
         if (lane == 0) {
@@ -344,7 +346,7 @@ ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
             if (!tc::mbar_wait(mma_done, 0, budget)) oz_fail(info);
         }
     } else if (warp >= 4) {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(OZ_REGS_EPI));
+        if (kMoveRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(OZ_REGS_EPI));
         // --------------------------------------------------------------- epilogue
         // Two warps per TMEM lane quarter, 64 columns each. The tensor cores wait
         // from a pass's last MMA until its accumulators are drained, so that comes
@@ -616,30 +618,41 @@ size_t oz_smem_bytes(int ns) {
            OZ_BAR_BYTES + OZ_ALIGN;
 }
 
-thread_local tc::TestHooks t_hooks = {0, 0, 0, 0};
+thread_local tc::TestHooks t_hooks = {0, 0, 0, 0, 0};
 
+// `move`: as built, the kernel can move registers between its warpgroups. That takes
+// a start with OZ_REGS each (setmaxnreg.inc would wait for registers it cannot get), which
+// depends on the compiler; otherwise the form without it runs (m = 16384, k = 1024, s = 6,
+// with the split: 3.17 ms and 3.94).
 template <int NS>
 int launch_oz(const OzMaps &maps, const OzakiSlices &s, const OzParams &p, double *C, int *info,
-              int grid, size_t smem, long long budget, cudaStream_t st) {
+              int grid, size_t smem, const tc::TestHooks &hooks, cudaStream_t st) {
     static_assert(NS <= OZAKI_MAX_SLICES, "digit planes");
     static int attr_dev = -1;
+    static bool move = false;
     int dev = 0;
     FMLB_TRY(cuda_status(cudaGetDevice(&dev), "ozaki: cudaGetDevice"));
     if (attr_dev != dev) {
-        FMLB_TRY(cuda_status(cudaFuncSetAttribute(ozaki_syrk_kernel<NS>,
+        FMLB_TRY(cuda_status(cudaFuncSetAttribute(ozaki_syrk_kernel<NS, true>,
+                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  OZ_SMEM_LIMIT),
+                             "ozaki: smem attribute"));
+        FMLB_TRY(cuda_status(cudaFuncSetAttribute(ozaki_syrk_kernel<NS, false>,
                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   OZ_SMEM_LIMIT),
                              "ozaki: smem attribute"));
         cudaFuncAttributes fa;
-        FMLB_TRY(cuda_status(cudaFuncGetAttributes(&fa, ozaki_syrk_kernel<NS>),
+        FMLB_TRY(cuda_status(cudaFuncGetAttributes(&fa, ozaki_syrk_kernel<NS, true>),
                              "ozaki: kernel attributes"));
-        if (fa.numRegs != OZ_REGS) {  // setmaxnreg.inc would wait for registers it cannot get
-            set_error("ozaki: built with %d registers a thread instead of %d", fa.numRegs, OZ_REGS);
-            return FMLB_ENOTSUP;
-        }
+        move = fa.numRegs == OZ_REGS;
         attr_dev = dev;
     }
-    ozaki_syrk_kernel<NS><<<grid, OZ_THREADS, smem, st>>>(maps, s.exps, s.rsum, p, C, info, budget);
+    if (move && !hooks.fixed_regs)
+        ozaki_syrk_kernel<NS, true><<<grid, OZ_THREADS, smem, st>>>(maps, s.exps, s.rsum, p, C, info,
+                                                                    hooks.wait_budget);
+    else
+        ozaki_syrk_kernel<NS, false><<<grid, OZ_THREADS, smem, st>>>(maps, s.exps, s.rsum, p, C,
+                                                                     info, hooks.wait_budget);
     return launch_status("ozaki_syrk_kernel");
 }
 
@@ -699,14 +712,14 @@ int ozaki_syrk(double *C, long long ldc, int m, const OzakiSlices &s, int p_row0
     const int grid = (int)std::min<long long>(
         p.ntiles, std::max<long long>(sm_count(), (p.ntiles + 3) / 4));
     switch (s.ns) {
-        case 1: return launch_oz<1>(maps, s, p, C, info, grid, smem, hooks.wait_budget, st);
-        case 2: return launch_oz<2>(maps, s, p, C, info, grid, smem, hooks.wait_budget, st);
-        case 3: return launch_oz<3>(maps, s, p, C, info, grid, smem, hooks.wait_budget, st);
-        case 4: return launch_oz<4>(maps, s, p, C, info, grid, smem, hooks.wait_budget, st);
-        case 5: return launch_oz<5>(maps, s, p, C, info, grid, smem, hooks.wait_budget, st);
-        case 6: return launch_oz<6>(maps, s, p, C, info, grid, smem, hooks.wait_budget, st);
-        case 7: return launch_oz<7>(maps, s, p, C, info, grid, smem, hooks.wait_budget, st);
-        default: return launch_oz<8>(maps, s, p, C, info, grid, smem, hooks.wait_budget, st);
+        case 1: return launch_oz<1>(maps, s, p, C, info, grid, smem, hooks, st);
+        case 2: return launch_oz<2>(maps, s, p, C, info, grid, smem, hooks, st);
+        case 3: return launch_oz<3>(maps, s, p, C, info, grid, smem, hooks, st);
+        case 4: return launch_oz<4>(maps, s, p, C, info, grid, smem, hooks, st);
+        case 5: return launch_oz<5>(maps, s, p, C, info, grid, smem, hooks, st);
+        case 6: return launch_oz<6>(maps, s, p, C, info, grid, smem, hooks, st);
+        case 7: return launch_oz<7>(maps, s, p, C, info, grid, smem, hooks, st);
+        default: return launch_oz<8>(maps, s, p, C, info, grid, smem, hooks, st);
     }
 }
 
@@ -763,8 +776,9 @@ extern "C" int fmlb_tc_test_hooks(long long wait_cycles, int skip_loads) {
     using namespace fmlb;
     FMLB_REQUIRE(wait_cycles >= 0, "fmlb_tc_test_hooks: negative wait budget");
     t_hooks.wait_budget = wait_cycles;
-    t_hooks.skip_loads = skip_loads ? 1 : 0;
+    t_hooks.skip_loads = skip_loads != 0 && skip_loads != 8;
     t_hooks.extra_block = (skip_loads & 2) != 0;
     t_hooks.withhold = (skip_loads & 4) != 0;
+    t_hooks.fixed_regs = (skip_loads & 8) != 0;
     return FMLB_OK;
 }

@@ -156,6 +156,7 @@ struct TestHooks {
     int skip_loads;
     int extra_block;
     int withhold;
+    int fixed_regs;  // the int8 update in its form that moves no registers
 };
 TestHooks test_hooks();
 

@@ -361,16 +361,19 @@ int fmlb_syrk_lower_ozaki(double *C, long long ldc, int m, const double *P, long
                           int strip_cols, int nslices, void *work, size_t ws_bytes, int *info,
                           void *stream);
 
-/* Test hooks of the tensor-core kernels (fmlb_gaussian_kernel_tc,
- * fmlb_syrk_lower_ozaki, fmlb_potrf_ozaki_f64) and of fmlb_potrs_f64 for later
- * launches from the calling host thread: wait_cycles > 0 sets the clock-cycle limit
- * of every device-side wait (0 restores the default, about 2 s); skip_loads
- * != 0 makes the TMA producer issue no copies, so the waits run out with
- * nothing in flight and the kernel reports FMLB_ETIMEDOUT. skip_loads & 2 also
- * makes fmlb_potrs_f64 launch one thread block more than it has work for (what a
- * solve meets when another one overlaps on its workspace), skip_loads & 4 keeps
- * its first block's values from the others, so that their waits run out. No reference
- * counterpart (failure-path testing). */
+/* Test hooks for later launches from the calling host thread, of the tensor-core
+ * kernels (fmlb_gaussian_kernel_tc, fmlb_syrk_lower_ozaki, fmlb_potrf_ozaki_f64) and
+ * of fmlb_potrs_f64. wait_cycles > 0 sets the clock-cycle limit of every
+ * device-side wait (0 restores the default, about 2 s). skip_loads: 0 for none, or
+ *   1  the TMA producer issues no copies, so the waits run out with nothing in
+ *      flight and the kernel reports FMLB_ETIMEDOUT; 2 and 4 do this too;
+ *   2  fmlb_potrs_f64 launches one thread block more than it has work for (what a
+ *      solve meets when another one overlaps on its workspace);
+ *   4  fmlb_potrs_f64 keeps its first block's values from the others, so that
+ *      their waits run out;
+ *   8  the int8 update runs in the form for a build whose registers cannot be
+ *      moved between its warps.
+ * No reference counterpart (failure-path testing). */
 int fmlb_tc_test_hooks(long long wait_cycles, int skip_loads);
 
 /* Double-double iterative refinement after an in-place factorisation of
