@@ -1195,6 +1195,7 @@ arad_fast_pair_kernel(SetWs w1, const int *__restrict__ N1, int nm1, SetWs w2,
 // slots. One J at a time and 256 threads left half of the warps waiting for the
 // one with the longest pairs.
 constexpr int F6_TPB = 512;
+constexpr int F6_ROWS = 65535;  // molecules I of a launch (the grid's limit in y)
 constexpr int F6_AP = 1024;    // atom pairs at a time (a pair of the largest molecules)
 constexpr int F6_WIN = 12288;  // runs at a time (24 KB): the atoms j1 go in chunks above that
 constexpr int F6_JA = 128, F6_JM = 16;  // atoms and molecules J at a time
@@ -1402,18 +1403,17 @@ __device__ __forceinline__ double f64_pair_sum(const F64View &v, int i1, int j1,
     return sum;
 }
 
-// Molecule I = blockIdx / nbj against the bj molecules J of block blockIdx % nbj.
+// Molecule I = I0 + blockIdx.y against the bj molecules J of block blockIdx.x.
 __global__ void __launch_bounds__(F6_TPB, 2)
 arad_f64_pair_kernel(const double *__restrict__ X1, SetWs w1, const int *__restrict__ N1, int nm1,
                      const double *__restrict__ X2, SetWs w2, const int *__restrict__ N2, int nm2,
                      int amax, AradParams P, const ClassInfo *ci,
                      const __grid_constant__ SigmaTable sig, int nsig, int symmetric, int bj,
-                     double *__restrict__ K) {
+                     int I0, double *__restrict__ K) {
     extern __shared__ __align__(16) unsigned char fc_smem_raw[];
     if (ci->flag) return;
-    const int nbj = (nm2 + bj - 1) / bj;
-    const int I = (int)(blockIdx.x / nbj), jb = (int)(blockIdx.x % nbj);
-    const int jend = min(nm2, (jb + 1) * bj);
+    const int I = I0 + (int)blockIdx.y, jb = (int)blockIdx.x;
+    const int jend = min(nm2 - jb * bj, bj) + jb * bj;
     if (symmetric && jend <= I) return;  // below the diagonal
     const F64View v = f64_view(fc_smem_raw, amax);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1847,11 +1847,14 @@ static int arad_kernels_impl(const double *X1, const double *Z1, const int *N1, 
         if (precision == 0) {
             if (try_fast) {
                 const int bj = f64_block(npairs);
-                const long long nblk = (long long)nm1 * ceil_div(nm2, bj);
-                FMLB_REQUIRE(nblk < (1LL << 31), "fmlb_arad_kernels: too many molecule blocks");
-                arad_f64_pair_kernel<<<(unsigned)nblk, F6_TPB, f64_smem_bytes(amax), st>>>(
-                    X1, w1, N1, nm1, X2, w2, N2, nm2, amax, P, ci, sig, ns, symmetric, bj, Ks);
-                FMLB_TRY(launch_status("arad_f64_pair_kernel"));
+                for (int I0 = 0; I0 < nm1; I0 += F6_ROWS) {
+                    const dim3 grid(ceil_div(nm2, bj), std::min(F6_ROWS, nm1 - I0));
+                    arad_f64_pair_kernel<<<grid, F6_TPB, f64_smem_bytes(amax), st>>>(
+                        X1, w1, N1, nm1, X2, w2, N2, nm2, amax, P, ci, sig, ns, symmetric, bj, I0,
+                        Ks);
+                    FMLB_TRY(launch_status("arad_f64_pair_kernel"));
+                    if (nm1 - I0 <= F6_ROWS) break;  // I0 + F6_ROWS may pass 32 bits
+                }
             }
             arad_pair_kernel<true><<<blocks, tpb, 0, st>>>(X1, Z1, N1, w1, nm1, X2, Z2, N2, w2, nm2,
                                                            amax, P, sig, ns, symmetric, Ks,

@@ -216,7 +216,8 @@ def _arad(X1, X2, Z1, Z2, sigmas, width, cut_distance, r_width, c_width, symmetr
 
 
 def arad_launches(symmetric, precision, amax, nsigma):
-    """Kernel launches of one ``fmlb_arad_kernels`` call (mirrors its host code)."""
+    """Kernel launches of one ``fmlb_arad_kernels`` call of at most 65535 molecules in the
+    first set (mirrors its host code)."""
     sets = 1 if symmetric else 2
     chunks = -(-nsigma // (8 if precision == "fp32" and amax <= 32 else 16))
     if amax <= 32:  # prep, class assign, self, gated generic self (FP32: record sort) per set;
