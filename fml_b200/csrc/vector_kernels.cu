@@ -14,7 +14,7 @@
 // distance tiles (dist_tile.cuh). A tile's distances go to shared memory, each
 // row is summed over the columns of one molecule and these sums over the rows
 // of one molecule, in a fixed order, so the result does not depend on
-// scheduling.
+// scheduling. (Small sets of short descriptors: vector_pair_kernel.)
 //
 // Bound by FP64 issue: subtract, multiply, add per feature and atom pair, as
 // the reference rounds them (a contracted FMA moves kernels of 1e-100 by more
@@ -50,6 +50,17 @@ struct VkSide {
     int nm, amax, group;
 };
 
+// Atoms of molecule m and its first row in X.
+__device__ __forceinline__ int vk_molecule(const VkSide &s, int m, long long &first, int *status) {
+    int n = s.O ? s.O[m + 1] - s.O[m] : s.N[m];
+    first = s.O ? s.O[m] : (long long)m * s.amax;  // 2^24 molecules x 128 atoms pass 32 bits
+    if (n < 0 || n > s.amax) {  // rejected on the host as well
+        if (status) atomicCAS(status, 0, 1);
+        n = min(max(n, 0), s.amax);
+    }
+    return n;
+}
+
 // Atom list of molecules [m0, m0 + group): seg[q] = first list entry of
 // molecule m0 + q, row[] = its rows in X. One whole warp.
 __device__ __forceinline__ void vk_list(const VkSide &s, int m0, int *seg, long long *row,
@@ -57,15 +68,7 @@ __device__ __forceinline__ void vk_list(const VkSide &s, int m0, int *seg, long 
     const int lane = threadIdx.x & 31;
     int n = 0;
     long long first = 0;
-    if (lane < s.group && m0 + lane < s.nm) {
-        const int m = m0 + lane;
-        n = s.O ? s.O[m + 1] - s.O[m] : s.N[m];
-        first = s.O ? s.O[m] : (long long)m * s.amax;
-        if (n < 0 || n > s.amax) {  // rejected on the host as well
-            if (status) atomicCAS(status, 0, 1);
-            n = min(max(n, 0), s.amax);
-        }
-    }
+    if (lane < s.group && m0 + lane < s.nm) n = vk_molecule(s, m0 + lane, first, status);
     int incl = n;
     for (int d = 1; d <= VK_MAX_GROUP; d <<= 1) {
         const int o = __shfl_up_sync(0xffffffffu, incl, d);
@@ -106,7 +109,7 @@ vector_kernels_kernel(const VkSide s1, const VkSide s2, int d, const __grid_cons
     __shared__ double stage[dist::stage_doubles<4, 8>()];  // features, then the distance tile
     __shared__ double part[VK_T][VK_MAX_GROUP + 1];
     __shared__ int seg1[VK_MAX_GROUP + 1], seg2[VK_MAX_GROUP + 1];
-    __shared__ long long row1[VK_ROWS], row2[VK_ROWS];  // 2^24 molecules x 128 atoms pass 32 bits
+    __shared__ long long row1[VK_ROWS], row2[VK_ROWS];
     static_assert(VK_T * VK_P <= dist::stage_doubles<4, 8>(), "the tile fits");
     double(*D)[VK_P] = reinterpret_cast<double(*)[VK_P]>(stage);
     const int tid = threadIdx.x, warp = tid >> 5;
@@ -160,14 +163,83 @@ vector_kernels_kernel(const VkSide s1, const VkSide s2, int d, const __grid_cons
     }
 }
 
+// Small sets of short descriptors: a CTA per molecule pair, two atom pairs at most per
+// thread, 32 features of all atoms in shared memory at a time. What counts there is the
+// time of one CTA from its start to its end, of which the tile takes 2 to 4 us more. us
+// with a CTA per pair and with tiles: 30 x 36 molecules of 7 atoms, d = 28, 6, 10; 10
+// atoms, d = 55, 9, 12; 45 x 54 of 11, d = 120, 23, 25; 52 x 62 of 11, d = 66, 19, 19, d =
+// 100, 29, 27; 1 and 100 atoms, d = 30, 19, 27, 100 x 120 of these 57, 67.
+constexpr int VP_TPB = 64, VP_ATOM_PAIRS = 2 * VP_TPB, VP_FEATURES = 32, VP_PITCH = 33;
+constexpr int VP_MAX_D = 128, VP_PAIRS_PER_SM = 24;
+
+template <int KIND>
+__global__ void __launch_bounds__(VP_TPB)
+vector_pair_kernel(const VkSide s1, const VkSide s2, int d, const __grid_constant__ Coefs coef,
+                   int nsig, double *__restrict__ K, int *__restrict__ status) {
+    extern __shared__ double ksum[];  // features of the first side's atoms, then the second's
+    __shared__ double half[VK_MAX_SIGMAS];
+    double *A = ksum, *B = A + s1.amax * VP_PITCH;
+    const int i = (int)(blockIdx.x / (unsigned)s2.nm), j = (int)(blockIdx.x % (unsigned)s2.nm);
+    const int t = threadIdx.x, lane = t & 31;
+    int *stat = t == 0 ? status : nullptr;
+    long long f1, f2;
+    const int ni = vk_molecule(s1, i, f1, stat), nj = vk_molecule(s2, j, f2, stat), np = ni * nj;
+    const double *x1 = s1.X + f1 * d, *x2 = s2.X + f2 * d;
+    int at[2], bt[2];
+    double dist[2] = {0.0, 0.0};
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {  // atom pair t + 64 q; past the last: the last once more
+        const int p = max(min(t + q * VP_TPB, np - 1), 0), b = ni ? p / ni : 0;
+        at[q] = (p - b * ni) * VP_PITCH;
+        bt[q] = b * VP_PITCH;
+    }
+    for (int c = 0; c < d && np > 0; c += VP_FEATURES) {
+        const int nf = min(VP_FEATURES, d - c);
+        __syncthreads();
+        for (int e = t; e < ni * VP_FEATURES; e += VP_TPB) {
+            const int a = e / VP_FEATURES, f = e % VP_FEATURES;
+            if (f < nf) A[a * VP_PITCH + f] = x1[(size_t)a * d + c + f];
+        }
+        for (int e = t; e < nj * VP_FEATURES; e += VP_TPB) {
+            const int b = e / VP_FEATURES, f = e % VP_FEATURES;
+            if (f < nf) B[b * VP_PITCH + f] = x2[(size_t)b * d + c + f];
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int k = 0; k < nf; ++k)
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                dist[q] = dist::add_term<KIND == 0 ? dist::kSquareUnfused : dist::kAbs>(
+                    dist[q], A[at[q] + k], B[bt[q] + k]);
+    }
+    double mine = 0.0;  // lane k's: the first warp's sum of sigma k
+#pragma unroll 1
+    for (int k = 0; k < nsig; ++k) {
+        double v = 0.0;
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+            if (t + q * VP_TPB < np) v += exp(dist[q] * coef.c[k]);
+        for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (t == VP_TPB / 2) half[k] = v;
+        if (lane == k) mine = v;
+    }
+    __syncthreads();
+    if (t < nsig) K[((size_t)t * s1.nm + i) * s2.nm + j] = mine + half[t];
+}
+
+bool vk_small(const VkSide &s1, const VkSide &s2, int d) {
+    return s1.amax * s2.amax <= VP_ATOM_PAIRS && d <= VP_MAX_D &&
+           (long long)s1.nm * s2.nm <= (long long)VP_PAIRS_PER_SM * sm_count();
+}
+
 // Molecules per group: about 80 atoms at the usual fill of a padded row (the
 // tile's unused rows and columns then cost a sixth), fewer while the blocks
-// would not fill the GPU a few times over. Two blocks per SM are enough where a
-// block is one tile: smaller ones leave more of it empty. us for groups of 1 x 1, 2 x 1
-// and 2 x 2 of 23 atoms, d = 276, one sigma: 30 x 30 molecules 73, 62, -; 40 x 40 105, 95,
-// 76; 60 x 60 (2 x 1, 2 x 2) 159, 122; 74, 113 and 215 us with a CTA per molecule pair.
-// Only small sets of short descriptors were faster with that, where the tile's own
-// latency is all there is (30 x 36 molecules of 7 atoms, d = 28: 6 us, now 10).
+// would not fill the GPU a few times over: a side of more than one tile is halved until
+// there are eight blocks per SM, one within a tile only until there are two, since that
+// leaves more of the tile empty. us for groups of 1 x 1, 2 x 1 and 2 x 2 of 23 atoms, d =
+// 276, one sigma: 30 x 30 molecules 73, 62, -; 40 x 40 105, 95, 76; 60 x 60 (2 x 1, 2 x 2)
+// 159, 122. 100 x 120 of 4 and 30 atoms, d = 100: 8 x 2 molecules 53, 2 x 2 126. With a CTA
+// per molecule pair: 74, 113, 215 and 84 us.
 void vk_groups(VkSide &s1, VkSide &s2) {
     auto most = [](const VkSide &s) { return std::max(1, std::min(VK_MAX_GROUP, VK_ROWS / s.amax)); };
     s1.group = most(s1);
@@ -175,16 +247,23 @@ void vk_groups(VkSide &s1, VkSide &s2) {
     auto blocks = [&] {
         return (long long)ceil_div(s1.nm, s1.group) * ceil_div(s2.nm, s2.group);
     };
-    auto one_tile = [&] { return s1.group * s1.amax <= VK_T && s2.group * s2.amax <= VK_T; };
-    while (blocks() < (one_tile() ? 2LL : 8LL) * sm_count() && (s1.group > 1 || s2.group > 1)) {
-        int &g = s1.group >= s2.group ? s1.group : s2.group;
-        g = (g + 1) / 2;
+    for (;;) {
+        const bool first = s2.group == 1 || (s1.group > 1 && s1.group * s1.amax >= s2.group * s2.amax);
+        VkSide &s = first ? s1 : s2;
+        if (s.group == 1 || blocks() >= (s.group * s.amax > VK_T ? 8LL : 2LL) * sm_count()) break;
+        s.group = (s.group + 1) / 2;
     }
 }
 
 template <int KIND>
 int launch_vk(VkSide s1, VkSide s2, int d, const Coefs &coef, int nsig, double *K, int *status,
               cudaStream_t st) {
+    if (vk_small(s1, s2, d)) {
+        const size_t smem = sizeof(double) * VP_PITCH * (s1.amax + s2.amax);  // at most 34 KB
+        vector_pair_kernel<KIND><<<(unsigned)(s1.nm * s2.nm), VP_TPB, smem, st>>>(s1, s2, d, coef,
+                                                                                 nsig, K, status);
+        return launch_status("vector_pair_kernel");
+    }
     vk_groups(s1, s2);
     // at most 16 KB, but beside 41 KB of static shared memory: with many sigmas the two
     // pass the 48 KB that a launch gets without the attribute

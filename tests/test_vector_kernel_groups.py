@@ -14,17 +14,18 @@ def _groups(nm1, nm2, amax):
     """Molecules of a CTA per side (the rule of vector_kernels.cu, same amax)."""
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     g = [max(1, min(8, 160 // amax))] * 2
-    while -(-nm1 // g[0]) * -(-nm2 // g[1]) < (2 if max(g) * amax <= 64 else 8) * sms and max(g) > 1:
+    while True:
         q = 0 if g[0] >= g[1] else 1
+        if g[q] == 1 or -(-nm1 // g[0]) * -(-nm2 // g[1]) >= (8 if g[q] * amax > 64 else 2) * sms:
+            return tuple(g)
         g[q] = (g[q] + 1) // 2
-    return tuple(g)
 
 
 @pytest.mark.parametrize("amax,nm1,nm2,d,nsig,groups", [
     (7, 300, 290, 5, 3, (8, 8)), (20, 290, 283, 5, 1, (8, 8)), (20, 300, 300, 3, 19, (8, 8)),
     (8, 300, 300, 3, 32, (8, 8)), (22, 260, 250, 3, 24, (7, 7)), (23, 220, 230, 9, 2, (6, 6)),
     (50, 110, 109, 7, 2, (3, 3)), (23, 40, 43, 9, 2, (2, 2)), (23, 30, 31, 5, 1, (1, 2)),
-    (7, 100, 99, 5, 2, (4, 8)), (10, 50, 48, 5, 1, (2, 4))])
+    (7, 100, 99, 5, 2, (4, 8)), (10, 80, 75, 5, 1, (4, 4))])
 @pytest.mark.parametrize("kind", ["gaussian", "laplacian"])
 def test_groups_of_several_molecules(oracle_mod, kind, amax, nm1, nm2, d, nsig, groups):
     assert _groups(nm1, nm2, amax) == groups
