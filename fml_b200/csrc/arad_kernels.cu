@@ -110,9 +110,9 @@ SetWs carve(char *&p, int nm, int amax) {
 
 // exp(x) for the terms inside the window, x in [-16, 0] (the reduction holds to
 // -700): x = k ln2 + r with ln2 in two parts, exp(r) by the polynomial of degree
-// 11 that interpolates it at the Chebyshev nodes of [-ln2/2, ln2/2] (relative
-// error 1.5e-17; coefficients computed in 60 digits and rounded), the exponent
-// added as an integer. Within 0.9 ulp (0.26 on average); half the instructions of the general
+// 11 that interpolates it at the Chebyshev nodes of [-ln2/2, ln2/2] widened by 0.05 %
+// (k rounds a product that is itself rounded; relative error 1.5e-17; coefficients
+// computed in 60 digits and rounded), the exponent added as an integer. Within 0.9 ulp (0.26 on average); half the instructions of the general
 // function, which has to look after every argument.
 __device__ __forceinline__ double exp_window(double x) {
     const double magic = 6755399441055744.0;  // 1.5 * 2^52: rounds to an integer
@@ -299,8 +299,12 @@ __device__ __forceinline__ void pair_index(long long t, int symmetric, int nm2, 
 // Stage 2: one warp per molecule pair; lanes stride over atom pairs.
 // kDist: store every atom pair's l2 in D (nm1, nm2, amax, amax) instead of
 // the kernel sums (atomic_arad_l2_distance_all, farad.f90:452-600).
+// The bounds keep FP64 at four CTAs per SM, the distances at five: with the constants
+// of the exponential in registers they took three and four (200 molecules of up to 33
+// atoms, symmetric: 31.6 ms, 37.3 without the bound; 100 x 120 distances 28.9, 33.4). The
+// lanes' atom pairs share j1 rather than i1 (28.2 ms; FP32, 40 atoms 14.3 instead of 38.7).
 template <bool kF64, bool kDist = false>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, kDist ? 5 : kF64 ? 4 : 0)
 arad_pair_kernel(const double *__restrict__ X1, const double *__restrict__ Z1,
                  const int *__restrict__ N1, SetWs w1, int nm1, const double *__restrict__ X2,
                  const double *__restrict__ Z2, const int *__restrict__ N2, SetWs w2, int nm2,
@@ -326,7 +330,9 @@ arad_pair_kernel(const double *__restrict__ X1, const double *__restrict__ Z1,
         for (int s = 0; s < MAXSIG; ++s) acc[s] = 0.0;
         const int P2 = nI * nJ;
         for (int p = lane; p < P2; p += 32) {
-            const int i1 = p / nJ, j1 = p - i1 * nJ;
+            // kernels: i1 fastest, the order in which the fast FP64 kernel sums its pairs too
+            const int n1 = kDist ? nJ : nI, hi = p / n1, lo = p - hi * n1;
+            const int i1 = kDist ? hi : lo, j1 = kDist ? lo : hi;
             const size_t b1 = (size_t)I * amax + i1, b2 = (size_t)J * amax + j1;
             const double dz1 = __dsub_rn(Z1[b1 * 2 + 0], Z2[b2 * 2 + 0]);
             const double dz2 = __dsub_rn(Z1[b1 * 2 + 1], Z2[b2 * 2 + 1]);
@@ -1628,7 +1634,7 @@ __global__ void arad_atom_prep_kernel(const double *__restrict__ Q, const int *_
 // kDistance the l2 itself is stored, K[i, j] = l2(i, j) (the distances of
 // fget_atomic_distance_arad, :902-1030).
 template <bool kDistance>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 7)
 arad_atom_pair_kernel(const double *__restrict__ Q1, const double *__restrict__ Z1,
                       const int *__restrict__ nnb1, const double *__restrict__ S1,
                       const double *__restrict__ self1, int na1,
@@ -1793,6 +1799,7 @@ static int arad_kernels_impl(const double *X1, const double *Z1, const int *N1, 
     SetWs w2 = symmetric ? w1 : carve(p, nm2, amax);
     ClassInfo *ci = reinterpret_cast<ClassInfo *>(p);
     const int tpb = 128;
+    const long long npairs = symmetric ? (long long)nm1 * (nm1 + 1) / 2 : (long long)nm1 * nm2;
     // fast paths: amax <= 32 and at most 16 element classes (decided on the device)
     const bool try_fast = amax <= FC_MAXA;
     ClassInfo *fast_ci = try_fast ? ci : nullptr;
@@ -1835,7 +1842,6 @@ static int arad_kernels_impl(const double *X1, const double *Z1, const int *N1, 
             s.X, s.N, s.nm, amax, P, s.w, fast_ci);
         FMLB_TRY(launch_status("arad_generic_self_kernel"));
     }
-    const long long npairs = symmetric ? (long long)nm1 * (nm1 + 1) / 2 : (long long)nm1 * nm2;
     const int blocks = (int)std::min<long long>(ceil_div(npairs, tpb / 32), (long long)sm_count() * 64);
     const int chunk = try_fast && precision == 1 ? FC_MAXSIG : MAXSIG;
     for (int s0 = 0; s0 < nsigma; s0 += chunk) {
