@@ -1582,6 +1582,17 @@ arad_f64_pair_kernel(const double *__restrict__ X1, SetWs w1, const int *__restr
 // such blocks fill the GPU several times over.
 inline int f64_block(long long npairs) { return npairs >= (1LL << 13) ? 4 : 1; }
 
+// Small molecules keep the fast kernel's CTA waiting for itself: it orders and prepares a
+// few dozen terms, and a warp per molecule pair does them in less. The fewer the pairs,
+// the smaller the molecules for which that holds: a lone warp takes longer for its pair
+// than a CTA. Both give the same bits. us of a warp per pair and of the fast kernel,
+// symmetric: 5 atoms, 30 molecules 35, 53, 1000 2487, 5529; 6 atoms, 30 58, 59, 200 205,
+// 301; 7 atoms, 30 74, 68, 200 292, 345; 8 atoms, 200 365, 388; 9 atoms, 200 526, 432, 1000
+// 8246, 9043.
+bool f64_generic(int amax, long long npairs) {
+    return amax <= 5 || (amax <= 9 && npairs >= 1LL << (3 * amax - 10));
+}
+
 // The fast kernels' shared memory is dynamic (above the 48 KB static limit);
 // the attribute is set once per device.
 int fast_smem_attrs() {
@@ -1801,7 +1812,7 @@ static int arad_kernels_impl(const double *X1, const double *Z1, const int *N1, 
     const int tpb = 128;
     const long long npairs = symmetric ? (long long)nm1 * (nm1 + 1) / 2 : (long long)nm1 * nm2;
     // fast paths: amax <= 32 and at most 16 element classes (decided on the device)
-    const bool try_fast = amax <= FC_MAXA;
+    const bool try_fast = amax <= FC_MAXA && !(precision == 0 && f64_generic(amax, npairs));
     ClassInfo *fast_ci = try_fast ? ci : nullptr;
     if (try_fast)
         FMLB_TRY(cuda_status(cudaMemsetAsync(ci, 0, sizeof(ClassInfo), st), "clear class info"));

@@ -215,12 +215,15 @@ def _arad(X1, X2, Z1, Z2, sigmas, width, cut_distance, r_width, c_width, symmetr
     return to_output(K, as_np)
 
 
-def arad_launches(symmetric, precision, amax, nsigma):
-    """Kernel launches of one ``fmlb_arad_kernels`` call of at most 65535 molecules in the
-    first set (mirrors its host code)."""
+def arad_launches(symmetric, precision, amax, nsigma, pairs=1 << 20):
+    """Kernel launches of one ``fmlb_arad_kernels`` call of ``pairs`` molecule pairs and at
+    most 65535 molecules in the first set (mirrors its host code)."""
     sets = 1 if symmetric else 2
-    chunks = -(-nsigma // (8 if precision == "fp32" and amax <= 32 else 16))
-    if amax <= 32:  # prep, class assign, self, gated generic self (FP32: record sort) per set;
+    fast = amax <= 32
+    if precision != "fp32" and (amax <= 5 or (amax <= 9 and pairs >= 1 << (3 * amax - 10))):
+        fast = False  # a warp per molecule pair
+    chunks = -(-nsigma // (8 if precision == "fp32" and fast else 16))
+    if fast:  # prep, class assign, self, gated generic self (FP32: record sort) per set;
         # class build; fast + gated generic pair per sigma chunk
         return (5 if precision == "fp32" else 4) * sets + 1 + 2 * chunks
     return 2 * sets + chunks
