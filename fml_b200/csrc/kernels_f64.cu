@@ -91,9 +91,11 @@ distance_kernel_f64(const double *__restrict__ A, int na, int lda, const double 
         if (mirror) {
             __syncthreads();
             // T[c][r] -> K[col0 + c][row0 + r], coalesced in r
-            for (int t = threadIdx.x; t < BN * BM; t += TPB) {
-                const int c = t / BM, r = t % BM;
-                if (c < nc && r < nr) Ks[(size_t)(col0 + c) * ldk + row0 + r] = T[c][r];
+            const int r = threadIdx.x % BM, first = threadIdx.x / BM;
+            double *out = Ks + (size_t)(col0 + first) * ldk + row0 + r;
+            if (r < nr) {
+#pragma unroll 8
+                for (int c = first; c < nc; c += TPB / BM, out += (TPB / BM) * ldk) *out = T[c][r];
             }
             __syncthreads();
         }
