@@ -61,16 +61,9 @@ namespace fmlb {
 namespace {
 
 constexpr int OZ_BM = 128, OZ_BN = 128;
-#ifndef OZ_PASS_DIAGONALS
-#define OZ_PASS_DIAGONALS 4
-#endif
-// Diagonals (int32 accumulators of 128 columns) per pass, and the TMEM buffers
-// the 512 columns hold: with two, a pass's MMAs run while the epilogue drains
-// the previous pass.
-constexpr int OZ_PASS_Q = OZ_PASS_DIAGONALS;
-constexpr int OZ_TMEM_BUFS = 4 / OZ_PASS_Q;  // 512 columns: 2 buffers of 2, 1 of 3 or 4
+// Diagonals (int32 accumulators of 128 columns) per pass: what the 512 TMEM columns hold.
+constexpr int OZ_PASS_Q = 4;
 constexpr int OZ_MAX_PASSES = (8 + OZ_PASS_Q - 1) / OZ_PASS_Q;
-static_assert(OZ_PASS_Q == 4, "one TMEM buffer of four diagonals, at most two passes");
 constexpr int OZ_KB = 64;          // int8 k values (bytes) per stage: two MMA K steps
 constexpr int OZ_MMA_K = 32;       // k values of one MMA
 constexpr int OZ_MAX_STAGES = 8;  // the ring depth is set per launch from shared memory
@@ -95,7 +88,7 @@ constexpr int OZ_NONFINITE = 0x7fffffff;    // exponent marking a row with Inf /
 
 constexpr long long kOzDefaultBudget = 4000000000LL;  // clock cycles (~2 s)
 constexpr int OZ_SMEM_LIMIT = 232448 - 64;  // opt-in shared memory per CTA, less static
-constexpr int OZ_BAR_BYTES = (2 * OZ_MAX_STAGES + 2 * OZ_TMEM_BUFS + 1) * 8 + 8;
+constexpr int OZ_BAR_BYTES = (2 * OZ_MAX_STAGES + 3) * 8 + 8;
 
 struct OzParams {
     int m;             // rows (= columns) of C
@@ -238,8 +231,8 @@ ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
     double *cstage = reinterpret_cast<double *>(smem + nst * stage_bytes);
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + nst * stage_bytes + OZ_CSTAGE_BYTES);
     uint64_t *full = bars, *empty = bars + OZ_MAX_STAGES;
-    uint64_t *tmem_full = bars + 2 * OZ_MAX_STAGES, *tmem_empty = tmem_full + OZ_TMEM_BUFS,
-             *mma_done = tmem_empty + OZ_TMEM_BUFS;
+    uint64_t *tmem_full = bars + 2 * OZ_MAX_STAGES, *tmem_empty = tmem_full + 1,
+             *mma_done = tmem_empty + 1;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mma_done + 1);
     __shared__ int abort_cta;
 
@@ -250,10 +243,8 @@ ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
             tc::mbar_init(&full[s], 1);
             tc::mbar_init(&empty[s], 1);
         }
-        for (int b = 0; b < OZ_TMEM_BUFS; ++b) {
-            tc::mbar_init(&tmem_full[b], 1);
-            tc::mbar_init(&tmem_empty[b], OZ_EPI_WARPS);
-        }
+        tc::mbar_init(tmem_full, 1);
+        tc::mbar_init(tmem_empty, OZ_EPI_WARPS);
         tc::mbar_init(mma_done, 1);
         tc::mbar_fence_init();
     }
@@ -311,9 +302,7 @@ ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
                 int row0, col0;
                 if (!oz_tile(t, p, row0, col0)) continue;
                 for (int ps = 0; ps < npass; ++ps, ++lp) {
-                    const int buf = lp % OZ_TMEM_BUFS;
-                    if (!tc::mbar_wait(&tmem_empty[buf], (uint32_t)(((lp / OZ_TMEM_BUFS) & 1) ^ 1),
-                                       budget)) {
+                    if (!tc::mbar_wait(tmem_empty, (uint32_t)((lp & 1) ^ 1), budget)) {
                         oz_fail(info);
                         ok = false;
                         break;
@@ -332,13 +321,12 @@ ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
                         const uint8_t *sb = sa + NS * OZ_A_PLANE;
                         const uint64_t da = tc::smem_desc_kmajor(sa, OZ_KB);
                         const uint64_t db = tc::smem_desc_kmajor(sb, OZ_KB);
-                        const uint32_t dacc = tmem_base + (uint32_t)(buf * OZ_PASS_Q * OZ_BN);
-                        if (ps == 0) oz_issue<NS, 0>(dacc, da, db, kb > 0);
-                        else oz_issue<NS, npass - 1>(dacc, da, db, kb > 0);
+                        if (ps == 0) oz_issue<NS, 0>(tmem_base, da, db, kb > 0);
+                        else oz_issue<NS, npass - 1>(tmem_base, da, db, kb > 0);
                         tc::mma_commit(&empty[st]);  // frees the stage once these MMAs finish
                     }
                     if (!ok) break;
-                    tc::mma_commit(&tmem_full[buf]);
+                    tc::mma_commit(tmem_full);
                 }
             }
             // every MMA issued has finished before TMEM is released
@@ -401,15 +389,14 @@ ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
                 const bool last = ps == npass - 1;
                 // Horner over diagonals q0 .. q1-1 carries 256^(q1-1-q): scale by 256^-(q1+1)
                 const double pbias = __longlong_as_double((long long)(1023 - 8 * (q1 + 1)) << 52);
-                const int buf = lp % OZ_TMEM_BUFS;
-                if (!tc::mbar_wait(&tmem_full[buf], (uint32_t)((lp / OZ_TMEM_BUFS) & 1), budget)) {
+                if (!tc::mbar_wait(tmem_full, (uint32_t)(lp & 1), budget)) {
                     oz_fail(info);
                     ok = false;
                     break;
                 }
                 tc::fence_after_sync();
                 const uint32_t tbase = tmem_base + ((uint32_t)(qw * 32) << 16) +
-                                       (uint32_t)(buf * OZ_PASS_Q * OZ_BN + half * 64);
+                                       (uint32_t)(half * 64);
                 double acc[64];
                 {
                     uint32_t v[OZ_PASS_Q][OZ_CHUNK];
@@ -437,7 +424,7 @@ ozaki_syrk_kernel(const __grid_constant__ OzMaps maps,
                 }
                 tc::fence_before_sync();
                 __syncwarp();
-                if (lane == 0) tc::mbar_arrive(&tmem_empty[buf]);  // the buffer is free
+                if (lane == 0) tc::mbar_arrive(tmem_empty);  // the accumulators are free
 #pragma unroll
                 for (int ch = 0; ch < 64 / OZ_CHUNK; ++ch) {
                     const int cb = ch * OZ_CHUNK;
