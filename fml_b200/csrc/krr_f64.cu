@@ -10,7 +10,7 @@
 // partial sums are reduced in a second pass in a fixed order (deterministic).
 // A chunk is worked by a cluster of eight CTAs, 128 training points each, whose
 // sums meet in distributed shared memory: with one CTA per chunk, 1000 queries
-// against 1000 training points ran on 16 of the SMs (600 us, now about 60).
+// against 1000 training points ran on 16 of the SMs (600 us, now 75).
 #include <cooperative_groups.h>
 #include <limits.h>
 #include <math.h>
@@ -98,8 +98,8 @@ predict_partial_kernel(const double *__restrict__ Q, int nq, int ldq, const doub
 
 // The partial sums of every chunk, in tiles of 16, 32 or 64 queries by the number
 // of CTAs that the largest would give. us for 16, 32, 64 queries, d = 276: 200 x 1000
-// 44, 56, 107; 500 x 1000 66, 74, 107; 1000 x 1000 118, 78, 115; 2000 x 1000 220, 139,
-// 151; 1000 x 2000 220, 140, 130; 2000 x 2000 396, 257, 225.
+// 41, 52, 70; 500 x 1000 64, 71, 70; 1000 x 1000 114, 76, 113; 2000 x 1000 213, 134,
+// 117; 1000 x 2000 214, 134, 117; 2000 x 2000 392, 249, 211.
 int launch_predict_partial(int kind, const double *Xq, int nq, int ldq, const double *Xt, int nt,
                            int ldt, int d, const Scales &sc, int nsigma, const double *alpha,
                            long long lda_alpha, double *partial, cudaStream_t st) {
