@@ -14,8 +14,8 @@
 // the registers, which leaves room for 16 warps per SM (a warp cannot issue FP64
 // instructions back to back); they are issued behind a chunk's arithmetic, since
 // between the barrier and the chunk's first loads every warp waited for their
-// address arithmetic. Gaussian, 8191 x 8191, d = 435, symmetric, 3 sigmas: 2.18 ms
-// (72 % of the FP64 issue rate); 2.41 ms with 64 x 64 tiles of 4 x 4 pairs, 256 threads
+// address arithmetic. Gaussian, 8191 x 8191, d = 435, symmetric, 3 sigmas: 2.16 ms
+// (73 % of the FP64 issue rate); 2.41 ms with 64 x 64 tiles of 4 x 4 pairs, 256 threads
 // and a single buffer, 2.38 with 4 x 4 pairs and these copies.
 #pragma once
 

@@ -20,7 +20,7 @@
 // the reference rounds them (a contracted FMA moves kernels of 1e-100 by more
 // than the 1e-13 they agree with it to). A CTA per molecule pair with one atom
 // pair per thread and load pair was bound by shared memory (300 x 401 molecules
-// of up to 23 atoms, d = 276, 3 sigmas: 6.27 ms, now 2.13 ms).
+// of up to 23 atoms, d = 276, 3 sigmas: 6.27 ms, now 2.17 ms).
 #include <math.h>
 
 #include <algorithm>
